@@ -32,6 +32,7 @@ from ..ops import rope as rope_ops
 from ..ops import swiglu as swiglu_ops
 from ..parallel import fused_ops, tp_ops
 from ..parallel.sequence_parallel import ulysses as sp
+from . import decode_path
 
 IGNORE_INDEX = -100
 
@@ -324,11 +325,21 @@ class DecoderBackbone(nn.Module):
         self.gradient_checkpointing = False
         self.register_buffer("inv_freq", rope_ops.inv_freq(cfg.head_dim, cfg.rope_theta), persistent=False)
 
+    def _frequencies(self, dim: int, device) -> torch.Tensor:
+        """Rotary frequencies in fp32.  Casting a model to bf16 casts the buffer too; the fp32 values are then computed
+        once per device and kept (they are constants of the configuration)."""
+        invf = self.inv_freq
+        if invf.dtype == torch.float32 and invf.device == device:
+            return invf
+        kept = self.__dict__.setdefault("_fp32_frequencies", {})
+        key = (dim, float(self.cfg.rope_theta), device)
+        if key not in kept:
+            kept[key] = rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
+        return kept[key]
+
     def rope_tables(self, position_ids: torch.Tensor):
         cfg = self.cfg
-        invf = self.inv_freq
-        if invf.dtype != torch.float32 or invf.device != position_ids.device:
-            invf = rope_ops.inv_freq(cfg.head_dim, cfg.rope_theta, device=position_ids.device)
+        invf = self._frequencies(cfg.head_dim, position_ids.device)
         mode = {"none": rope_ops.MODE_PLAIN, "sectioned": rope_ops.MODE_SECTIONED, "interleaved": rope_ops.MODE_INTERLEAVED}[
             cfg.mrope_mode if position_ids.dim() == 2 else "none"
         ]
@@ -336,6 +347,11 @@ class DecoderBackbone(nn.Module):
         return rope_ops.rope_table(position_ids, invf, mode, sections)
 
     def forward(self, inputs_embeds: torch.Tensor, ctx: PackedContext) -> torch.Tensor:
+        if getattr(ctx, "kv_cache", None) is not None:
+            # one new token per sequence: all layers in one native call where it applies
+            hidden = decode_path.decode_layers(self, inputs_embeds, ctx)
+            if hidden is not None:
+                return hidden
         h, residual = inputs_embeds, None
         for i, layer in enumerate(self.layers):
             if self.gradient_checkpointing and self.training:

@@ -5,9 +5,9 @@ Rollouts of the policy-gradient trainers (src/lmms_engine/train in the reference
 ``capacity`` rows in one buffer per layer; a forward pass writes the rotated keys and the values of its new tokens behind
 the rows already held and attends to the gathered rows of every sequence (``cu_seqlens`` of the keys differ from those
 of the queries; the attention kernel aligns its causal mask bottom-right, so new token j of a sequence sees the cached
-rows and the new rows up to itself).  The gather costs one pass over the cached rows per layer and step - bandwidth
-that is small against reading the layer's weights - and keeps the kernel's packed layout, so no second attention
-kernel exists for decoding.
+rows and the new rows up to itself).  A pass that feeds one token per sequence runs all layers in one native call that
+reads the slabs in place (``models/decode_path.py``); the gather into the packed layout remains for passes with several
+new tokens per sequence on top of cached rows of several sequences.
 """
 from __future__ import annotations
 
@@ -26,13 +26,14 @@ class PackedKVCache:
         self.k: List[Optional[torch.Tensor]] = [None] * n_layers
         self.v: List[Optional[torch.Tensor]] = [None] * n_layers
         self.device = device
-        self._write = self._read = self._cu_k = None
-        self._max_k = 0
+        self._rows: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]] = None
         # layers that carry a recurrent state instead of keys / values (linear attention) keep it here:
         # ``state[layer][sequence]`` is whatever that layer stores (convolution tail, state matrix)
         self.state: dict = {}
         self.new_lens: List[int] = []
         self.had: List[int] = []
+        self.decode_window = -1
+        self._counters: Optional[torch.Tensor] = None
 
     def advance(self, new_lens: Sequence[int]) -> torch.Tensor:
         """Declare the next forward pass: ``new_lens[i]`` new tokens for sequence ``i`` (0 = none).  Returns the rotary
@@ -40,35 +41,71 @@ class PackedKVCache:
         new_lens = [int(n) for n in new_lens]
         if len(new_lens) != len(self.lens):
             raise ValueError(f"{len(new_lens)} lengths for a cache of {len(self.lens)} sequences")
-        write, read, pos, cu = [], [], [], [0]
         self.new_lens, self.had = new_lens, list(self.lens)
         for i, n in enumerate(new_lens):
-            have = self.lens[i]
-            if have + n > self.capacities[i]:
-                raise ValueError(f"sequence {i}: {have} cached + {n} new tokens exceed its capacity of {self.capacities[i]}")
-            if n == 0:
-                continue  # a sequence without new tokens has no query rows, hence no key document either
-            write.append(torch.arange(self.base[i] + have, self.base[i] + have + n))
-            read.append(torch.arange(self.base[i], self.base[i] + have + n))
-            pos.append(torch.arange(have, have + n))
-            cu.append(cu[-1] + have + n)
-            self.lens[i] = have + n
-        if not write:
+            if self.lens[i] + n > self.capacities[i]:
+                raise ValueError(f"sequence {i}: {self.lens[i]} cached + {n} new tokens exceed its capacity of {self.capacities[i]}")
+            self.lens[i] += n
+        if not any(new_lens):
             raise ValueError("a forward pass needs at least one new token")
-        dev = self.device
-        self._write, self._read = torch.cat(write).to(dev), torch.cat(read).to(dev)
-        self._cu_k = torch.tensor(cu, dtype=torch.int32, device=dev)
-        self._max_k = max(b - a for a, b in zip(cu[:-1], cu[1:]))
-        return torch.cat(pos).to(dev)
+        self._rows = None
+        return self._spread(self.had)
+
+    def _spread(self, starts: Sequence[int]) -> torch.Tensor:
+        """``starts[i], starts[i] + 1, ...`` for the new tokens of every sequence, on the cache's device."""
+        if max(self.new_lens) == 1:
+            return torch.tensor([s for s, n in zip(starts, self.new_lens) if n]).to(self.device)
+        return torch.cat([torch.arange(s, s + n) for s, n in zip(starts, self.new_lens) if n]).to(self.device)
+
+    def _row_tables(self) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]:
+        """Rows that this pass' tokens go to, rows that they attend to, and the boundaries of the latter; built once per
+        pass, when the first layer asks (the one-call decode path needs none of them)."""
+        if self._rows is None:
+            # a sequence without new tokens has no query rows, hence no key document either
+            live = [i for i, n in enumerate(self.new_lens) if n]
+            cu = [0]
+            for i in live:
+                cu.append(cu[-1] + self.lens[i])
+            write = self._spread([b + h for b, h in zip(self.base, self.had)])
+            read = write if not any(self.had[i] for i in live) else torch.cat(
+                [torch.arange(self.base[i], self.base[i] + self.lens[i]) for i in live]).to(self.device)
+            self._rows = (write, read, torch.tensor(cu, dtype=torch.int32, device=self.device), max(self.lens[i] for i in live))
+        return self._rows
+
+    def slabs(self, layer: int, n_heads: int, dim: int, dtype: torch.dtype, device) -> Tuple[torch.Tensor, torch.Tensor]:
+        """Key and value buffers of a layer, ``[rows of all sequences, n_heads, dim]``; rows past a sequence's length are
+        not initialised and never read."""
+        if self.k[layer] is None:
+            self.k[layer] = torch.empty((self.base[-1], n_heads, dim), dtype=dtype, device=device)
+            self.v[layer] = torch.empty_like(self.k[layer])
+        return self.k[layer], self.v[layer]
+
+    def decode_counters(self, n: int, device) -> torch.Tensor:
+        """Arrival counters of the split-key attention, zero between passes."""
+        if self._counters is None or self._counters.numel() < n or self._counters.device != device:
+            self._counters = torch.zeros(n, dtype=torch.int32, device=device)
+        return self._counters
 
     def extend(self, layer: int, k: torch.Tensor, v: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]:
         """Store this pass' keys / values of ``layer``; returns ``(keys, values, cu_seqlens_k, max_seqlen_k)`` of everything
         the new tokens attend to."""
-        if self._write is None or k.shape[0] != self._write.numel():
+        if not self.new_lens or k.shape[0] != sum(self.new_lens):
             raise ValueError("call advance() with this pass' token counts before the forward pass")
+        write, read, cu_k, max_k = self._row_tables()
+        k, v = k.detach(), v.detach()
         if self.k[layer] is None:
-            self.k[layer] = k.new_zeros((self.base[-1],) + tuple(k.shape[1:]))
-            self.v[layer] = v.new_zeros((self.base[-1],) + tuple(v.shape[1:]))
-        self.k[layer].index_copy_(0, self._write, k.detach())
-        self.v[layer].index_copy_(0, self._write, v.detach())
-        return self.k[layer].index_select(0, self._read), self.v[layer].index_select(0, self._read), self._cu_k, self._max_k
+            self.k[layer] = k.new_empty((self.base[-1],) + tuple(k.shape[1:]))
+            self.v[layer] = v.new_empty((self.base[-1],) + tuple(v.shape[1:]))
+        if sum(1 for n in self.new_lens if n) == 1:
+            i = next(i for i, n in enumerate(self.new_lens) if n)
+            lo, hi = self.base[i] + self.had[i], self.base[i] + self.lens[i]
+            self.k[layer][lo:hi].copy_(k)
+            self.v[layer][lo:hi].copy_(v)
+            if self.had[i]:
+                return self.k[layer][self.base[i]:hi], self.v[layer][self.base[i]:hi], cu_k, max_k
+        else:
+            self.k[layer].index_copy_(0, write, k)
+            self.v[layer].index_copy_(0, write, v)
+        if read is write:  # nothing was cached before this pass: its own rows are all there is
+            return k, v, cu_k, max_k
+        return self.k[layer].index_select(0, read), self.v[layer].index_select(0, read), cu_k, max_k

@@ -353,9 +353,7 @@ class Qwen35Backbone(DecoderBackbone):
 
     def rope_tables(self, position_ids: torch.Tensor):
         cfg = self.cfg
-        invf = self.inv_freq
-        if invf.dtype != torch.float32 or invf.device != position_ids.device:
-            invf = rope_ops.inv_freq(self.rot_dim, cfg.rope_theta, device=position_ids.device)
+        invf = self._frequencies(self.rot_dim, position_ids.device)
         mode = {"none": rope_ops.MODE_PLAIN, "sectioned": rope_ops.MODE_SECTIONED, "interleaved": rope_ops.MODE_INTERLEAVED}[
             cfg.mrope_mode if position_ids.dim() == 2 else "none"]
         sections = tuple(cfg.mrope_section) if (cfg.mrope_section and mode != rope_ops.MODE_PLAIN) else (0, 0, 0)

@@ -19,6 +19,11 @@ from . import _cuda
 # the library GEMM (torch.matmul) and only the fused epilogues use the in-tree kernel.
 LINEAR_BACKEND = "tcgen05"
 
+_cuda.register("b200_skinny_linear", "decode", "pppp" + "iii" + "lll" + "s")
+# Products of at most this many rows are bound by reading the weights once: one kernel spreads the weight rows over the
+# whole chip (csrc/decode.cu) where a 256-column tile would leave most of it idle.
+SKINNY_ROWS = 64
+
 
 def _ok(t: torch.Tensor) -> bool:
     return (
@@ -69,6 +74,10 @@ def gemm(
         raise TypeError("bad output tensor")
     if cin is not None and not _ok(cin):
         raise TypeError("bad cin tensor")
+    if M <= SKINNY_ROWS and not (a_mn_major or b_mn_major or symmetric) and alpha == 1.0 and cin is None and (N | K) % 8 == 0:
+        _cuda.call("b200_skinny_linear", a.data_ptr(), b.data_ptr(), _cuda.ptr(bias), out.data_ptr(), M, N, K, a.stride(0),
+                   b.stride(0), out.stride(0), _cuda.stream())
+        return out
     st = _cuda.status_word(a.device)
     _cuda.call(
         "b200_gemm_bf16",

@@ -93,8 +93,10 @@ def newton_schulz_graphed(X: torch.Tensor, steps: int, work: dict, max_ctas: int
         with torch.cuda.graph(graph):
             xs.copy_(xin)  # the chain overwrites its input (ping-pong buffer)
             out = newton_schulz(xs, steps, inner, max_ctas)
-        entry = work[key] = (graph, xin, out, inner)
-    graph, xin, out, _ = entry
+        # every buffer whose address the graph holds lives as long as the graph: xin, both ping-pong buffers (xs and the
+        # one in ``inner``) and the products in ``inner``
+        entry = work[key] = (graph, xin, xs, out, inner)
+    graph, xin, _, out, _ = entry
     xin.copy_(X)
     graph.replay()
     return out

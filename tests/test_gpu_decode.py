@@ -1,0 +1,92 @@
+"""One-token passes through the native layer loop against the layer-by-layer path on the same cache."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DENSE = dict(vocab_size=512, hidden_size=256, intermediate_size=520, num_hidden_layers=2, rms_norm_eps=1e-6)
+
+
+def _model(kind):
+    from lmms_engine_b200.mapping_func import create_model_from_config
+
+    torch.manual_seed(3)
+    if kind == "hybrid":
+        cfg = dict(DENSE, num_attention_heads=4, num_key_value_heads=2, head_dim=128, linear_conv_kernel_dim=4, linear_key_head_dim=128,
+                   linear_value_head_dim=128, linear_num_key_heads=4, linear_num_value_heads=8, partial_rotary_factor=0.25,
+                   full_attention_interval=2)
+        m = create_model_from_config("qwen3_5_text", cfg)
+    else:
+        heads, kv, dim, extra = {"grouped": (14, 2, 128, {}), "normed": (4, 2, 128, dict(attention_bias=False, qk_norm=True)),
+                                 "narrow": (4, 4, 64, {}), "wide_group": (12, 1, 128, {}),
+                                 "window": (4, 2, 128, dict(sliding_window=70, use_sliding_window=True))}[kind]
+        m = create_model_from_config("qwen2", dict(DENSE, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, **extra))
+    m = m.to("cuda", torch.bfloat16).eval()
+    with torch.no_grad():
+        for n, p in m.named_parameters():
+            if "norm" in n:
+                p.add_(torch.randn_like(p) * 0.1)
+            elif n.endswith("bias") and "dt_bias" not in n:
+                p.copy_(torch.randn_like(p) * 0.1)
+    return m
+
+
+def _go(model, prompts, steps, native):
+    from lmms_engine_b200.models import decode_path
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+    from lmms_engine_b200.ops import _cuda
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    n = len(prompts)
+    cache = PackedKVCache(len(model.model.layers), [p + steps for p in prompts], device=torch.device("cuda", 0))
+    ids = torch.randint(0, 512, (sum(prompts),), device="cuda", generator=gen)
+    keep, out = decode_path.MAX_SEQS, []
+    decode_path.MAX_SEQS = keep if native else 0
+    try:
+        with torch.no_grad():
+            pos = cache.advance(prompts)
+            cu = torch.tensor([0] + torch.tensor(prompts).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+            model(input_ids=ids, cu_seqlens=cu, position_ids=pos, kv_cache=cache)
+            for s in range(steps):
+                live = [1 if (i + s) % 3 or n == 1 else 0 for i in range(n)]  # sequences pause and resume
+                pos = cache.advance(live)
+                m = sum(live)
+                tok = torch.randint(0, 512, (m,), device="cuda", generator=gen)
+                cu = torch.arange(m + 1, dtype=torch.int32, device="cuda")
+                out.append(model(input_ids=tok, cu_seqlens=cu, position_ids=pos, kv_cache=cache)["hidden_states"])
+        _cuda.check_status()
+    finally:
+        decode_path.MAX_SEQS = keep
+    return torch.cat(out).float()
+
+
+@pytest.mark.parametrize("kind,prompts", [("grouped", [1]), ("grouped", [63, 64, 65, 700]), ("normed", [2100]), ("normed", [5] * 7 + [130] * 11),
+                                          ("narrow", [17, 300]), ("wide_group", [129, 40]), ("window", [50, 200]), ("hybrid", [100]),
+                                          ("hybrid", [64, 1, 130]), ("normed", list(range(1, 41))), ("normed", list(range(1, 65)))])
+def test_one_call_matches_layer_loop(kind, prompts):
+    """Both paths round every intermediate to bf16 at the same place, so only elements whose fp32 sums land on either side of
+    a rounding boundary differ, by one bf16 step (2^-8); two layers carry a few of those into an output of rms 1."""
+    model = _model(kind)
+    want, got = _go(model, prompts, 5, False), _go(model, prompts, 5, True)
+    assert torch.isfinite(got).all()
+    rel = ((got - want).norm() / want.norm()).item()
+    assert rel < 2.0 ** -7, rel
+
+
+def test_native_path_is_taken_and_hooks_keep_the_layer_loop():
+    from lmms_engine_b200.ops import _cuda
+
+    model = _model("grouped")
+    _go(model, [10], 1, True)
+    seen, real = [], _cuda.call
+    try:
+        _cuda.call = lambda name, *a: (seen.append(name), real(name, *a))[1]
+        _go(model, [10], 2, True)
+        assert seen.count("b200_decode_layers") == 2
+        del seen[:]
+        hook = model.model.layers[1].mlp.register_forward_hook(lambda *a: None)
+        _go(model, [10], 2, True)
+        hook.remove()
+        assert "b200_decode_layers" not in seen
+    finally:
+        _cuda.call = real

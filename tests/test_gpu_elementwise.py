@@ -336,3 +336,19 @@ def test_newton_schulz_graph_replay_equals_eager_and_reports_time():
             b.record()
             torch.cuda.synchronize()
             print(f"MUON_GRAPH_TIME {name}: {a.elapsed_time(b) / 100 * 1000:.1f} us per 1152 x 1152 chain (15 products)", flush=True)
+
+
+def test_newton_schulz_graph_owns_every_buffer_it_writes():
+    """Memory handed out after the capture is not written by a replay: the graph keeps all of its buffers alive."""
+    from lmms_engine_b200.ops import muon
+
+    torch.manual_seed(1)
+    work = {}
+    x = torch.randn(512, 640, device="cuda", dtype=torch.bfloat16)
+    x = x / x.float().norm()
+    muon.orthogonalize(x, 5, work)
+    torch.cuda.synchronize()
+    later = [torch.full((512, 640), 3.0, device="cuda", dtype=torch.bfloat16) for _ in range(16)]
+    muon.orthogonalize(x, 5, work)
+    torch.cuda.synchronize()
+    assert all(bool((t == 3.0).all()) for t in later)

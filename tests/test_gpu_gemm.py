@@ -127,3 +127,21 @@ def test_linear_autograd_matches_torch():
     _check(x.grad, xr.grad)
     _check(w.grad, wr.grad)
     _check(b.grad, br.grad)
+
+
+@pytest.mark.parametrize("M", [1, 4, 8, 9, 16, 17, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("N,K", [(8, 8), (1000, 520), (4608, 3584)])
+def test_few_rows(M, N, K):
+    """Weight-streaming product of at most 64 rows: tile edges of the row groups, ragged K and N, bias, strided input."""
+    from lmms_engine_b200.ops import gemm, _cuda
+
+    torch.manual_seed(M * N + K)
+    x = torch.randn(M, K + 8, device="cuda").to(torch.bfloat16)[:, :K]
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    b = torch.randn(N, device="cuda").to(torch.bfloat16)
+    want = x.float() @ w.float().t()
+    # one rounding to bf16 (2^-9 of the value) on top of fp32 sums
+    for bias, ref in ((None, want), (b, want + b.float())):
+        y = gemm.matmul_nt(x, w, bias)
+        _cuda.check_status()
+        assert ((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4 * K ** 0.5).all()
