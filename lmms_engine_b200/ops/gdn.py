@@ -1,11 +1,11 @@
 """Chunked gated delta rule over a packed batch of documents.
 
 Every document is padded to a multiple of 64 tokens and all chunks of all documents form one batch:
-the in-chunk work (decay matrices, the unit-triangular solve, in-chunk attention) runs as batched ops
-over ``[heads, chunks, 64, d]``; the chunk-to-chunk state recurrence runs in one CUDA kernel per
-direction (``csrc/gdn_scan.cu``) with a reset flag at the first chunk of every document.  On CPU (and for
-head dims the kernel does not cover) the recurrence is a plain loop over chunks, which is also the oracle
-of the kernel.
+the in-chunk work (decay matrices, the unit-triangular solve, in-chunk attention) runs in one kernel per
+direction that reads the packed rows through the row map (``csrc/gdn_chunk.cu``); the chunk-to-chunk state
+recurrence runs in one CUDA kernel per direction (``csrc/gdn_scan.cu``) with a reset flag at the first chunk of
+every document.  On CPU (and for head dims the kernels do not cover) the in-chunk work is batched framework ops over
+``[heads, chunks, 64, d]`` and the recurrence a plain loop over chunks, which are also the oracles of the kernels.
 
 Reference: the FLA ``chunk_gated_delta_rule`` call of the patched Gated-DeltaNet layers,
 src/lmms_engine/models/qwen3_5/qwen3_5_ops.py.
@@ -23,6 +23,10 @@ CHUNK = 64
 
 _cuda.register("b200_gdn_scan_fwd", "gdn_scan", "ppppppppp" + "iiii" + "s")
 _cuda.register("b200_gdn_scan_bwd", "gdn_scan", "pppppppppppppp" + "iiii" + "s")
+_cuda.register("b200_gdn_chunk_fwd", "gdn_chunk", "ppp" + "lll" + "ppp" + "l" + "ii" + "f" + "i" + "pppppppp" + "s")
+_cuda.register("b200_gdn_chunk_bwd", "gdn_chunk", "ppp" + "lll" + "ppp" + "l" + "ii" + "f" + "i" + "ppppp" + "pppppp" + "ppppp" + "s")
+_cuda.register("b200_gdn_chunk_out", "gdn_chunk", "ppppp" + "l" + "iii" + "s")
+_cuda.register("b200_gdn_chunk_out_bwd", "gdn_chunk", "ppppppp" + "l" + "iii" + "s")
 _cuda.register("b200_conv_silu_fwd", "gdn_conv", "pppp" + "l" + "iii" + "s")
 _cuda.register("b200_conv_silu_bwd", "gdn_conv", "pppppp" + "l" + "iii" + "s")
 
@@ -159,8 +163,102 @@ def plan_for(ctx, device):
     return plan
 
 
+def chunk_kernels_cover(q, k, v, back) -> bool:
+    """The fused in-chunk kernels hold one 64 x 128 block per operand: both head dims are 128 (any other runs as framework
+    ops), q, k and v share one 16- or 32-bit dtype, and every stream row belongs to a chunk (what they do not name is not
+    written)."""
+    return (q.is_cuda and q.shape[-1] == 128 and v.shape[-1] == 128 and q.dtype == k.dtype == v.dtype
+            and q.dtype in (torch.bfloat16, torch.float32) and q.shape == k.shape == v.shape and q.shape[0] == back.numel()
+            and 0 < q.shape[1] <= 65535)
+
+
+def _rows16(t: torch.Tensor) -> torch.Tensor:
+    """Rows of contiguous heads at any row stride that keeps 16-byte alignment."""
+    ok = t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.clone(memory_format=torch.contiguous_format)
+
+
+class _ChunkTerms(torch.autograd.Function):
+    """``_chunk_terms`` in one kernel per direction; the backward pass reads T, A and attn (64 x 64 per chunk and head) and
+    u, w again instead of solving a second time."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, src, n):
+        T, H, d = q.shape
+        q, k, v = _rows16(q), _rows16(k), _rows16(v)
+        gf, bf = g.float().contiguous(), beta.float().contiguous()
+        w, u, qt, kt = (torch.empty((H, n, CHUNK, d), dtype=torch.float32, device=q.device) for _ in range(4))
+        attn, inv, a = (torch.empty((H, n, CHUNK, CHUNK), dtype=torch.float32, device=q.device) for _ in range(3))
+        gamma = torch.empty((H, n), dtype=torch.float32, device=q.device)
+        _cuda.call("b200_gdn_chunk_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
+                   gf.data_ptr(), bf.data_ptr(), src.data_ptr(), T, H, n, d ** -0.5, int(q.dtype == torch.bfloat16), w.data_ptr(),
+                   u.data_ptr(), qt.data_ptr(), kt.data_ptr(), gamma.data_ptr(), attn.data_ptr(), inv.data_ptr(), a.data_ptr(),
+                   _cuda.stream())
+        ctx.save_for_backward(q, k, v, gf, bf, src, w, u, attn, inv, a)
+        ctx.gdt, ctx.bdt = g.dtype, beta.dtype
+        return w, u, qt, kt, gamma, attn
+
+    @staticmethod
+    def backward(ctx, dw, du, dqt, dkt, dgamma, dattn):
+        q, k, v, gf, bf, src, w, u, attn, inv, a = ctx.saved_tensors
+        T, H, d = q.shape
+        n = w.shape[1]
+        dw, du, dqt, dkt, dgamma, dattn = (_dense16(t) for t in (dw, du, dqt, dkt, dgamma, dattn))
+        dq, dk, dv = (torch.empty((T, H, d), dtype=q.dtype, device=q.device) for _ in range(3))
+        dg, db = torch.empty_like(gf), torch.empty_like(bf)
+        _cuda.call("b200_gdn_chunk_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
+                   gf.data_ptr(), bf.data_ptr(), src.data_ptr(), T, H, n, d ** -0.5, int(q.dtype == torch.bfloat16), w.data_ptr(),
+                   u.data_ptr(), attn.data_ptr(), inv.data_ptr(), a.data_ptr(), dw.data_ptr(), du.data_ptr(), dqt.data_ptr(),
+                   dkt.data_ptr(), dgamma.data_ptr(), dattn.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                   dg.data_ptr(), db.data_ptr(), _cuda.stream())
+        return dq, dk, dv, dg.to(ctx.gdt), db.to(ctx.bdt), None, None
+
+
+class _ChunkOut(torch.autograd.Function):
+    """``o_state + attn @ v_new`` written to the stream rows in the stream's dtype."""
+
+    @staticmethod
+    def forward(ctx, o_state, attn, v_new, src, T, dt):
+        o_state, attn, v_new = _dense16(o_state), _dense16(attn), _dense16(v_new)
+        H, n, _, dv = v_new.shape
+        out = torch.empty((T, H, dv), dtype=dt, device=v_new.device)
+        _cuda.call("b200_gdn_chunk_out", o_state.data_ptr(), attn.data_ptr(), v_new.data_ptr(), src.data_ptr(), out.data_ptr(), T, H, n,
+                   int(dt == torch.bfloat16), _cuda.stream())
+        ctx.save_for_backward(attn, v_new, src)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        attn, v_new, src = ctx.saved_tensors
+        dout = _dense16(dout)
+        H, n, _, dv = v_new.shape
+        d_o, d_v, d_a = torch.empty_like(v_new), torch.empty_like(v_new), torch.empty_like(attn)
+        _cuda.call("b200_gdn_chunk_out_bwd", dout.data_ptr(), attn.data_ptr(), v_new.data_ptr(), src.data_ptr(), d_o.data_ptr(),
+                   d_v.data_ptr(), d_a.data_ptr(), dout.shape[0], H, n, int(dout.dtype == torch.bfloat16), _cuda.stream())
+        return d_o, d_a, d_v, None, None, None
+
+
 def _chunk_terms(q, k, v, g, beta, src, back, n):
     """Per-chunk quantities of the rule from packed inputs: what the scan consumes and what finishes the output."""
+    if chunk_kernels_cover(q, k, v, back):
+        return _ChunkTerms.apply(q, k, v, g, beta, src, n)
+    return chunk_terms_ref(q, k, v, g, beta, src, back, n)
+
+
+def _chunk_output(o_state, attn, v_new, src, back, n, dt):
+    """Rows of the stream in ``dt`` from the state's and the chunk's own contribution."""
+    H, dv = v_new.shape[0], v_new.shape[-1]
+    if v_new.is_cuda and dv == 128 and dt in (torch.bfloat16, torch.float32) and H <= 65535 and v_new.dtype == torch.float32:
+        return _ChunkOut.apply(o_state, attn, v_new, src, back.numel(), dt)
+    out = o_state + attn @ v_new                   # [H, n, C, dv]
+    # back to the stream: cast first (half the bytes for bf16 streams), one strided copy, one gather
+    out = out.to(dt).movedim(0, 2).reshape(n * CHUNK, H, dv)
+    # stream row t sits at padded row back[t]; the gradient of this gather is the gather by ``src`` of [g; 0]
+    return _unpad(out, back, src)
+
+
+def chunk_terms_ref(q, k, v, g, beta, src, back, n):
+    """Framework-op form (CPU path, head dims the kernels do not cover, oracle of the kernels)."""
     dk = k.shape[-1]
 
     def lay(x):  # [T, H, ...] -> contiguous fp32 [H, n, C, ...] with zero padding rows
@@ -230,11 +328,7 @@ def chunk_gated_delta_rule_packed(q, k, v, g, beta, lengths: List[int], plan=Non
         return v.new_zeros((T, H, dv))
     w, u, qt, kt, gamma, attn = _chunk_terms(q, k, v, g, beta, src, back, n)
     v_new, o_state = scan(w, u, qt, kt, gamma, reset)
-    out = o_state + attn @ v_new                   # [H, n, C, dv]
-    # back to the stream: cast first (half the bytes for bf16 streams), one strided copy, one gather
-    out = out.to(dt).movedim(0, 2).reshape(n * CHUNK, H, dv)
-    # stream row t sits at padded row back[t]; the gradient of this gather is the gather by ``src`` of [g; 0]
-    return _unpad(out, back, src)
+    return _chunk_output(o_state, attn, v_new, src, back, n, dt)
 
 
 # ------------------------------------------------------------------------------ state hand-off between ranks
@@ -276,8 +370,7 @@ def chunk_gated_delta_rule_stateful(q, k, v, g, beta, state=None):
     n = len(reset)
     w, u, qt, kt, gamma, attn = _chunk_terms(q, k, v, g, beta, src, back, n)
     v_new, o_state, final = scan_with_state(w, u, qt, kt, gamma, reset, state, True)
-    out = (o_state + attn @ v_new).to(dt).movedim(0, 2).reshape(n * CHUNK, H, v.shape[-1])
-    return _unpad(out, back, src), final
+    return _chunk_output(o_state, attn, v_new, src, back, n, dt), final
 
 
 def chunk_gated_delta_rule_cp(q, k, v, g, beta, lengths: List[int], first_continues: bool, group, plan=None):

@@ -141,3 +141,72 @@ def test_conv_silu_bandwidth_report():
     fwd, bwd = min(times["fwd"]), min(times["bwd"])
     print(f"GDN_TIME conv fwd {fwd:.3f} ms = {2 * nbytes / fwd / 1e6:.0f} GB/s (x read + y written); "
           f"bwd {bwd:.3f} ms = {3 * nbytes / bwd / 1e6:.0f} GB/s (x, dy read + dx written)", flush=True)
+
+
+def _rule64(q, k, v, g, beta, lengths):
+    """Token-by-token rule in 64 bits: what the chunked form computes."""
+    q, k, v, g, beta = (t.double() for t in (q, k, v, g, beta))
+    q = q * torch.rsqrt((q * q).sum(-1, keepdim=True) + 1e-6) * q.shape[-1] ** -0.5
+    k = k * torch.rsqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    out, at = [], 0
+    for n in lengths:
+        s = torch.zeros(k.shape[1], k.shape[2], v.shape[2], dtype=torch.float64)
+        for t in range(at, at + n):
+            s = s * g[t].exp()[:, None, None]
+            d = (v[t] - torch.einsum("hk,hkv->hv", k[t], s)) * beta[t][:, None]
+            s = s + k[t][:, :, None] * d[:, None, :]
+            out.append(torch.einsum("hk,hkv->hv", q[t], s))
+        at += n
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("lengths,heads,dtype,strided", [((1,), 1, torch.bfloat16, False), ((63, 64, 65), 2, torch.float32, True),
+                                                         ((128, 7, 150), 3, torch.bfloat16, True), ((200,), 2, torch.float32, False)])
+def test_fused_chunk_kernels_match_64_bit_rule(lengths, heads, dtype, strided):
+    """One-row, one-short-of-a-chunk, exact and one-over documents; rows of a wider projection as q, k and v come in practice.
+    The bound of the fp32 form is 64 products deep sums at 2^-24 each, far inside 1e-4 of the largest value; bf16 streams add
+    the rounding of the stored rows (2^-9).  The fused kernels may not be further off than the framework-op form."""
+    from lmms_engine_b200.ops import _cuda, gdn
+
+    torch.manual_seed(1)
+    T = sum(lengths)
+    base = torch.randn(T, 3 * heads * 128).to(dtype)
+    q, k, v = (base[:, i * heads * 128:(i + 1) * heads * 128].reshape(T, heads, 128) for i in range(3))
+    g, beta = -2.0 * torch.rand(T, heads) ** 4, torch.rand(T, heads).to(dtype)
+    go = torch.randn(T, heads, 128).to(dtype)
+    ref = [t.double().requires_grad_() for t in (q, k, v, g, beta)]
+    want = _rule64(*ref, lengths)
+    (want * go.double()).sum().backward()
+
+    def run(fused):
+        leaf = None
+        if strided:
+            leaf = base.cuda().requires_grad_()
+            parts = [leaf[:, i * heads * 128:(i + 1) * heads * 128].view(T, heads, 128) for i in range(3)]
+        else:
+            parts = [t.cuda().requires_grad_() for t in (q, k, v)]
+        gg, bb = g.cuda().requires_grad_(), beta.cuda().requires_grad_()
+        keep = gdn.chunk_kernels_cover
+        if not fused:
+            gdn.chunk_kernels_cover = lambda *a: False
+        try:
+            n0 = _cuda.launch_count
+            out = gdn.chunk_gated_delta_rule_packed(*parts, gg, bb, list(lengths))
+            (out.float() * go.cuda().float()).sum().backward()
+            launched = _cuda.launch_count - n0
+        finally:
+            gdn.chunk_kernels_cover = keep
+        grads = [leaf.grad[:, i * heads * 128:(i + 1) * heads * 128].view(T, heads, 128) for i in range(3)] if strided else [t.grad for t in parts]
+        return launched, [out, *grads, gg.grad, bb.grad]
+
+    launched, got = run(True)
+    _, old = run(False)
+    assert launched == 6, "chunk, scan and output kernels in both directions"
+    tol = 1e-4 if dtype == torch.float32 else 2 ** -7
+    for name, a, o, b in zip(("out", "q", "k", "v", "g", "beta"), got, old, [want, *(r.grad for r in ref)]):
+        b = b.detach()
+        err = (a.detach().cpu().double() - b).norm() / b.norm().clamp_min(1e-30)
+        was = (o.detach().cpu().double() - b).norm() / b.norm().clamp_min(1e-30)
+        print(f"{name}: fused {err:.3e} framework ops {was:.3e}")
+        assert err < tol, name
+        assert err < 1.5 * was + 1e-6, f"{name}: {err} against {was}"
