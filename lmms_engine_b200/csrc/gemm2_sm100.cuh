@@ -279,11 +279,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
-            if (EPI == EPI_PLAIN && p.bias != nullptr) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
-            }
+            if (EPI == EPI_PLAIN && p.bias != nullptr) add_bias32(v, p.bias, col0, p.N);
             if ((EPI == EPI_PLAIN || EPI == EPI_SYMM) && p.cin != nullptr && row < p.M) {
               const __nv_bfloat16* crow = p.cin + static_cast<size_t>(row) * p.ldcin + col0;
               if (col0 + 32 <= p.N) {
@@ -368,10 +364,18 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tmem_ld_32x32b_x32(t_acc + c64 * 64 + h * 32, rg);
             tmem_ld_32x32b_x32(t_acc + 128 + c64 * 64 + h * 32, ru);
             tmem_ld_wait();
+            float vg[32], vu[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              vg[j] = __uint_as_float(rg[j]) * p.alpha;
+              vu[j] = __uint_as_float(ru[j]) * p.alpha;
+            }
+            if (p.bias != nullptr) add_bias32(vg, p.bias, n0 + c64 * 64 + h * 32, p.N);
+            if (p.bias2 != nullptr) add_bias32(vu, p.bias2, n0 + c64 * 64 + h * 32, p.N);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              pg[h][j] = pack_bf16x2(__uint_as_float(rg[2 * j]) * p.alpha, __uint_as_float(rg[2 * j + 1]) * p.alpha);
-              pu[h][j] = pack_bf16x2(__uint_as_float(ru[2 * j]) * p.alpha, __uint_as_float(ru[2 * j + 1]) * p.alpha);
+              pg[h][j] = pack_bf16x2(vg[2 * j], vg[2 * j + 1]);
+              pu[h][j] = pack_bf16x2(vu[2 * j], vu[2 * j + 1]);
               float2 g = unpack_bf16x2(pg[h][j]), u = unpack_bf16x2(pu[h][j]);
               phh[h][j] = pack_bf16x2(silu_f(g.x) * u.x, silu_f(g.y) * u.y);
             }

@@ -53,7 +53,8 @@ struct GemmParams {
   int a_mn_major, b_mn_major;
   int a_mn3d, b_mn3d;          // MN-major operand fetched with ONE 3-D TMA box (all 64-wide chunks at once)
   float alpha, beta;
-  const __nv_bfloat16* bias;   // [N] or null (PLAIN)
+  const __nv_bfloat16* bias;   // [N] or null (PLAIN; SWIGLU: of the gate half)
+  const __nv_bfloat16* bias2;  // SWIGLU: of the up half, or null
   const __nv_bfloat16* cin;    // [M, ldcin] or null (PLAIN / SYMM)
   int ldcin;
   float2* stats;               // [M, n_tiles] (STATS)
@@ -146,6 +147,25 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
+
+// v[j] += bias[col0 + j] for the columns below n.  Every lane reads the same 64 bytes, four 16-byte loads instead of 32
+// two-byte ones where the slice is whole and the pointer allows it (col0 is a multiple of 32).
+__device__ __forceinline__ void add_bias32(float (&v)[32], const __nv_bfloat16* bias, int col0, int n) {
+  if (col0 + 32 <= n && (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
+    const uint4* b4 = reinterpret_cast<const uint4*>(bias + col0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 b = __ldg(b4 + q);
+      const float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
+      v[q * 8 + 0] += f0.x; v[q * 8 + 1] += f0.y; v[q * 8 + 2] += f1.x; v[q * 8 + 3] += f1.y;
+      v[q * 8 + 4] += f2.x; v[q * 8 + 5] += f2.y; v[q * 8 + 6] += f3.x; v[q * 8 + 7] += f3.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (col0 + j < n) v[j] += __bfloat162float(bias[col0 + j]);
+  }
+}
 
 // Map a linear tile index to (m_block, n_block).  Sixteen m-blocks share each sweep
 // over N so that concurrently resident CTAs reuse the same B panels out of L2.
@@ -486,11 +506,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = empty_k ? 0.f : __uint_as_float(r[j]) * p.alpha;
-            if (EPI == EPI_PLAIN && p.bias != nullptr) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
-            }
+            if (EPI == EPI_PLAIN && p.bias != nullptr) add_bias32(v, p.bias, col0, p.N);
             if ((EPI == EPI_PLAIN || EPI == EPI_SYMM) && p.cin != nullptr && row < p.M) {
               const __nv_bfloat16* crow = p.cin + static_cast<size_t>(row) * p.ldcin + col0;
               if (col0 + 32 <= p.N) {
@@ -653,11 +669,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tmem_ld_32x32b_x32(t_acc + c64 * 64 + h * 32, rg);
             tmem_ld_32x32b_x32(t_acc + 128 + c64 * 64 + h * 32, ru);
             tmem_ld_wait();
+            float vg[32], vu[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              vg[j] = __uint_as_float(rg[j]) * p.alpha;
+              vu[j] = __uint_as_float(ru[j]) * p.alpha;
+            }
+            if (p.bias != nullptr) add_bias32(vg, p.bias, n0 + c64 * 64 + h * 32, p.N);
+            if (p.bias2 != nullptr) add_bias32(vu, p.bias2, n0 + c64 * 64 + h * 32, p.N);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               // round gate/up to bf16 first so that H matches silu(G)*U of the stored tensors
-              pg[h][j] = pack_bf16x2(__uint_as_float(rg[2 * j]) * p.alpha, __uint_as_float(rg[2 * j + 1]) * p.alpha);
-              pu[h][j] = pack_bf16x2(__uint_as_float(ru[2 * j]) * p.alpha, __uint_as_float(ru[2 * j + 1]) * p.alpha);
+              pg[h][j] = pack_bf16x2(vg[2 * j], vg[2 * j + 1]);
+              pu[h][j] = pack_bf16x2(vu[2 * j], vu[2 * j + 1]);
               float2 g = unpack_bf16x2(pg[h][j]), u = unpack_bf16x2(pu[h][j]);
               phh[h][j] = pack_bf16x2(silu_f(g.x) * u.x, silu_f(g.y) * u.y);
             }
@@ -1133,9 +1157,11 @@ int b200_gemm_comm_bf16(const void* A, const void* B, void* C, int M, int N, int
   return rc != 0 ? rc : launched;
 }
 
-// H = silu(X Wg^T) * (X Wu^T); optionally also writes G and U.  X [M,K], Wg/Wu [I,K].
+// H = silu(X Wg^T + bg) * (X Wu^T + bu); optionally also writes G and U.  X [M,K], Wg/Wu [I,K]; the biases [I] may be
+// null.  I may be any number: rows of H, G and U are ldh elements apart (a multiple of 8) and nothing is written past I.
 int b200_gemm_swiglu_bf16(const void* X, const void* Wg, const void* Wu, void* H, void* G, void* U, int M, int I,
-                          int K, int ldx, int ldw, int ldh, int store_gu, int* status, cudaStream_t stream) {
+                          int K, int ldx, int ldw, int ldh, int store_gu, const void* bg, const void* bu, int* status,
+                          cudaStream_t stream) {
   if (M <= 0 || I <= 0 || K <= 0) return 0;
   if ((ldx | ldw | ldh) & 7) return -10;
   CUtensorMap tA, tB, tB2, tC, tC2, tC3;
@@ -1154,6 +1180,8 @@ int b200_gemm_swiglu_bf16(const void* X, const void* Wg, const void* Wu, void* H
   p.n_tiles_m = pair ? (M + kTile2M - 1) / kTile2M : (M + BM - 1) / BM;
   p.n_tiles_n = (I + 127) / 128;
   p.store_gu = store_gu;
+  p.bias = static_cast<const __nv_bfloat16*>(bg);
+  p.bias2 = static_cast<const __nv_bfloat16*>(bu);
   p.status = status;
   if (pair) return launch2<EPI_SWIGLU>(tA, tB, tB2, tC, tC2, tC3, p, 0, stream);
   return launch<EPI_SWIGLU>(tA, tB, tB2, tC, tC2, tC3, p, 0, stream);

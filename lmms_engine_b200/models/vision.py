@@ -145,9 +145,8 @@ class GatedVisionMLP(nn.Module):
         self.down_proj = nn.Linear(inter, dim, bias=True)
 
     def forward(self, x):
-        g = gemm_ops.linear(x, self.gate_proj.weight, self.gate_proj.bias)
-        u = gemm_ops.linear(x, self.up_proj.weight, self.up_proj.bias)
-        return gemm_ops.linear(swiglu_ops.swiglu(g, u), self.down_proj.weight, self.down_proj.bias)
+        g, u, d = self.gate_proj, self.up_proj, self.down_proj
+        return swiglu_ops.gated_mlp(x, g.weight, g.bias, u.weight, u.bias, d.weight, d.bias)
 
 
 class PlainVisionMLP(nn.Module):

@@ -16,7 +16,7 @@ from .. import _native
 _SIG: Dict[str, Tuple[str, str]] = {
     # gemm_sm100
     "b200_gemm_bf16": ("gemm_sm100", "pppiiiiiiiiffppiiips"),
-    "b200_gemm_swiglu_bf16": ("gemm_sm100", "ppppppiiiiiiips"),
+    "b200_gemm_swiglu_bf16": ("gemm_sm100", "ppppppiiiiiiippps"),
     "b200_gemm_stats_bf16": ("gemm_sm100", "ppppiiiiiifps"),
     "b200_gemm_tile_n": ("gemm_sm100", ""),
     "b200_gemm_set_pair_mode": ("gemm_sm100", "i"),

@@ -103,21 +103,26 @@ def matmul_tn(dy: torch.Tensor, x: torch.Tensor, out=None, cin=None, beta: float
     return gemm(dy, x, a_mn_major=True, b_mn_major=True, out=out, cin=cin, beta=beta)
 
 
-def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, store_gu: bool = True):
-    """``h = silu(x wg^T) * (x wu^T)`` in one kernel; also returns gate/up when asked."""
+def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, store_gu: bool = True, bg: Optional[torch.Tensor] = None,
+                bu: Optional[torch.Tensor] = None):
+    """``h = silu(x wg^T + bg) * (x wu^T + bu)`` in one kernel; also returns gate/up when asked.  A width that is no multiple
+    of 8 gets rows padded to one: the results are views ``[M, width]`` of them, and nothing writes the padding."""
     if not (_ok(x) and _ok(wg) and _ok(wu)):
         raise TypeError("gemm_swiglu needs contiguous CUDA bf16 operands")
     M, K = x.shape
     inter = wg.shape[0]
-    h = torch.empty((M, inter), dtype=torch.bfloat16, device=x.device)
+    ld = (inter + 7) // 8 * 8
+    h = torch.empty((M, ld), dtype=torch.bfloat16, device=x.device)
     g = torch.empty_like(h) if store_gu else None
     u = torch.empty_like(h) if store_gu else None
     st = _cuda.status_word(x.device)
     _cuda.call(
         "b200_gemm_swiglu_bf16",
         x.data_ptr(), wg.data_ptr(), wu.data_ptr(), h.data_ptr(), _cuda.ptr(g), _cuda.ptr(u), M, inter, K,
-        x.stride(0), wg.stride(0), h.stride(0), int(store_gu), st.data_ptr(), _cuda.stream(),
+        x.stride(0), wg.stride(0), ld, int(store_gu), _cuda.ptr(bg), _cuda.ptr(bu), st.data_ptr(), _cuda.stream(),
     )
+    if ld != inter:
+        h, g, u = h[:, :inter], (g[:, :inter] if store_gu else None), (u[:, :inter] if store_gu else None)
     return h, g, u
 
 

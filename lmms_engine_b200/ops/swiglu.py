@@ -103,3 +103,82 @@ def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Te
         return _SwiGLUMLPFn.apply(x, wg, wu, wd)
     lin = torch.nn.functional.linear
     return lin(swiglu(lin(x, wg), lin(x, wu)), wd)
+
+
+class _GatedMLPFn(torch.autograd.Function):
+    """``swiglu_mlp`` with biases and an inner width that may be any number (3420 in the windowed vision tower): rows of the
+    inner activations are padded to 16 bytes, which is all that TMA needs, and the products stop at the true width."""
+
+    @staticmethod
+    def forward(ctx, x, wg, bg, wu, bu, wd, bd):
+        shp = x.shape
+        x2 = _rows16(x.reshape(-1, shp[-1]))
+        h, g, u = _gemm.gemm_swiglu(x2, wg, wu, True, bg, bu)
+        y = _gemm.gemm(h, _padded(wd), bias=bd)
+        ctx.save_for_backward(x2, wg, wu, wd, g, u)
+        ctx.shp, ctx.biases = shp, (bg is not None, bu is not None, bd is not None)
+        return y.view(*shp[:-1], wd.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, wg, wu, wd, g, u = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dy2 = _rows16(dy.reshape(-1, dy.shape[-1]))
+        M, inter = x2.shape[0], wg.shape[0]
+        ld = (inter + 7) // 8 * 8
+        # elementwise passes run over whole padded rows: the padding holds anything and is not read again
+        h, dg, du = (torch.empty((M, ld), dtype=g.dtype, device=g.device) for _ in range(3))
+        _cuda.call("b200_swiglu_fwd", g.data_ptr(), u.data_ptr(), h.data_ptr(), M * ld, _cuda.stream())
+        dwd = None
+        if need[5]:
+            dwd = torch.empty((wd.shape[0], ld), dtype=wd.dtype, device=wd.device)[:, :inter]
+            _gemm.matmul_tn(dy2, h[:, :inter], out=dwd)
+        _gemm.matmul_nn(dy2, _padded(wd), out=h[:, :inter])
+        _cuda.call("b200_swiglu_bwd", h.data_ptr(), g.data_ptr(), u.data_ptr(), dg.data_ptr(), du.data_ptr(), M * ld, _cuda.stream())
+        dg, du = dg[:, :inter], du[:, :inter]
+        dx = None
+        if need[0]:
+            dx = _gemm.matmul_nn(dg, wg)
+            dx = _gemm.gemm(du, wu, b_mn_major=True, cin=dx, beta=1.0, out=dx).view(ctx.shp)
+        dwg = _gemm.matmul_tn(dg, x2) if need[1] else None
+        dwu = _gemm.matmul_tn(du, x2) if need[3] else None
+        has_g, has_u, has_d = ctx.biases
+        return (dx, dwg, _column_sum(dg) if has_g and need[2] else None, dwu, _column_sum(du) if has_u and need[4] else None, dwd,
+                _column_sum(dy2) if has_d and need[6] else None)
+
+
+def _rows16(t):
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _column_sum(t):
+    return t.sum(0, dtype=torch.float32).to(t.dtype)
+
+
+def _padded(wd):
+    """The down projection with rows on 16-byte boundaries (one copy of the weight where its width is not a multiple of 8);
+    the padding lies outside every tensor map."""
+    n, i = wd.shape
+    if i % 8 == 0:
+        return wd
+    return torch.empty((n, (i + 7) // 8 * 8), dtype=wd.dtype, device=wd.device)[:, :i].copy_(wd)
+
+
+def gated_mlp(x, wg, bg, wu, bu, wd, bd) -> torch.Tensor:
+    """``(silu(x wg^T + bg) * (x wu^T + bu)) wd^T + bd``; any of the biases may be ``None``.
+
+    One fused function for every width: as three linears, an inner width that is no multiple of 8 went to the library's
+    unaligned kernels (49 of the 94 device ms of an eight-block tower with 3420 over 21.9k patches, forward + backward)."""
+    plain = (torch.Tensor, torch.nn.Parameter)
+    native = (
+        _gemm.LINEAR_BACKEND == "tcgen05" and x.is_cuda and x.dtype == torch.bfloat16 and x.numel() > 0 and wg.shape == wu.shape
+        and x.shape[-1] % 8 == 0 and wd.shape[0] % 8 == 0 and wd.shape[1] == wg.shape[0]
+        and all(type(w) in plain and w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0
+                for w in (wg, wu, wd))
+        and all(b is None or (type(b) in plain and b.is_cuda and b.dtype == torch.bfloat16 and b.is_contiguous())
+                for b in (bg, bu, bd))
+    )
+    if native:
+        return _GatedMLPFn.apply(x, wg, bg, wu, bu, wd, bd)
+    g, u = _gemm.linear(x, wg, bg), _gemm.linear(x, wu, bu)
+    return _gemm.linear(swiglu(g, u), wd, bd)

@@ -145,3 +145,34 @@ def test_few_rows(M, N, K):
         y = gemm.matmul_nt(x, w, bias)
         _cuda.check_status()
         assert ((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4 * K ** 0.5).all()
+
+
+@pytest.mark.parametrize("P,K,inter,N,biases", [(1, 64, 36, 64, True), (65, 72, 100, 136, True), (300, 128, 130, 64, False),
+                                               (257, 1280, 3420, 1280, True), (129, 64, 3, 8, True)])
+def test_gated_mlp_any_width(P, K, inter, N, biases):
+    """Inner widths that are no multiple of 8 (rows padded to 16 bytes, products stop at the true width): against fp32
+    linears.  Two bf16 roundings between the products and one of the result: 2^-6 of the 2-norm bounds them."""
+    from lmms_engine_b200.ops import swiglu
+
+    torch.manual_seed(0)
+    shapes = [(P, K), (inter, K), (inter,), (inter, K), (inter,), (N, inter), (N,)]
+    raw = [torch.randn(s) * (1.0 if i == 0 else K ** -0.5 if i < 5 else inter ** -0.5) for i, s in enumerate(shapes)]
+    raw = [t.bfloat16() for t in raw]
+    if not biases:
+        raw[2] = raw[4] = raw[6] = None
+    ref = [None if t is None else t.float().requires_grad_() for t in raw]
+    F = torch.nn.functional
+    want = F.linear(F.silu(F.linear(ref[0], ref[1], ref[2])) * F.linear(ref[0], ref[3], ref[4]), ref[5], ref[6])
+    dy = torch.randn(P, N).bfloat16()
+    want.backward(dy.float())
+    dev = [None if t is None else t.cuda().requires_grad_() for t in raw]
+    got = swiglu.gated_mlp(*dev)
+    got.backward(dy.cuda(), retain_graph=True)
+    first = [None if t is None else t.grad.clone() for t in dev]
+    for a, b in [(got.detach(), want.detach())] + [(f, r.grad) for f, r in zip(first, ref) if r is not None]:
+        assert torch.isfinite(a).all()
+        assert (a.float().cpu() - b).norm() < 2 ** -6 * b.norm() + 1e-6
+    got.backward(dy.cuda())  # the saved activations are not overwritten: a second pass adds the same gradients
+    for t, f in zip(dev, first):
+        if t is not None:
+            assert torch.equal(t.grad, f + f)
