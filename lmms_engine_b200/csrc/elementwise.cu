@@ -410,11 +410,34 @@ __global__ void rope_table_kernel(const int64_t* __restrict__ pos, const float* 
 // x: [T, Hn, D] (row stride ldx elements between tokens), rotate-half convention:
 // y[:half] = x1*c1 - x2*s1 ; y[half:] = x2*c2 + x1*s2.  `conj` applies the transpose
 // (backward).  rot_dim <= D: dims beyond rot_dim are copied.
+// W pairs per thread: 8 where the second half starts on a 16-byte boundary (rot_dim a multiple of 16), else 4 (heads of 72:
+// the second half starts on an 8-byte one).  Bound by memory either way; a head of 72 through framework operations took
+// eight passes in fp32.
+template <int W>
+__device__ __forceinline__ void load_w(const bf16* p, float (&v)[W]);
+template <>
+__device__ __forceinline__ void load_w<8>(const bf16* p, float (&v)[8]) { load8(p, v); }
+template <>
+__device__ __forceinline__ void load_w<4>(const bf16* p, float (&v)[4]) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+template <int W>
+__device__ __forceinline__ void store_w(bf16* p, const float (&v)[W]);
+template <>
+__device__ __forceinline__ void store_w<8>(bf16* p, const float (&v)[8]) { store8(p, v); }
+template <>
+__device__ __forceinline__ void store_w<4>(bf16* p, const float (&v)[4]) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+}
+
+template <int W>
 __global__ void rope_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ cosb,
                                   const float* __restrict__ sinb, int T, int Hn, int D, int rot_dim, long ldx,
                                   long ldy, int conj) {
   const int half = rot_dim / 2;
-  const int per_head = half / 8;  // vectors of 8 pairs
+  const int per_head = half / W;  // vectors of W pairs
   const long total = static_cast<long>(T) * Hn * per_head;
   for (long idx = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -424,15 +447,15 @@ __global__ void rope_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__
     const long t = th / Hn;
     const bf16* xp = x + t * ldx + static_cast<long>(h) * D;
     bf16* yp = y + t * ldy + static_cast<long>(h) * D;
-    float x1[8], x2[8], o1[8], o2[8];
-    load8(xp + v * 8, x1);
-    load8(xp + half + v * 8, x2);
+    float x1[W], x2[W], o1[W], o2[W];
+    load_w<W>(xp + v * W, x1);
+    load_w<W>(xp + half + v * W, x2);
     const float* c = cosb + t * rot_dim;
     const float* s = sinb + t * rot_dim;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float c1 = c[v * 8 + j], c2 = c[half + v * 8 + j];
-      const float s1 = s[v * 8 + j], s2 = s[half + v * 8 + j];
+    for (int j = 0; j < W; ++j) {
+      const float c1 = c[v * W + j], c2 = c[half + v * W + j];
+      const float s1 = s[v * W + j], s2 = s[half + v * W + j];
       if (!conj) {
         o1[j] = x1[j] * c1 - x2[j] * s1;
         o2[j] = x2[j] * c2 + x1[j] * s2;
@@ -441,8 +464,8 @@ __global__ void rope_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__
         o2[j] = x2[j] * c2 - x1[j] * s1;
       }
     }
-    store8(yp + v * 8, o1);
-    store8(yp + half + v * 8, o2);
+    store_w<W>(yp + v * W, o1);
+    store_w<W>(yp + half + v * W, o2);
   }
 }
 
@@ -946,10 +969,16 @@ int b200_rope_table(const void* pos, const void* inv_freq, void* cos_out, void* 
 int b200_rope_apply(const void* x, void* y, const void* cosb, const void* sinb, int T, int Hn, int D, int rot_dim,
                     long ldx, long ldy, int conj, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (rot_dim % 16 || D % 8 || ldx % 8 || ldy % 8) return -10;
-  long total = static_cast<long>(T) * Hn * (rot_dim / 16);
-  rope_apply_kernel<<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x, (bf16*)y, (const float*)cosb,
-                                                          (const float*)sinb, T, Hn, D, rot_dim, ldx, ldy, conj);
+  if (rot_dim % 8 || D % 8 || ldx % 8 || ldy % 8) return -10;
+  if (rot_dim % 16 == 0) {
+    const long total = static_cast<long>(T) * Hn * (rot_dim / 16);
+    rope_apply_kernel<8><<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x, (bf16*)y, (const float*)cosb, (const float*)sinb, T, Hn, D,
+                                                               rot_dim, ldx, ldy, conj);
+  } else {
+    const long total = static_cast<long>(T) * Hn * (rot_dim / 8);
+    rope_apply_kernel<4><<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x, (bf16*)y, (const float*)cosb, (const float*)sinb, T, Hn, D,
+                                                               rot_dim, ldx, ldy, conj);
+  }
   return CHECK_LAUNCH();
 }
 

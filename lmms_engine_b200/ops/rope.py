@@ -78,8 +78,8 @@ def rope_apply_ref(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, conj: 
 
 def _apply_native(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, conj: bool, inplace: bool) -> torch.Tensor:
     T, Hn, D = x.shape
-    if x.stride(2) != 1 or x.stride(1) != D:
-        x = x.contiguous()
+    if x.stride(2) != 1 or x.stride(1) != D or x.stride(0) % 8 or x.data_ptr() % 16:
+        x = x.clone(memory_format=torch.contiguous_format)
         inplace = True  # the contiguous copy is ours
     rot = cos.shape[-1]
     y = x if inplace else torch.empty((T, Hn, D), dtype=x.dtype, device=x.device)
@@ -106,6 +106,10 @@ class _RopeFn(torch.autograd.Function):
 
 def rope_apply(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """Rotate ``x [T, H, D]`` by the per-token table; differentiable."""
+    if (x.is_cuda and x.dtype == torch.bfloat16 and cos.shape[-1] % 16 == 8 and x.shape[-1] % 8 == 0 and x.dim() == 3
+            and cos.shape[-1] <= x.shape[-1] and cos.shape == sin.shape == (x.shape[0], cos.shape[-1]) and cos.is_cuda and sin.is_cuda
+            and cos.dtype == sin.dtype == torch.float32 and not (cos.requires_grad or sin.requires_grad)):
+        return _RopeFn.apply(x, cos.contiguous(), sin.contiguous())  # any other table of such a width takes the form below
     if x.is_cuda and x.dtype == torch.bfloat16 and cos.shape[-1] % 16 == 0 and x.shape[-1] % 8 == 0:
         if cos.dtype != torch.float32 or sin.dtype != torch.float32:
             # the kernel reads the tables as fp32; a table that some wrapper cast down would be read past its end

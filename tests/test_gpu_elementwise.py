@@ -352,3 +352,25 @@ def test_newton_schulz_graph_owns_every_buffer_it_writes():
     muon.orthogonalize(x, 5, work)
     torch.cuda.synchronize()
     assert all(bool((t == 3.0).all()) for t in later)
+
+
+@pytest.mark.parametrize("T,H,D,rot", [(5, 3, 72, 72), (130, 16, 72, 72), (7, 2, 80, 40), (3, 1, 8, 8)])
+def test_rope_in_fours(T, H, D, rot):
+    """Rotation widths whose second half starts on an 8-byte boundary: the fp32 arithmetic of the framework form and one
+    rounding, so at most one bf16 step apart (near zero: a rounding of the fp32 terms, which are below 8)."""
+    from lmms_engine_b200.ops import _cuda, rope
+
+    torch.manual_seed(0)
+    base = torch.randn(T, 3 * H * D, device="cuda", dtype=torch.bfloat16)
+    ang = torch.randn(T, rot // 2, device="cuda").repeat(1, 2)
+    dy = torch.randn(T, H, D, device="cuda", dtype=torch.bfloat16)
+    x = base.view(T, 3, H, D)[:, 1].detach().requires_grad_()
+    y = base.view(T, 3, H, D)[:, 1].detach().clone().requires_grad_()
+    n0 = _cuda.launch_count
+    a = rope.rope_apply(x, ang.cos(), ang.sin())
+    assert _cuda.launch_count > n0
+    b = rope.rope_apply_ref(y, ang.cos(), ang.sin())
+    a.backward(dy)
+    b.backward(dy)
+    for u, v in ((a.detach(), b.detach()), (x.grad, y.grad)):
+        assert torch.allclose(u.float(), v.float(), rtol=2 ** -7, atol=2 ** -20)
