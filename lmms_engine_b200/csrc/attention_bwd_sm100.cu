@@ -76,31 +76,6 @@ __device__ __forceinline__ uint64_t desc_lbo(uint32_t addr, uint32_t lbo_bytes) 
   return (d & ~(uint64_t(0x3FFF) << 16)) | (uint64_t(lbo_bytes >> 4) << 16);
 }
 
-__device__ __forceinline__ bool find_work(const int* cu_a, const int* cu_b, int n_docs, int block, int item,
-                                          int* work, int total_a, int total_b, int* status) {
-  // work: doc, a0 (offset of the 128-block inside the doc), len_a, len_b, a_start, b_start
-  int acc = 0;
-  for (int d = 0; d < n_docs; ++d) {
-    const int la = cu_a[d + 1] - cu_a[d];
-    const int nb = (la + block - 1) / block;
-    if (item < acc + nb) {
-      work[0] = d;
-      work[1] = (item - acc) * block;
-      work[2] = la;
-      work[3] = cu_b[d + 1] - cu_b[d];
-      work[4] = cu_a[d];
-      work[5] = cu_b[d];
-      if (!doc_in_bounds(work[4], work[2], total_a, status) || !doc_in_bounds(work[5], work[3], total_b, status)) {
-        work[0] = -1;
-        return false;
-      }
-      return true;
-    }
-    acc += nb;
-  }
-  return false;
-}
-
 // ============================================================================ dK / dV
 __global__ void __launch_bounds__(384, 1)
 attn_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -121,9 +96,8 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   int* work = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    work[0] = -1;
-    find_work(p.cu_k, p.cu_q, p.n_docs, kKeys, blockIdx.x, work, p.Tk, p.Tq, p.status);
+  if (warp == 0) find_block(p.cu_k, p.cu_q, p.n_docs, kKeys, blockIdx.x, false, p.Tk, p.Tq, work, p.status);
+  if (threadIdx.x == 32) {
     mbar_init(kv_full, 1);
     for (int i = 0; i < S; ++i) {
       mbar_init(&q_full[i], 1);
@@ -424,13 +398,8 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   int* work = reinterpret_cast<int*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    // heavy (late, long-context) query blocks first
-    int total = 0;
-    for (int d = 0; d < p.n_docs; ++d) total += (p.cu_q[d + 1] - p.cu_q[d] + kKeys - 1) / kKeys;
-    work[0] = -1;
-    const int item = total - 1 - static_cast<int>(blockIdx.x);
-    if (item >= 0) find_work(p.cu_q, p.cu_k, p.n_docs, kKeys, item, work, p.Tq, p.Tk, p.status);
+  if (warp == 0) find_block(p.cu_q, p.cu_k, p.n_docs, kKeys, blockIdx.x, true, p.Tq, p.Tk, work, p.status);  // heavy blocks first
+  if (threadIdx.x == 32) {
     mbar_init(q_full, 1);
     for (int i = 0; i < S; ++i) {
       mbar_init(&kv_full[i], 1);

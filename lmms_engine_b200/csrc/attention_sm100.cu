@@ -95,29 +95,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // ---- decode the work item: heavy (late) query blocks are scheduled first ------------
-  if (threadIdx.x == 0) {
-    int total = 0;
-    for (int d = 0; d < p.n_docs; ++d) total += (p.cu_q[d + 1] - p.cu_q[d] + kBlockQ - 1) / kBlockQ;
-    int item = total - 1 - static_cast<int>(blockIdx.x);
-    work[0] = -1;
-    if (item >= 0) {
-      int acc = 0;
-      for (int d = 0; d < p.n_docs; ++d) {
-        const int lq = p.cu_q[d + 1] - p.cu_q[d];
-        const int nb = (lq + kBlockQ - 1) / kBlockQ;
-        if (item < acc + nb) {
-          work[0] = d;
-          work[1] = (item - acc) * kBlockQ;
-          work[2] = lq;
-          work[3] = p.cu_k[d + 1] - p.cu_k[d];
-          work[4] = p.cu_q[d];
-          work[5] = p.cu_k[d];
-          if (!doc_in_bounds(work[4], work[2], p.Tq, p.status) || !doc_in_bounds(work[5], work[3], p.Tk, p.status)) work[0] = -1;
-          break;
-        }
-        acc += nb;
-      }
-    }
+  if (warp == 0) find_block(p.cu_q, p.cu_k, p.n_docs, kBlockQ, blockIdx.x, true, p.Tq, p.Tk, work, p.status);
+  if (threadIdx.x == 32) {
     mbar_init(q_full, 1);
     for (int i = 0; i < S; ++i) {
       mbar_init(&k_full[i], 1);

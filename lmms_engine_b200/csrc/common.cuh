@@ -275,6 +275,47 @@ __device__ __forceinline__ bool doc_in_bounds(int start, int len, int total, int
   return false;
 }
 
+// Block `item` of a packed stream whose documents (boundaries cu_a) are cut into blocks of `block` rows, counted over the
+// documents in order or, with `from_end`, backwards from the last block of the last document.  One whole warp calls it;
+// work[0..5] = document, first row of the block inside it, its length in a and in b, its start in a and in b, or work[0] = -1
+// when the stream has fewer blocks.  Thirty-two documents per step: a CTA of a small document lasts a few microseconds, and
+// walking 48 to 370 boundaries with one thread cost as much again.
+__device__ __forceinline__ void find_block(const int* cu_a, const int* cu_b, int n_docs, int block, int item, bool from_end,
+                                           int total_a, int total_b, int* work, int* status) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) work[0] = -1;
+  __syncwarp();
+  for (int base = 0; base < n_docs; base += 32) {
+    const int i = base + lane;
+    const int d = from_end ? n_docs - 1 - i : i;
+    int lo = 0, len = 0;
+    if (i < n_docs) {
+      lo = cu_a[d];
+      len = cu_a[d + 1] - lo;
+    }
+    const int nb = len > 0 ? (len + block - 1) / block : 0;
+    int sum = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+    }
+    const bool here = item >= sum - nb && item < sum;
+    if (here) {
+      const int b = item - (sum - nb);
+      work[1] = (from_end ? nb - 1 - b : b) * block;
+      work[2] = len;
+      work[4] = lo;
+      work[5] = cu_b[d];
+      work[3] = cu_b[d + 1] - work[5];
+      const bool ok = doc_in_bounds(lo, len, total_a, status) && doc_in_bounds(work[5], work[3], total_b, status);
+      work[0] = ok ? d : -1;
+    }
+    if (__any_sync(0xffffffffu, here)) return;
+    item -= __shfl_sync(0xffffffffu, sum, 31);
+  }
+}
+
 // ---------------------------------------------------------------- index bounds
 // Rows addressed through an index table (routing tables, gather / scatter maps) are checked against the tensor they
 // index: an index past the end raises kStatusBadIndex and the access is skipped.  The check is one compare per row and
