@@ -161,6 +161,12 @@ class Attention(nn.Module):
                     # rank's heads; the row-parallel output projection below reduce-scatters back
                     x = tp_ops.all_gather_tokens(x, ctx.tp_group)
                 qkv = gemm_ops.linear(x, w, b)
+            if not (self.cfg.qk_norm or ctx.sp_size > 1 or ctx.tp_size > 1 or getattr(self, "nsa", None) is not None
+                    or getattr(ctx, "kv_cache", None) is not None):
+                o = attn_ops.rope_attention(qkv, ctx.cos, ctx.sin, ctx.cu_seqlens, self.n_q, self.n_kv, D, ctx.causal,
+                                            1.0 / math.sqrt(D), self.window[0])
+                if o is not None:
+                    return gemm_ops.linear(o.reshape(o.shape[0], -1), _w(self.o_proj.weight), None)
             T = qkv.shape[0]
             q = qkv[:, :nq].view(T, self.n_q, D)
             k = qkv[:, nq : nq + nkv].view(T, self.n_kv, D)

@@ -125,9 +125,15 @@ class VisionAttention(nn.Module):
         self.qkv = nn.Linear(dim, dim * 3, bias=True)
         self.proj = nn.Linear(dim, dim, bias=True)
 
-    def forward(self, x, cu, cos, sin):
+    def forward(self, x, cu, cos, sin, max_len=None):
+        """``max_len``: longest span of ``cu``, where the caller knows it."""
         P = x.shape[0]
-        qkv = gemm_ops.linear(x, self.qkv.weight, self.qkv.bias).view(P, 3, self.heads, self.head_dim)
+        qkv = gemm_ops.linear(x, self.qkv.weight, self.qkv.bias)
+        o = attn_ops.rope_attention(qkv, cos, sin, cu, self.heads, self.heads, self.head_dim, False, 1.0 / math.sqrt(self.head_dim),
+                                    max_len=max_len)
+        if o is not None:
+            return gemm_ops.linear(o.reshape(P, -1), self.proj.weight, self.proj.bias)
+        qkv = qkv.view(P, 3, self.heads, self.head_dim)
         q, k, v = qkv[:, 0], qkv[:, 1], qkv[:, 2]
         q = rope_ops.rope_apply(q, cos, sin)
         k = rope_ops.rope_apply(k, cos, sin)
@@ -184,8 +190,8 @@ class VisionBlock(nn.Module):
         self.mlp = (GatedVisionMLP(cfg.hidden_size, cfg.intermediate_size) if gated
                     else PlainVisionMLP(cfg.hidden_size, cfg.intermediate_size, cfg.hidden_act))
 
-    def forward(self, x, cu, cos, sin):
-        x = x + self.attn(self.norm1(x), cu, cos, sin)
+    def forward(self, x, cu, cos, sin, max_len=None):
+        x = x + self.attn(self.norm1(x), cu, cos, sin, max_len)
         return x + self.mlp(self.norm2(x))
 
 
@@ -280,12 +286,13 @@ class Qwen25VisionTower(_TowerBase):
         P = x.shape[0]
         x = x.view(P // unit, unit, -1).index_select(0, order_t).reshape(P, -1)
         full = set(cfg.fullatt_block_indexes)
+        longest = int(np.diff(cu_win).max(initial=0))
         for i, blk in enumerate(self.blocks):
-            cu = cu_full if i in full else cu_win_t
+            cu, max_len = (cu_full, None) if i in full else (cu_win_t, longest)
             if self.gradient_checkpointing and self.training:
-                x = torch.utils.checkpoint.checkpoint(blk, x, cu, cos, sin, use_reentrant=False)
+                x = torch.utils.checkpoint.checkpoint(blk, x, cu, cos, sin, max_len, use_reentrant=False)
             else:
-                x = blk(x, cu, cos, sin)
+                x = blk(x, cu, cos, sin, max_len)
         merged = self.merger(x)
         inverse = torch.from_numpy(np.argsort(order)).to(dev, non_blocking=True)
         return merged.index_select(0, inverse)

@@ -18,6 +18,8 @@ from . import _cuda
 
 _cuda.register("b200_attn_fwd", "attention_sm100", "ppppppp" + "iiiiii" + "llll" + "fii" + "ps")
 _cuda.register("b200_attn_bwd", "attention_sm100", "ppppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
+_cuda.register("b200_attn_small_fwd", "attention_small", "ppppppp" + "iiiiii" + "llll" + "fii" + "ps")
+_cuda.register("b200_attn_small_bwd", "attention_small", "ppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
 _cuda.register("b200_attn_bwd_v2", "attention_bwd_sm100", "pppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
 
 # "split": dK/dV and dQ in two reduction-free kernels (default); "fused": the single-kernel
@@ -58,22 +60,61 @@ def _token_stride_ok(t: torch.Tensor) -> bool:
     return t.stride(2) == 1 and t.stride(1) == t.shape[2] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
 
 
+# Longest document of the one-CTA-per-document kernels (csrc/attention_small.cu).  They need the caller's word that no
+# document is longer, so only callers that build the boundaries on the host from the lengths themselves pass ``max_len``.
+# The line lies at the tile: a longer document would need a loop over keys, which the tcgen05 kernels do better.
+SMALL_DOC = 64
+
+
+def _fwd(q, k, v, cu_q, cu_k, causal, scale, window_left, small=False):
+    Tq, Hq, D = q.shape
+    Tk, Hkv, _ = k.shape
+    o = torch.empty((Tq, Hq, D), dtype=q.dtype, device=q.device)
+    lse = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device)
+    st = _cuda.status_word(q.device)
+    _cuda.call(
+        "b200_attn_small_fwd" if small else "b200_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
+        lse.data_ptr(), cu_q.data_ptr(), cu_k.data_ptr(), cu_q.numel() - 1, Tq, Tk, Hq, Hkv, D, q.stride(0), k.stride(0),
+        v.stride(0), o.stride(0), float(scale), int(causal), int(window_left), st.data_ptr(), _cuda.stream(),
+    )
+    return o, lse
+
+
+def _bwd(q, k, v, o, lse, do, cu_q, cu_k, causal, scale, window_left, dq, dk, dv, small=False):
+    """Writes the gradients into ``dq, dk, dv`` (rows of contiguous heads at any 16-byte row stride)."""
+    do = do if _token_stride_ok(do) else do.clone(memory_format=torch.contiguous_format)
+    Tq, Hq, D = q.shape
+    Tk, Hkv, _ = k.shape
+    st = _cuda.status_word(q.device)
+    # the single-kernel variant converts its fp32 accumulator into a dense dq
+    out_q = dq if BACKWARD_IMPL == "split" or small or dq.is_contiguous() else torch.empty((Tq, Hq, D), dtype=q.dtype, device=q.device)
+    strides = (q.stride(0), k.stride(0), v.stride(0), o.stride(0), do.stride(0), out_q.stride(0), dk.stride(0), dv.stride(0))
+    tail = (cu_q.data_ptr(), cu_k.data_ptr(), cu_q.numel() - 1, Tq, Tk, Hq, Hkv, D, *strides, float(scale), int(causal),
+            int(window_left), st.data_ptr(), _cuda.stream())
+    if small:
+        _cuda.call("b200_attn_small_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                   dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *tail)
+        return
+    delta = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device)
+    if BACKWARD_IMPL == "split":
+        # two reduction-free kernels (dK/dV per key block, dQ per query block)
+        _cuda.call("b200_attn_bwd_v2", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                   delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *tail)
+        return
+    dq_acc = torch.empty((Tq, Hq, D), dtype=torch.float32, device=q.device)
+    _cuda.call("b200_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+               delta.data_ptr(), dq_acc.data_ptr(), out_q.data_ptr(), dk.data_ptr(), dv.data_ptr(), *tail)
+    if out_q is not dq:
+        dq.copy_(out_q)
+
+
 class _VarlenAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_q, cu_k, causal, scale, window_left):
         q = q if _token_stride_ok(q) else q.contiguous()
         k = k if _token_stride_ok(k) else k.contiguous()
         v = v if _token_stride_ok(v) else v.contiguous()
-        Tq, Hq, D = q.shape
-        Tk, Hkv, _ = k.shape
-        o = torch.empty((Tq, Hq, D), dtype=q.dtype, device=q.device)
-        lse = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device)
-        st = _cuda.status_word(q.device)
-        _cuda.call(
-            "b200_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), cu_q.data_ptr(),
-            cu_k.data_ptr(), cu_q.numel() - 1, Tq, Tk, Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
-            float(scale), int(causal), int(window_left), st.data_ptr(), _cuda.stream(),
-        )
+        o, lse = _fwd(q, k, v, cu_q, cu_k, causal, scale, window_left)
         ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k)
         ctx.cfg = (causal, scale, window_left)
         return o
@@ -81,34 +122,62 @@ class _VarlenAttnFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, o, lse, cu_q, cu_k = ctx.saved_tensors
-        causal, scale, window_left = ctx.cfg
-        do = do if _token_stride_ok(do) else do.contiguous()
-        Tq, Hq, D = q.shape
-        Tk, Hkv, _ = k.shape
-        dq = torch.empty((Tq, Hq, D), dtype=q.dtype, device=q.device)
-        dk = torch.empty((Tk, Hkv, D), dtype=q.dtype, device=q.device)
-        dv = torch.empty((Tk, Hkv, D), dtype=q.dtype, device=q.device)
-        delta = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device)
-        st = _cuda.status_word(q.device)
-        if BACKWARD_IMPL == "split":
-            # two reduction-free kernels (dK/dV per key block, dQ per query block)
-            _cuda.call(
-                "b200_attn_bwd_v2", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(),
-                lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu_q.data_ptr(),
-                cu_k.data_ptr(), cu_q.numel() - 1, Tq, Tk, Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0),
-                o.stride(0), do.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), float(scale), int(causal),
-                int(window_left), st.data_ptr(), _cuda.stream(),
-            )
-            return dq, dk, dv, None, None, None, None, None
-        dq_acc = torch.empty((Tq, Hq, D), dtype=torch.float32, device=q.device)
-        _cuda.call(
-            "b200_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-            delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu_q.data_ptr(),
-            cu_k.data_ptr(), cu_q.numel() - 1, Tq, Tk, Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
-            do.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), float(scale), int(causal), int(window_left),
-            st.data_ptr(), _cuda.stream(),
-        )
+        dq, dk, dv = (torch.empty(t.shape, dtype=q.dtype, device=q.device) for t in (q, k, v))
+        _bwd(q, k, v, o, lse, do, cu_q, cu_k, *ctx.cfg, dq, dk, dv)
         return dq, dk, dv, None, None, None, None, None
+
+
+class _RopeAttnFn(torch.autograd.Function):
+    """Rotary embedding + attention on the rows of ONE projection ``[T, (n_q + 2 n_kv) * D]`` (heads of q, then k, then v).
+
+    As separate operations on slices of the projection, the backward pass builds three zero-filled gradients of its whole
+    size and adds them (five passes over it, twice that for a 3-way view); here the attention backward writes its three
+    gradients into the rows of one buffer and the rotation runs in place on the q and k part.  Query and key heads are
+    neighbours in a row, so both are rotated by one launch."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, cu, n_q, n_kv, D, causal, scale, window_left, small):
+        T = qkv.shape[0]
+        rot = torch.empty((T, n_q + n_kv, D), dtype=qkv.dtype, device=qkv.device)
+        _rotate(qkv, qkv.stride(0), rot, cos, sin, n_q + n_kv, D, False)
+        v = qkv[:, (n_q + n_kv) * D:].view(T, n_kv, D)
+        o, lse = _fwd(rot[:, :n_q], rot[:, n_q:], v, cu, cu, causal, scale, window_left, small)
+        ctx.save_for_backward(rot, v, o, lse, cu, cos, sin)
+        ctx.cfg = (causal, scale, window_left)
+        ctx.dims = (n_q, n_kv, D, small)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        rot, v, o, lse, cu, cos, sin = ctx.saved_tensors
+        n_q, n_kv, D, small = ctx.dims
+        T = rot.shape[0]
+        d = torch.empty((T, n_q + 2 * n_kv, D), dtype=rot.dtype, device=rot.device)
+        _bwd(rot[:, :n_q], rot[:, n_q:], v, o, lse, do, cu, cu, *ctx.cfg, d[:, :n_q], d[:, n_q:n_q + n_kv], d[:, n_q + n_kv:], small)
+        _rotate(d, d.stride(0), d, cos, sin, n_q + n_kv, D, True)
+        return (d.view(T, -1),) + (None,) * 10
+
+
+def _rotate(x, ldx, y, cos, sin, heads, D, conj):
+    _cuda.call("b200_rope_apply", x.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), y.shape[0], heads, D, D, ldx, y.stride(0),
+               int(conj), _cuda.stream())
+
+
+def rope_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, cu_seqlens: torch.Tensor, n_q: int, n_kv: int, D: int,
+                   causal: bool, softmax_scale: float, window_left: int = -1, max_len: Optional[int] = None) -> Optional[torch.Tensor]:
+    """Rotary embedding over whole heads, then attention, from one projection's rows; ``None`` where the fused form does not
+    apply (other dtypes, partial rotation, rows off 16-byte boundaries) and the caller runs the operations one by one.
+    ``max_len``: no document is longer, from a caller that made the boundaries; ``None`` where it is not known."""
+    ok = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and qkv.shape[1] == (n_q + 2 * n_kv) * D
+          and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and D % 8 == 0 and D <= 128
+          and n_q % n_kv == 0 and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
+          and cos.shape == sin.shape == (qkv.shape[0], D) and not (cos.requires_grad or sin.requires_grad))
+    if not ok:
+        return None
+    cu = cu_seqlens.to(torch.int32).contiguous()
+    small = max_len is not None and max_len <= SMALL_DOC and cu.numel() <= 65536
+    return _RopeAttnFn.apply(qkv, cos.contiguous(), sin.contiguous(), cu, n_q, n_kv, D, bool(causal), float(softmax_scale), int(window_left),
+                             small)
 
 
 def varlen_attn(

@@ -114,3 +114,46 @@ def test_queries_shorter_than_keys_bottom_right_aligned(causal):
     for name, a, b in (("dq", q.grad, qr.grad), ("dk", k.grad, kr.grad), ("dv", v.grad, vr.grad)):
         err = (a.float() - b).abs().max().item() / (b.abs().max().item() + 1e-6)
         assert err < 3e-2, (name, err)
+
+
+@pytest.mark.parametrize("lens,n_q,n_kv,D,causal,window,max_len", [
+    ((64, 1, 17, 63, 48, 16), 3, 3, 80, False, -1, 64),      # windows of a vision tower, ragged edges
+    ((33, 64, 5), 4, 2, 72, True, -1, 64),                   # grouped heads, a head of 72 (rotation in fours), causal
+    ((64, 64, 31), 4, 1, 128, True, 9, 64),
+    ((2, 64), 2, 2, 64, False, -1, 64),
+    ((130, 1, 127, 257), 4, 2, 80, False, -1, None),         # the long-document kernels behind the same entry
+    ((40,) * 70 + (200,), 2, 1, 128, True, -1, None),        # more documents than one step of the block search
+])
+def test_rope_attention_matches_separate_operations(lens, n_q, n_kv, D, causal, window, max_len):
+    """Against the fp32 formulation of both operations.  Outputs and gradients carry four bf16 roundings of 2^-9 each on
+    the way (rotated rows, probabilities, score gradients, the result), so 2^-6 of the 2-norm bounds them."""
+    from lmms_engine_b200.ops import _cuda, attention, rope
+
+    torch.manual_seed(3)
+    T = sum(lens)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * D).bfloat16()
+    ang = torch.randn(T, D // 2).repeat(1, 2)
+    cos, sin, do = ang.cos(), ang.sin(), torch.randn(T, n_q, D).bfloat16()
+    ref = qkv.float().requires_grad_()
+    q, k, v = ref.view(T, -1, D).split([n_q, n_kv, n_kv], 1)
+    want = attention.varlen_attn_ref(rope.rope_apply_ref(q, cos, sin), rope.rope_apply_ref(k, cos, sin), v, cu, cu, causal, D ** -0.5, window)
+    want.backward(do.float())
+    x = qkv.cuda().requires_grad_()
+    got = attention.rope_attention(x, cos.cuda(), sin.cuda(), cu.cuda(), n_q, n_kv, D, causal, D ** -0.5, window, max_len)
+    got.backward(do.cuda())
+    _cuda.check_status()
+    for a, b in ((got.detach(), want.detach()), (x.grad, ref.grad)):
+        assert torch.isfinite(a).all()
+        assert (a.float().cpu() - b).norm() < 2 ** -6 * b.norm()
+
+
+def test_small_document_kernel_refuses_a_longer_document():
+    """The promise of ``max_len`` is checked: the document is skipped and the status word raised, nothing is read past a tile."""
+    from lmms_engine_b200.ops import _cuda, attention
+
+    x = torch.randn(70, 3 * 64, device="cuda", dtype=torch.bfloat16)
+    cs = torch.ones(70, 64, device="cuda")
+    attention.rope_attention(x, cs, cs, torch.tensor([0, 70], dtype=torch.int32, device="cuda"), 1, 1, 64, False, 0.125, max_len=64)
+    with pytest.raises(RuntimeError):
+        _cuda.check_status()
