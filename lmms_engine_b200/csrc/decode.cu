@@ -84,7 +84,8 @@ struct SkinnyParams {
 // so lane (g = lane / 4, t = lane % 4) loads 16 contiguous bytes of row g at k0 + 8 t and k0 + 32 + 8 t: full 128-byte
 // lines of eight rows per warp and step, straight into fragments.
 // RT = 1 below 17 rows: N / 8 CTAs are enough to fill the chip from N = 1024 on, and a row's slice of K per warp is short.
-// From 17 rows on the activations (M x K) that every CTA reads from L2 outweigh eight weight rows, so RT grows with MT.
+// From 17 rows on the activations (M x K) that every CTA reads from L2 outweigh eight weight rows, so RT grows - as long as
+// the grid still has a CTA for every SM (RT = 4 left 32 CTAs for the 1024 output rows of a narrow model).
 template <int RT, int MT, int MODE, bool NORM>
 __global__ void __launch_bounds__(kSkWarps * 32) skinny_kernel(const __grid_constant__ SkinnyParams p) {
   extern __shared__ __align__(16) uint8_t dyn[];
@@ -300,7 +301,7 @@ struct DecAttnParams {
   float scale_log2;
   int window;                    // keys further back than this are not seen (< 0: all)
   int splits;
-  float* ws;                     // [n_seq, n_kv, splits, group, D + 2] partial results
+  float* ws;                     // partial results [n_seq, n_kv, splits, group, D], then their (max, sum) [..., 2]
   int* count;                    // [n_seq, n_kv] arrivals; returned to zero
   bf16* out;                     // [n_seq, n_kv * group * D]
   long ldo;
@@ -371,6 +372,36 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
   bf16* kc = p.kc + head_off;
   bf16* vc = p.vc + head_off;
 
+  // The cached rows do not depend on the kernel in front of this one: a warp whose first block holds older keys only loads
+  // it before the wait.
+  bf16* vt = sV + warp * 2 * 16 * D;
+  const int n_blk = (hi - lo + 15) / 16;
+  uint4 kf[2][NC];
+  auto load_k = [&](int b) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int key = min(lo + b * 16 + n * 8 + g, hi - 1);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) kf[n][c] = *reinterpret_cast<const uint4*>(kc + key * row_ld + c * 32 + t * 8);
+    }
+  };
+  auto load_v = [&](int b, int buf) {  // 16-byte pieces, piece index xor key so that ldmatrix rows fall on distinct banks
+    constexpr int kPieces = D / 8;
+#pragma unroll
+    for (int i = 0; i < 16 * kPieces / 32; ++i) {
+      const int idx = i * 32 + lane, r = idx / kPieces, c = idx % kPieces;
+      const int key = min(lo + b * 16 + r, hi - 1);
+      const uint32_t dst = smem_u32(vt + buf * 16 * D + r * D + ((c ^ (r & 7)) * 8));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(vc + key * row_ld + c * 8) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const bool early = warp < n_blk && lo + (warp + 1) * 16 <= total - 1;
+  if (early) {
+    load_v(warp, 0);
+    load_k(warp);
+  }
+
   pdl_go();
   pdl_wait();
   const bf16* pr = p.proj + seq * p.ld;
@@ -402,30 +433,7 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
 #pragma unroll
   for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
   float mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.f, 0.f};
-  bf16* vt = sV + warp * 2 * 16 * D;
-  const int n_blk = (hi - lo + 15) / 16;
-
-  uint4 kf[2][NC];
-  auto load_k = [&](int b) {
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      const int key = min(lo + b * 16 + n * 8 + g, hi - 1);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) kf[n][c] = *reinterpret_cast<const uint4*>(kc + key * row_ld + c * 32 + t * 8);
-    }
-  };
-  auto load_v = [&](int b, int buf) {  // 16-byte pieces, piece index xor key so that ldmatrix rows fall on distinct banks
-    constexpr int kPieces = D / 8;
-#pragma unroll
-    for (int i = 0; i < 16 * kPieces / 32; ++i) {
-      const int idx = i * 32 + lane, r = idx / kPieces, c = idx % kPieces;
-      const int key = min(lo + b * 16 + r, hi - 1);
-      const uint32_t dst = smem_u32(vt + buf * 16 * D + r * D + ((c ^ (r & 7)) * 8));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(vc + key * row_ld + c * 8) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  if (warp < n_blk) {
+  if (warp < n_blk && !early) {
     load_v(warp, 0);
     load_k(warp);
   }
@@ -519,7 +527,9 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
       r = r * sigmoid_f(__bfloat162float(pr[p.gate_off + static_cast<long>(kvh * p.group + h) * p.q_hs + d]));
     p.out[seq * p.ldo + static_cast<long>(kvh * p.group + h) * D + d] = __float2bfloat16(r);
   };
-  float* ws = p.ws + static_cast<size_t>((seq * p.n_kv + kvh)) * p.splits * p.group * (D + 2);
+  const size_t share0 = static_cast<size_t>(seq * p.n_kv + kvh) * p.splits * p.group;   // (share, head) pairs in front
+  float* wo = p.ws + share0 * D;
+  float2* wml = reinterpret_cast<float2*>(p.ws + static_cast<size_t>(gridDim.z) * p.n_kv * p.splits * p.group * D) + share0;
   for (int i = threadIdx.x; i < p.group * D; i += 128) {
     const int h = i / D, d = i % D;
     float m = -INFINITY;
@@ -538,12 +548,8 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
     if (p.splits == 1) {
       store(h, d, v / l);
     } else {
-      float* dst = ws + (static_cast<size_t>(split) * p.group + h) * (D + 2);
-      dst[d] = v;
-      if (d == 0) {
-        dst[D] = m;
-        dst[D + 1] = l;
-      }
+      wo[(split * p.group + h) * D + d] = v;
+      if (d == 0) wml[split * p.group + h] = make_float2(m, l);
     }
   }
   if (p.splits == 1) return;
@@ -558,18 +564,37 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
   __syncthreads();
   if (!*sLast) return;
   __threadfence();
-  for (int i = threadIdx.x; i < p.group * D; i += 128) {
-    const int h = i / D, d = i % D;
-    float m = -INFINITY;
-    for (int s = 0; s < p.splits; ++s) m = fmaxf(m, __ldcg(ws + (static_cast<size_t>(s) * p.group + h) * (D + 2) + D));
-    float l = 0.f, v = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const float* src = ws + (static_cast<size_t>(s) * p.group + h) * (D + 2);
-      const float f = fast_exp2(__ldcg(src + D) - m);  // an empty share has m = -inf: weight 0
-      l += f * __ldcg(src + D + 1);
-      v += f * __ldcg(src + d);
+  // A warp per head, four columns per lane (two shares side by side for D = 64): the loads of a share depend on nothing, so
+  // eight of them are in flight.  One thread per element instead walked all shares once for the maximum and once for the sum:
+  // 64 shares x 7 heads took longer than the attention itself.
+  constexpr int LR = D / 4, SG = 32 / LR;
+  const int sg = lane / LR, d0 = (lane % LR) * 4;
+  for (int h = warp; h < p.group; h += 4) {
+    float2 ml[2] = {make_float2(-INFINITY, 0.f), make_float2(-INFINITY, 0.f)};   // shares lane and lane + 32 (at most 64)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (lane + 32 * i < p.splits) ml[i] = __ldcg(wml + (lane + 32 * i) * p.group + h);
+    const float m = warp_max(fmaxf(ml[0].x, ml[1].x));
+    const float f0 = fast_exp2(ml[0].x - m), f1 = fast_exp2(ml[1].x - m);  // an empty share has m = -inf: weight 0
+    const float l = warp_sum(f0 * ml[0].y + f1 * ml[1].y);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s0 = 0; s0 < p.splits; s0 += SG) {
+      const int s = s0 + sg;
+      const float g0 = __shfl_sync(0xffffffffu, f0, s & 31), g1 = __shfl_sync(0xffffffffu, f1, s & 31);
+      const float w = s < 32 ? g0 : g1;
+      if (s < p.splits) {
+        const float4 o4 = __ldcg(reinterpret_cast<const float4*>(wo + (s * p.group + h) * D + d0));
+        v.x += w * o4.x; v.y += w * o4.y; v.z += w * o4.z; v.w += w * o4.w;
+      }
     }
-    store(h, d, v / l);
+    if (SG == 2) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, 16); v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+      v.z += __shfl_xor_sync(0xffffffffu, v.z, 16); v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
+    }
+    if (sg == 0) {
+      store(h, d0, v.x / l); store(h, d0 + 1, v.y / l); store(h, d0 + 2, v.z / l); store(h, d0 + 3, v.w / l);
+    }
   }
 }
 
@@ -701,14 +726,23 @@ static int launch_skinny(const SkinnyParams& p, cudaStream_t st, bool early) {
   return launch_k(skinny_kernel<RT, MT, MODE, NORM>, dim3((p.N + per - 1) / per), kSkWarps * 32, smem, st, p, early);
 }
 
+template <int MT, int MODE>
+static int wide(const SkinnyParams& p, cudaStream_t st, bool early) {
+  constexpr int per = MODE == SK_SWIGLU ? 4 : 8;   // output rows per weight tile
+  constexpr int kSms = 148;
+  if (MT > 2 && p.N >= kSms * per * 4) return launch_skinny<4, MT, MODE, false>(p, st, early);
+  if (MODE == SK_SWIGLU || p.N >= kSms * per * 2) return launch_skinny<2, MT, MODE, false>(p, st, early);
+  return launch_skinny<MODE == SK_SWIGLU ? 2 : 1, MT, MODE, false>(p, st, early);
+}
+
 template <int MODE>
 static int skinny(const SkinnyParams& p, cudaStream_t st, bool early = true) {
   constexpr int R1 = MODE == SK_SWIGLU ? 2 : 1;
   if (p.norm_w != nullptr) return launch_skinny<R1, 1, MODE, true>(p, st, early);
   if (p.M <= 16) return launch_skinny<R1, 1, MODE, false>(p, st, early);
-  if (p.M <= 32) return launch_skinny<2, 2, MODE, false>(p, st, early);
-  if (p.M <= 48) return launch_skinny<4, 3, MODE, false>(p, st, early);
-  return launch_skinny<4, 4, MODE, false>(p, st, early);
+  if (p.M <= 32) return wide<2, MODE>(p, st, early);
+  if (p.M <= 48) return wide<3, MODE>(p, st, early);
+  return wide<4, MODE>(p, st, early);
 }
 
 static bool norm_fits(int M, int K) { return M <= kSkNormRows && static_cast<size_t>(M) * (K + 8) * 2 <= 96 * 1024; }

@@ -202,8 +202,9 @@ def _run(backbone, embeds, ctx, cache, seqs):
     longest = max(have) + 1
     if cache.decode_window >= 0:
         longest = min(longest, cache.decode_window + 1)
-    # shares of a key head: enough to fill the chip about twice, at least 64 keys each
-    splits = max(1, min(-(-296 // (nkv * M)), -(-longest // 64), 64))
+    # shares of a key head: enough to fill the chip about twice or 512 keys each (a batch waits for its longest sequence),
+    # whichever are more, and at least 64 keys each
+    splits = max(1, min(max(-(-296 // (nkv * M)), -(-longest // 512)), -(-longest // 64), 64))
     has_attn = any(t != 2 for t in types)
     np_ = max(nq * D * 2 + 2 * nkv * D if has_attn else 0, (2 * hk + 2 * hv) * 128 + 2 * hv)
     work = torch.empty(2 * M * (np_ + max(nq * D, hv * 128) + I + H) + 4096, dtype=torch.uint8, device=dev)
