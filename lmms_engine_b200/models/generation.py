@@ -79,7 +79,8 @@ class GenerationState:
         pos, out = _prompt_positions(self.model, lambda: self.model(input_ids=ids, cu_seqlens=cu, kv_cache=self.cache, **kw))
         pos = plain if pos is None else pos
         self.mrope = pos.dim() == 2
-        self.next_pos = int(pos.max()) + 1
+        # text positions are the token index, known here; only positions that the model built itself are read from the device
+        self.next_pos = self.cache.lens[0] if pos is plain else int(pos.max()) + 1
         return out["hidden_states"][-1:]
 
     def step(self, token: torch.Tensor, **inputs) -> torch.Tensor:
@@ -87,7 +88,7 @@ class GenerationState:
         self.cache.advance([1])
         p = torch.full((3, 1) if self.mrope else (1,), self.next_pos, dtype=torch.long, device=token.device)
         self.next_pos += 1
-        cu = torch.tensor([0, 1], dtype=torch.int32, device=token.device)
+        cu = torch.arange(2, dtype=torch.int32, device=token.device)  # [0, 1] without a copy from the host, which would wait
         return self.model(input_ids=token.reshape(1), cu_seqlens=cu, position_ids=p, kv_cache=self.cache, **inputs)["hidden_states"]
 
 

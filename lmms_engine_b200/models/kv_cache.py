@@ -53,9 +53,17 @@ class PackedKVCache:
 
     def _spread(self, starts: Sequence[int]) -> torch.Tensor:
         """``starts[i], starts[i] + 1, ...`` for the new tokens of every sequence, on the cache's device."""
+        live = [(s, n) for s, n in zip(starts, self.new_lens) if n]
+        if len(live) == 1:
+            return torch.arange(live[0][0], live[0][0] + live[0][1], device=self.device)
         if max(self.new_lens) == 1:
-            return torch.tensor([s for s, n in zip(starts, self.new_lens) if n]).to(self.device)
-        return torch.cat([torch.arange(s, s + n) for s, n in zip(starts, self.new_lens) if n]).to(self.device)
+            host = torch.tensor([s for s, _ in live])
+        else:
+            host = torch.cat([torch.arange(s, s + n) for s, n in live])
+        if self.device is None or torch.device(self.device).type != "cuda":
+            return host.to(self.device)
+        # from pinned memory: a pageable copy waits for everything queued on the device, once per generated token
+        return host.pin_memory().to(self.device, non_blocking=True)
 
     def _row_tables(self) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]:
         """Rows that this pass' tokens go to, rows that they attend to, and the boundaries of the latter; built once per
