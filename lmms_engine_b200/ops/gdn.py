@@ -22,7 +22,7 @@ from . import _cuda
 CHUNK = 64
 
 _cuda.register("b200_gdn_scan_fwd", "gdn_scan", "ppppppppp" + "iiii" + "s")
-_cuda.register("b200_gdn_scan_bwd", "gdn_scan", "pppppppppppppp" + "iiii" + "s")
+_cuda.register("b200_gdn_scan_bwd", "gdn_scan", "ppppppppppppppp" + "iiii" + "s")
 _cuda.register("b200_gdn_chunk_fwd", "gdn_chunk", "ppp" + "lll" + "ppp" + "l" + "ii" + "f" + "i" + "pppppppp" + "s")
 _cuda.register("b200_gdn_chunk_bwd", "gdn_chunk", "ppp" + "lll" + "ppp" + "l" + "ii" + "f" + "i" + "ppppp" + "pppppp" + "ppppp" + "s")
 _cuda.register("b200_gdn_chunk_out", "gdn_chunk", "ppppp" + "l" + "iii" + "s")
@@ -78,17 +78,15 @@ class _Scan(torch.autograd.Function):
         w, qt, kt, gamma, reset_t, vnew, hist = ctx.saved_tensors
         H, n, _, dk = w.shape
         dv = vnew.shape[-1]
-        ns = dv // 32
         d_vnew = _dense16(d_vnew) if d_vnew is not None else torch.zeros_like(vnew)
         d_o = _dense16(d_o) if d_o is not None else torch.zeros_like(vnew)
         du = torch.empty_like(vnew)
-        parts = torch.empty((3, ns, H, n, CHUNK, dk), dtype=torch.float32, device=w.device)
-        dg_p = torch.empty((ns, H, n), dtype=torch.float32, device=w.device)
+        dw, dq, dk_ = (torch.empty_like(w) for _ in range(3))
+        dgamma, dhist = torch.empty_like(gamma), torch.empty_like(hist)
         _cuda.call("b200_gdn_scan_bwd", w.data_ptr(), qt.data_ptr(), kt.data_ptr(), gamma.data_ptr(), reset_t.data_ptr(),
-                   vnew.data_ptr(), hist.data_ptr(), d_vnew.data_ptr(), d_o.data_ptr(), du.data_ptr(), parts[0].data_ptr(),
-                   parts[1].data_ptr(), parts[2].data_ptr(), dg_p.data_ptr(), H, n, dk, dv, _cuda.stream())
-        dw, dq, dk_ = parts.sum(1).unbind(0)
-        return dw, du, dq, dk_, dg_p.sum(0), None
+                   vnew.data_ptr(), hist.data_ptr(), d_vnew.data_ptr(), d_o.data_ptr(), du.data_ptr(), dw.data_ptr(), dq.data_ptr(),
+                   dk_.data_ptr(), dgamma.data_ptr(), dhist.data_ptr(), H, n, dk, dv, _cuda.stream())
+        return dw, du, dq, dk_, dgamma, None
 
 
 def scan(w, u, qt, kt, gamma, reset: List[bool]):
