@@ -469,6 +469,148 @@ __global__ void rope_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__
   }
 }
 
+// ------------------------------------------------------------------ per-head RMSNorm + rotary embedding
+// The q and k heads of a projection row [T, n_q + n_kv (+ ...), D] (row stride ldx): y = rope(rmsnorm(x) * w), the rotation over
+// the whole head; D = 64 or 128.  D / 8 lanes share a head and hold four columns of each half, so both the norm's sum and the
+// rotation's partner stay inside a lane group.  As separate passes a head was copied out of its strided row, normalised and
+// rotated (six reads and writes of q and k); here it is read and written once.  Bound by memory.
+__device__ __forceinline__ float group_sum(float v, int lanes) {
+  for (int o = lanes >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int D>
+__global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
+                                                               const bf16* __restrict__ wq, const bf16* __restrict__ wk,
+                                                               const float* __restrict__ cosb, const float* __restrict__ sinb,
+                                                               float* __restrict__ rstd, long T, int n_q, int n_kv, long ldx,
+                                                               long ldy, float eps) {
+  constexpr int L = D / 8, HPW = 32 / L;   // lanes per head, heads per warp
+  const int lane = threadIdx.x & 31, l = lane % L, heads = n_q + n_kv;
+  const long total = T * heads;
+  const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
+  // every lane of a warp takes part in the shuffles: a group past the end computes on the last head and stores nothing
+  for (long w0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * HPW; w0 < total; w0 += warps * HPW) {
+    const long idx = w0 + lane / L;
+    const bool live = idx < total;
+    const long at = live ? idx : total - 1;
+    const long t = at / heads;
+    const int h = static_cast<int>(at - t * heads);
+    const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
+    float a[4], b[4], ca[4], sa[4];
+    load_w<4>(xp, a);
+    load_w<4>(xp + D / 2, b);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ss += a[j] * a[j] + b[j] * b[j];
+    const float r = rsqrtf(group_sum(ss, L) / D + eps);
+    if (live && l == 0) rstd[at] = r;
+    float wa[4], wb[4];
+    const bf16* w = (h < n_q ? wq : wk) + 4 * l;
+    load_w<4>(w, wa);
+    load_w<4>(w + D / 2, wb);
+    const float* c = cosb + t * D + 4 * l;
+    const float* s = sinb + t * D + 4 * l;
+    float o1[4], o2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // the normalised head is a bf16 tensor of its own in the separate form: rounded here too
+      const float x1 = __bfloat162float(__float2bfloat16(a[j] * r * wa[j]));
+      const float x2 = __bfloat162float(__float2bfloat16(b[j] * r * wb[j]));
+      ca[j] = c[j]; sa[j] = s[j];
+      o1[j] = x1 * ca[j] - x2 * sa[j];
+      o2[j] = x2 * c[D / 2 + j] + x1 * s[D / 2 + j];
+    }
+    if (live) {
+      bf16* yp = y + t * ldy + static_cast<long>(h) * D + 4 * l;
+      store_w<4>(yp, o1);
+      store_w<4>(yp + D / 2, o2);
+    }
+  }
+}
+// d [T, heads, D] (row stride ldd): gradient of y on entry, of x on exit; part [gridDim.x][2][D] partial weight gradients.
+template <int D>
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf16* __restrict__ x, const bf16* __restrict__ wq,
+                                                               const bf16* __restrict__ wk, const float* __restrict__ cosb,
+                                                               const float* __restrict__ sinb, const float* __restrict__ rstd,
+                                                               float* __restrict__ part, long T, int n_q, int n_kv, long ldx,
+                                                               long ldd) {
+  constexpr int L = D / 8, HPW = 32 / L;
+  __shared__ float sw[2][D];
+  const int lane = threadIdx.x & 31, l = lane % L, heads = n_q + n_kv;
+  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&sw[0][0])[i] = 0.f;
+  __syncthreads();
+  float dw[2][8] = {};
+  const long total = T * heads;
+  const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
+  for (long w0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * HPW; w0 < total; w0 += warps * HPW) {
+    const long idx = w0 + lane / L;
+    const bool live = idx < total;
+    const long at = live ? idx : total - 1;
+    const long t = at / heads;
+    const int h = static_cast<int>(at - t * heads);
+    const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
+    bf16* dp = d + t * ldd + static_cast<long>(h) * D + 4 * l;
+    float a[4], b[4], da[4], db[4], wa[4], wb[4];
+    load_w<4>(xp, a);
+    load_w<4>(xp + D / 2, b);
+    load_w<4>(dp, da);
+    load_w<4>(dp + D / 2, db);
+    const bool is_q = h < n_q;
+    const bf16* w = (is_q ? wq : wk) + 4 * l;
+    load_w<4>(w, wa);
+    load_w<4>(w + D / 2, wb);
+    const float* c = cosb + t * D + 4 * l;
+    const float* s = sinb + t * D + 4 * l;
+    const float r = rstd[at];
+    float dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // transposed rotation, rounded where the separate form stores it
+      const float g1 = __bfloat162float(__float2bfloat16(da[j] * c[j] + db[j] * s[D / 2 + j]));
+      const float g2 = __bfloat162float(__float2bfloat16(db[j] * c[D / 2 + j] - da[j] * s[j]));
+      a[j] *= r;
+      b[j] *= r;
+      if (live) {
+        dw[is_q ? 0 : 1][j] += g1 * a[j];
+        dw[is_q ? 0 : 1][4 + j] += g2 * b[j];
+      }
+      da[j] = g1 * wa[j];
+      db[j] = g2 * wb[j];
+      dot += da[j] * a[j] + db[j] * b[j];
+    }
+    const float m = group_sum(dot, L) / D;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      da[j] = r * (da[j] - a[j] * m);
+      db[j] = r * (db[j] - b[j] * m);
+    }
+    __syncwarp();   // a group past the end read the last head: it must have before that head is rewritten
+    if (live) {
+      store_w<4>(dp, da);
+      store_w<4>(dp + D / 2, db);
+    }
+  }
+  // the groups of a warp in a fixed order, then the warps one after the other: the same sum on every run
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      for (int o = L; o < 32; o <<= 1) dw[k][j] += __shfl_xor_sync(0xffffffffu, dw[k][j], o);
+  for (int wv = 0; wv < static_cast<int>(blockDim.x >> 5); ++wv) {
+    if (static_cast<int>(threadIdx.x >> 5) == wv && lane < L) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sw[k][4 * l + j] += dw[k][j];
+          sw[k][D / 2 + 4 * l + j] += dw[k][4 + j];
+        }
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) part[static_cast<long>(blockIdx.x) * 2 * D + i] = (&sw[0][0])[i];
+}
+
 // ------------------------------------------------------------------ SwiGLU
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ g, const bf16* __restrict__ u, bf16* __restrict__ h,
                                   long n8) {
@@ -979,6 +1121,36 @@ int b200_rope_apply(const void* x, void* y, const void* cosb, const void* sinb, 
     rope_apply_kernel<4><<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x, (bf16*)y, (const float*)cosb, (const float*)sinb, T, Hn, D,
                                                                rot_dim, ldx, ldy, conj);
   }
+  return CHECK_LAUNCH();
+}
+
+// Partial weight gradients that b200_qk_norm_rope_bwd writes: part [this][2][D] fp32.
+int b200_qk_norm_rope_parts() { return 296; }
+
+// q and k heads of rows x [T, >= (n_q + n_kv) * D] into y; D 64 or 128, rows on 16-byte boundaries, rstd [T, n_q + n_kv].
+int b200_qk_norm_rope_fwd(const void* x, void* y, const void* wq, const void* wk, const void* cosb, const void* sinb, void* rstd,
+                          long T, int n_q, int n_kv, int D, long ldx, long ldy, float eps, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if ((D != 64 && D != 128) || ldx % 8 || ldy % 8 || n_q + n_kv <= 0) return -10;
+  const int blocks = grid_for(T * (n_q + n_kv) * (D / 8), 256);
+  if (D == 128)
+    qk_norm_rope_fwd_kernel<128><<<blocks, 256, 0, st>>>((const bf16*)x, (bf16*)y, (const bf16*)wq, (const bf16*)wk, (const float*)cosb,
+                                                         (const float*)sinb, (float*)rstd, T, n_q, n_kv, ldx, ldy, eps);
+  else
+    qk_norm_rope_fwd_kernel<64><<<blocks, 256, 0, st>>>((const bf16*)x, (bf16*)y, (const bf16*)wq, (const bf16*)wk, (const float*)cosb,
+                                                        (const float*)sinb, (float*)rstd, T, n_q, n_kv, ldx, ldy, eps);
+  return CHECK_LAUNCH();
+}
+int b200_qk_norm_rope_bwd(void* d, const void* x, const void* wq, const void* wk, const void* cosb, const void* sinb, const void* rstd,
+                          void* part, long T, int n_q, int n_kv, int D, long ldx, long ldd, cudaStream_t st) {
+  if ((D != 64 && D != 128) || ldx % 8 || ldd % 8 || n_q + n_kv <= 0 || T <= 0) return -10;
+  const int blocks = b200_qk_norm_rope_parts();
+  if (D == 128)
+    qk_norm_rope_bwd_kernel<128><<<blocks, 256, 0, st>>>((bf16*)d, (const bf16*)x, (const bf16*)wq, (const bf16*)wk, (const float*)cosb,
+                                                         (const float*)sinb, (const float*)rstd, (float*)part, T, n_q, n_kv, ldx, ldd);
+  else
+    qk_norm_rope_bwd_kernel<64><<<blocks, 256, 0, st>>>((bf16*)d, (const bf16*)x, (const bf16*)wq, (const bf16*)wk, (const float*)cosb,
+                                                        (const float*)sinb, (const float*)rstd, (float*)part, T, n_q, n_kv, ldx, ldd);
   return CHECK_LAUNCH();
 }
 

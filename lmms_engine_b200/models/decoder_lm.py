@@ -138,6 +138,27 @@ class Attention(nn.Module):
         window = cfg.sliding_window if (cfg.use_sliding_window and cfg.sliding_window) else None
         self.window = (window, -1) if window else (-1, -1)
 
+    def _head_norms(self):
+        """``(q weight, k weight, eps)`` of plain per-head norms, ``None`` without them, ``False`` where they have to be called."""
+        if not self.cfg.qk_norm:
+            return None
+        q, k = self.q_norm, self.k_norm
+        if type(q) is not RMSNorm or type(k) is not RMSNorm or q.eps != k.eps or q._forward_hooks or k._forward_hooks \
+                or q._forward_pre_hooks or k._forward_pre_hooks:
+            return False
+        return q.weight, k.weight, q.eps
+
+    def _cached_attention(self, qkv, ctx, norms):
+        """A pass against the key / value cache (several new tokens per sequence), without gradients."""
+        D, T = self.head_dim, qkv.shape[0]
+        heads = attn_ops.rope_heads(qkv, ctx.cos, ctx.sin, self.n_q, self.n_kv, D, norms)
+        if heads is None:
+            return None
+        v = qkv[:, (self.n_q + self.n_kv) * D:].view(T, self.n_kv, D)
+        k_all, v_all, cu_k, max_k = ctx.kv_cache.extend(self.layer_idx, heads[1], v)
+        return attn_ops.varlen_attn(heads[0], k_all, v_all, ctx.cu_seqlens, cu_k, ctx.max_seqlen, max_k, causal=ctx.causal,
+                                    softmax_scale=1.0 / math.sqrt(D), window_size=self.window)
+
     def forward(self, x: torch.Tensor, ctx: "PackedContext") -> torch.Tensor:
         D = self.head_dim
         # one GEMM for q, k, v: the three weights are concatenated on the fly (tens of MB,
@@ -161,10 +182,13 @@ class Attention(nn.Module):
                     # rank's heads; the row-parallel output projection below reduce-scatters back
                     x = tp_ops.all_gather_tokens(x, ctx.tp_group)
                 qkv = gemm_ops.linear(x, w, b)
-            if not (self.cfg.qk_norm or ctx.sp_size > 1 or ctx.tp_size > 1 or getattr(self, "nsa", None) is not None
-                    or getattr(ctx, "kv_cache", None) is not None):
-                o = attn_ops.rope_attention(qkv, ctx.cos, ctx.sin, ctx.cu_seqlens, self.n_q, self.n_kv, D, ctx.causal,
-                                            1.0 / math.sqrt(D), self.window[0])
+            norms = self._head_norms()
+            if norms is not False and ctx.sp_size <= 1 and ctx.tp_size <= 1 and getattr(self, "nsa", None) is None:
+                if getattr(ctx, "kv_cache", None) is None:
+                    o = attn_ops.rope_attention(qkv, ctx.cos, ctx.sin, ctx.cu_seqlens, self.n_q, self.n_kv, D, ctx.causal,
+                                                1.0 / math.sqrt(D), self.window[0], norms=norms)
+                else:
+                    o = self._cached_attention(qkv, ctx, norms)
                 if o is not None:
                     return gemm_ops.linear(o.reshape(o.shape[0], -1), _w(self.o_proj.weight), None)
             T = qkv.shape[0]

@@ -18,6 +18,9 @@ from . import _cuda
 
 _cuda.register("b200_attn_fwd", "attention_sm100", "ppppppp" + "iiiiii" + "llll" + "fii" + "ps")
 _cuda.register("b200_attn_bwd", "attention_sm100", "ppppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
+_cuda.register("b200_qk_norm_rope_parts", "elementwise", "")
+_cuda.register("b200_qk_norm_rope_fwd", "elementwise", "ppppppp" + "liii" + "ll" + "f" + "s")
+_cuda.register("b200_qk_norm_rope_bwd", "elementwise", "pppppppp" + "liii" + "ll" + "s")
 _cuda.register("b200_attn_small_fwd", "attention_small", "ppppppp" + "iiiiii" + "llll" + "fii" + "ps")
 _cuda.register("b200_attn_small_bwd", "attention_small", "ppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
 _cuda.register("b200_attn_bwd_v2", "attention_bwd_sm100", "pppppppppppp" + "iiiiii" + "llllllll" + "fii" + "ps")
@@ -127,57 +130,100 @@ class _VarlenAttnFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None, None
 
 
+def _rotate(x, ldx, y, cos, sin, heads, D, conj):
+    _cuda.call("b200_rope_apply", x.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), y.shape[0], heads, D, D, ldx, y.stride(0),
+               int(conj), _cuda.stream())
+
+
+def _rotated(qkv, cos, sin, n_q, n_kv, D, wq, wk, eps):
+    """q and k heads of the projection rows, normalised per head where weights are given, rotated: ``([T, n_q + n_kv, D], rstd)``."""
+    T = qkv.shape[0]
+    rot = torch.empty((T, n_q + n_kv, D), dtype=qkv.dtype, device=qkv.device)
+    if wq is None:
+        _rotate(qkv, qkv.stride(0), rot, cos, sin, n_q + n_kv, D, False)
+        return rot, None
+    rstd = torch.empty((T, n_q + n_kv), dtype=torch.float32, device=qkv.device)
+    _cuda.call("b200_qk_norm_rope_fwd", qkv.data_ptr(), rot.data_ptr(), wq.data_ptr(), wk.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+               rstd.data_ptr(), T, n_q, n_kv, D, qkv.stride(0), rot.stride(0), float(eps), _cuda.stream())
+    return rot, rstd
+
+
 class _RopeAttnFn(torch.autograd.Function):
-    """Rotary embedding + attention on the rows of ONE projection ``[T, (n_q + 2 n_kv) * D]`` (heads of q, then k, then v).
+    """(Per-head RMSNorm of q and k +) rotary embedding + attention on the rows of ONE projection
+    ``[T, (n_q + 2 n_kv) * D]`` (heads of q, then k, then v).
 
     As separate operations on slices of the projection, the backward pass builds three zero-filled gradients of its whole
     size and adds them (five passes over it, twice that for a 3-way view); here the attention backward writes its three
-    gradients into the rows of one buffer and the rotation runs in place on the q and k part.  Query and key heads are
-    neighbours in a row, so both are rotated by one launch."""
+    gradients into the rows of one buffer and the rotation (and norm) runs in place on the q and k part.  Query and key heads
+    are neighbours in a row, so both are handled by one launch."""
 
     @staticmethod
-    def forward(ctx, qkv, cos, sin, cu, n_q, n_kv, D, causal, scale, window_left, small):
-        T = qkv.shape[0]
-        rot = torch.empty((T, n_q + n_kv, D), dtype=qkv.dtype, device=qkv.device)
-        _rotate(qkv, qkv.stride(0), rot, cos, sin, n_q + n_kv, D, False)
-        v = qkv[:, (n_q + n_kv) * D:].view(T, n_kv, D)
+    def forward(ctx, qkv, wq, wk, cos, sin, cu, n_q, n_kv, D, eps, causal, scale, window_left, small):
+        rot, rstd = _rotated(qkv, cos, sin, n_q, n_kv, D, wq, wk, eps)
+        v = qkv[:, (n_q + n_kv) * D:].view(qkv.shape[0], n_kv, D)
         o, lse = _fwd(rot[:, :n_q], rot[:, n_q:], v, cu, cu, causal, scale, window_left, small)
-        ctx.save_for_backward(rot, v, o, lse, cu, cos, sin)
+        ctx.save_for_backward(rot, qkv, o, lse, cu, cos, sin, wq, wk, rstd)
         ctx.cfg = (causal, scale, window_left)
         ctx.dims = (n_q, n_kv, D, small)
         return o
 
     @staticmethod
     def backward(ctx, do):
-        rot, v, o, lse, cu, cos, sin = ctx.saved_tensors
+        rot, qkv, o, lse, cu, cos, sin, wq, wk, rstd = ctx.saved_tensors
         n_q, n_kv, D, small = ctx.dims
         T = rot.shape[0]
+        v = qkv[:, (n_q + n_kv) * D:].view(T, n_kv, D)
         d = torch.empty((T, n_q + 2 * n_kv, D), dtype=rot.dtype, device=rot.device)
         _bwd(rot[:, :n_q], rot[:, n_q:], v, o, lse, do, cu, cu, *ctx.cfg, d[:, :n_q], d[:, n_q:n_q + n_kv], d[:, n_q + n_kv:], small)
-        _rotate(d, d.stride(0), d, cos, sin, n_q + n_kv, D, True)
-        return (d.view(T, -1),) + (None,) * 10
+        dwq = dwk = None
+        if wq is None:
+            _rotate(d, d.stride(0), d, cos, sin, n_q + n_kv, D, True)
+        else:
+            part = torch.empty((_cuda.fn("b200_qk_norm_rope_parts")(), 2, D), dtype=torch.float32, device=rot.device)
+            _cuda.call("b200_qk_norm_rope_bwd", d.data_ptr(), qkv.data_ptr(), wq.data_ptr(), wk.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+                       rstd.data_ptr(), part.data_ptr(), T, n_q, n_kv, D, qkv.stride(0), d.stride(0), _cuda.stream())
+            dwq, dwk = part.sum(0).to(wq.dtype).unbind(0)
+        return (d.view(T, -1), dwq, dwk) + (None,) * 11
 
 
-def _rotate(x, ldx, y, cos, sin, heads, D, conj):
-    _cuda.call("b200_rope_apply", x.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), y.shape[0], heads, D, D, ldx, y.stride(0),
-               int(conj), _cuda.stream())
+def _fused_rows_ok(qkv, cos, sin, n_q, n_kv, D, wq, wk) -> bool:
+    """Rows, tables and norm weights that the fused kernels read: bf16 rows on 16-byte boundaries, whole-head rotation, fp32
+    tables of exactly these rows; with norms, heads of 64 or 128 (a lane group owns a head)."""
+    def plain(w):
+        return (type(w) in (torch.Tensor, torch.nn.Parameter) and w.is_cuda and w.dtype == torch.bfloat16 and w.shape == (D,)
+                and w.is_contiguous() and w.data_ptr() % 8 == 0)
+    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and qkv.shape[1] == (n_q + 2 * n_kv) * D
+            and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and D % 8 == 0 and D <= 128
+            and n_q % n_kv == 0 and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
+            and cos.shape == sin.shape == (qkv.shape[0], D) and not (cos.requires_grad or sin.requires_grad)
+            and (wq is None) == (wk is None) and (wq is None or (D in (64, 128) and plain(wq) and plain(wk))))
 
 
 def rope_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, cu_seqlens: torch.Tensor, n_q: int, n_kv: int, D: int,
-                   causal: bool, softmax_scale: float, window_left: int = -1, max_len: Optional[int] = None) -> Optional[torch.Tensor]:
-    """Rotary embedding over whole heads, then attention, from one projection's rows; ``None`` where the fused form does not
-    apply (other dtypes, partial rotation, rows off 16-byte boundaries) and the caller runs the operations one by one.
+                   causal: bool, softmax_scale: float, window_left: int = -1, max_len: Optional[int] = None,
+                   norms: Optional[Tuple[torch.Tensor, torch.Tensor, float]] = None) -> Optional[torch.Tensor]:
+    """Rotary embedding over whole heads (behind a per-head RMSNorm with ``norms`` = weights of q and k, eps), then attention,
+    from one projection's rows; ``None`` where the fused form does not apply (other dtypes, partial rotation, rows off 16-byte
+    boundaries) and the caller runs the operations one by one.
     ``max_len``: no document is longer, from a caller that made the boundaries; ``None`` where it is not known."""
-    ok = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and qkv.shape[1] == (n_q + 2 * n_kv) * D
-          and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and D % 8 == 0 and D <= 128
-          and n_q % n_kv == 0 and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
-          and cos.shape == sin.shape == (qkv.shape[0], D) and not (cos.requires_grad or sin.requires_grad))
-    if not ok:
+    wq, wk, eps = norms if norms is not None else (None, None, 0.0)
+    if not _fused_rows_ok(qkv, cos, sin, n_q, n_kv, D, wq, wk):
         return None
     cu = cu_seqlens.to(torch.int32).contiguous()
     small = max_len is not None and max_len <= SMALL_DOC and cu.numel() <= 65536
-    return _RopeAttnFn.apply(qkv, cos.contiguous(), sin.contiguous(), cu, n_q, n_kv, D, bool(causal), float(softmax_scale), int(window_left),
-                             small)
+    return _RopeAttnFn.apply(qkv, wq, wk, cos.contiguous(), sin.contiguous(), cu, n_q, n_kv, D, float(eps), bool(causal),
+                             float(softmax_scale), int(window_left), small)
+
+
+def rope_heads(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_q: int, n_kv: int, D: int,
+               norms: Optional[Tuple[torch.Tensor, torch.Tensor, float]] = None) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
+    """The first half of ``rope_attention`` without gradients: ``q [T, n_q, D]`` and ``k [T, n_kv, D]`` as they enter attention (and
+    a key / value cache), or ``None``."""
+    wq, wk, eps = norms if norms is not None else (None, None, 0.0)
+    if torch.is_grad_enabled() or not _fused_rows_ok(qkv, cos, sin, n_q, n_kv, D, wq, wk):
+        return None
+    rot, _ = _rotated(qkv, cos.contiguous(), sin.contiguous(), n_q, n_kv, D, wq, wk, eps)
+    return rot[:, :n_q], rot[:, n_q:]
 
 
 def varlen_attn(

@@ -157,3 +157,35 @@ def test_small_document_kernel_refuses_a_longer_document():
     attention.rope_attention(x, cs, cs, torch.tensor([0, 70], dtype=torch.int32, device="cuda"), 1, 1, 64, False, 0.125, max_len=64)
     with pytest.raises(RuntimeError):
         _cuda.check_status()
+
+
+@pytest.mark.parametrize("lens,n_q,n_kv,D", [((1,), 1, 1, 128), ((70, 3), 5, 1, 64), ((64, 129, 30), 4, 2, 128)])
+def test_head_norm_rotation_attention(lens, n_q, n_kv, D):
+    """Per-head norm + rotation + attention from the projection's rows against the fp32 formulation (six bf16 roundings of
+    2^-9 on the way: 2^-6 of the 2-norm bounds them), one head group past the end of the work included (odd head counts)."""
+    from lmms_engine_b200.ops import _cuda, attention, norm, rope
+
+    torch.manual_seed(4)
+    T = sum(lens)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
+    qkv = (2.0 * torch.randn(T, (n_q + 2 * n_kv) * D)).bfloat16()
+    wq, wk = (1 + 0.3 * torch.randn(D)).bfloat16(), (1 + 0.3 * torch.randn(D)).bfloat16()
+    ang = torch.randn(T, D // 2).repeat(1, 2)
+    cos, sin, do = ang.cos(), ang.sin(), torch.randn(T, n_q, D).bfloat16()
+    ref = [t.float().requires_grad_() for t in (qkv, wq, wk)]
+    q, k, v = ref[0].view(T, -1, D).split([n_q, n_kv, n_kv], 1)
+    q, k = norm.rmsnorm_ref(q, ref[1], 1e-6), norm.rmsnorm_ref(k, ref[2], 1e-6)
+    want = attention.varlen_attn_ref(rope.rope_apply_ref(q, cos, sin), rope.rope_apply_ref(k, cos, sin), v, cu, cu, True, D ** -0.5)
+    want.backward(do.float())
+    dev = [t.cuda().requires_grad_() for t in (qkv, wq, wk)]
+    got = attention.rope_attention(dev[0], cos.cuda(), sin.cuda(), cu.cuda(), n_q, n_kv, D, True, D ** -0.5, norms=(dev[1], dev[2], 1e-6))
+    got.backward(do.cuda())
+    _cuda.check_status()
+    for a, b in [(got.detach(), want.detach())] + [(x.grad, r.grad) for x, r in zip(dev, ref)]:
+        assert torch.isfinite(a).all()
+        assert (a.float().cpu() - b).norm() < 2 ** -6 * b.norm() + 1e-5
+    with torch.no_grad():
+        q2, k2 = attention.rope_heads(dev[0], cos.cuda(), sin.cuda(), n_q, n_kv, D, (dev[1], dev[2], 1e-6))
+        q1 = rope.rope_apply(norm.rmsnorm(dev[0][:, :n_q * D].reshape(-1, D), dev[1], 1e-6).view(T, n_q, D), cos.cuda(), sin.cuda())
+    # the separate kernels sum a head's squares in another order: one bf16 step
+    assert torch.allclose(q2.float(), q1.float(), rtol=2 ** -7, atol=2 ** -8) and k2.shape == (T, n_kv, D)
