@@ -153,6 +153,19 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (EPI != EPI_SYMM) return true;
     return (nb + 1) * BN > mb * kTile2M;
   };
+  // grouped-K (per-expert weight gradients): tile t = (expert, m-block, n-block), K runs over the expert's own rows
+  const int total_tiles = p.group_k ? n_tiles * p.n_experts : n_tiles;
+  auto decode = [&](int t, int& e, int& mb, int& nb, int& kb_lo, int& kb_n) {
+    e = 0; kb_lo = 0; kb_n = n_kb;
+    if (p.group_k) {
+      e = t / n_tiles;
+      t -= e * n_tiles;
+      const int r0 = p.expert_start[e], r1 = p.expert_start[e + 1];
+      kb_lo = r0 / BK;
+      kb_n = (r1 - r0) / BK;
+    }
+    tile_coords(t, tiles_m, tiles_n, mb, nb, p.group_m);
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -161,14 +174,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tma_prefetch_desc(&tmB);
       uint32_t it = 0;
       bool ok = true;
-      for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-        int mb, nb;
-        tile_coords(t, tiles_m, tiles_n, mb, nb, p.group_m);
+      for (int t = pair; t < total_tiles && ok; t += n_pairs) {
+        int ex, mb, nb, kb_lo, kb_n;
+        decode(t, ex, mb, nb, kb_lo, kb_n);
         if (!tile_active(mb, nb)) continue;
         const int m0 = mb * kTile2M + static_cast<int>(cta) * 128;
         // SWIGLU: the leader stages gate rows, the second CTA the matching up rows
         const int n0 = (EPI == EPI_SWIGLU) ? nb * 128 : nb * BN + static_cast<int>(cta) * 128;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        for (int kb = 0; kb < kb_n; ++kb, ++it) {
           const int s = it % kStages2;
           const uint32_t ph = (it / kStages2) & 1;
           if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_word)) { ok = false; break; }
@@ -176,7 +189,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const uint32_t sb = sa + kHalfBytes;
           const uint32_t fb = map_to_cta(smem_u32(&full_bar[s]), 0);
           if (cta == 0) mbar_expect_tx(&full_bar[s], 2 * kStage2Bytes);
-          const int k0 = kb * BK;
+          const int k0 = (kb_lo + kb) * BK;
           if (!p.a_mn_major) {
             tma2_load_2d(sa, &tmA, fb, k0, m0);
           } else if (p.a_mn3d) {
@@ -204,16 +217,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const uint32_t idesc = umma_idesc_bf16_major(kTile2M, BN, p.a_mn_major, p.b_mn_major);
       uint32_t it = 0, tl = 0;
       bool ok = true;
-      for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-        int mb, nb;
-        tile_coords(t, tiles_m, tiles_n, mb, nb, p.group_m);
+      for (int t = pair; t < total_tiles && ok; t += n_pairs) {
+        int ex, mb, nb, kb_lo, kb_n;
+        decode(t, ex, mb, nb, kb_lo, kb_n);
         if (!tile_active(mb, nb)) continue;
         const int acc = tl & 1;
         const uint32_t acc_ph = (tl >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1, abort_word)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < n_kb; ++kb, ++it) {
+        for (int kb = 0; kb < kb_n; ++kb, ++it) {
           const int s = it % kStages2;
           const uint32_t ph = (it / kStages2) & 1;
           if (!mbar_wait(&full_bar[s], ph, abort_word)) { ok = false; break; }
@@ -250,9 +263,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     uint32_t tl = 0;
     int buf = 0;
     bool ok = true;
-    for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-      int mb, nb;
-      tile_coords(t, tiles_m, tiles_n, mb, nb, p.group_m);
+    for (int t = pair; t < total_tiles && ok; t += n_pairs) {
+      int ex, mb, nb, kb_lo, kb_n;
+      decode(t, ex, mb, nb, kb_lo, kb_n);
       if (!tile_active(mb, nb)) continue;
       const int acc = tl & 1;
       const uint32_t acc_ph = (tl >> 1) & 1;
@@ -278,7 +291,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             const int col0 = n0 + c64 * 64 + h * 32;
             float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+            for (int j = 0; j < 32; ++j) v[j] = kb_n == 0 ? 0.f : __uint_as_float(r[j]) * p.alpha;  // an expert without rows: zero
             if (EPI == EPI_PLAIN && p.bias != nullptr) add_bias32(v, p.bias, col0, p.N);
             if ((EPI == EPI_PLAIN || EPI == EPI_SYMM) && p.cin != nullptr && row < p.M) {
               const __nv_bfloat16* crow = p.cin + static_cast<size_t>(row) * p.ldcin + col0;
@@ -347,7 +360,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(&tmC, slab, n0 + c64 * 64, m0 + q * 32);
+            if (p.group_k) tma_store_3d(&tmC, slab, n0 + c64 * 64, m0 + q * 32, ex);
+            else tma_store_2d(&tmC, slab, n0 + c64 * 64, m0 + q * 32);
             tma_store_commit();
           }
           buf ^= 1;

@@ -950,7 +950,7 @@ static int launch2(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorM
   }
   int pairs = g_pair_clusters;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
-  const int tiles = p.n_tiles_m * p.n_tiles_n;
+  const int tiles = p.n_tiles_m * p.n_tiles_n * (p.group_k ? p.n_experts : 1);
   if (tiles < pairs) pairs = tiles;
   if (pairs <= 0) return 0;
   GemmParams pp = p;
@@ -1269,20 +1269,29 @@ int b200_gemm_grouped_wgrad_bf16(const void* A, const void* B, void* dW, const v
   if (M <= 0 || N <= 0 || E <= 0) return 0;
   if ((lda | ldb) & 7) return -10;
   CUtensorMap tA, tB, tC;
-  int rc = make_map(&tA, A, rows, M, lda, 64, BK, true);
-  rc |= make_map(&tB, B, rows, N, ldb, 64, BK, true);
+  // CTA pairs (256 x 256 tiles) wherever the shape allows, like the plain products: the tiles of an expert do not depend on
+  // its row count, so nothing is wasted.  128 experts of 576 rows, 1536 x 2048 and 2048 x 768: 0.95 PFLOP/s on single CTAs.
+  const bool pair = pair_shape_ok(M, N);
+  int a3d = M % 64 == 0 && lda >= M, b3d = N % 64 == 0 && ldb >= N;
+  if (a3d && make_map_mn3d(&tA, A, rows, M, lda, 2) != 0) a3d = 0;
+  if (b3d && make_map_mn3d(&tB, B, rows, N, ldb, pair ? 2 : BN / 64) != 0) b3d = 0;
+  int rc = 0;
+  if (!a3d) rc |= make_map(&tA, A, rows, M, lda, 64, BK, true);
+  if (!b3d) rc |= make_map(&tB, B, rows, N, ldb, 64, BK, true);
   rc |= make_map_e3(&tC, dW, E, M, N, 64, 32);
   if (rc != 0) return rc;
   GemmParams p{};
   p.M = M; p.N = N; p.K = rows;
   p.a_mn_major = 1; p.b_mn_major = 1;
+  p.a_mn3d = a3d; p.b_mn3d = b3d;
   p.alpha = 1.f;
-  p.n_tiles_m = (M + BM - 1) / BM;
+  p.n_tiles_m = pair ? (M + kTile2M - 1) / kTile2M : (M + BM - 1) / BM;
   p.n_tiles_n = (N + BN - 1) / BN;
   p.expert_start = static_cast<const int*>(expert_start);
   p.group_k = 1;
   p.n_experts = E;
   p.status = status;
+  if (pair) return launch2<EPI_PLAIN>(tA, tB, tB, tC, tC, tC, p, 0, stream);
   return launch<EPI_PLAIN>(tA, tB, tB, tC, tC, tC, p, 0, stream);
 }
 

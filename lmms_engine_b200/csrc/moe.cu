@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(256) moe_rows_kernel(const int* __restrict__ t
 
 // ---------------------------------------------------------------------------- combine & friends
 // out[t, :] = sum_j (w ? w[t,j] : 1) * src[row_of[t,j], :]
+// Four rows' loads are issued before the first is used: one row after the other left the sum waiting for DRAM k times.
 __global__ void moe_combine_kernel(const bf16* __restrict__ src, const int* __restrict__ row_of,
                                    const float* __restrict__ w, bf16* __restrict__ out, int T, int k, int H,
                                    long n_src, int* status) {
@@ -188,17 +189,25 @@ __global__ void moe_combine_kernel(const bf16* __restrict__ src, const int* __re
     const long t = i / vec;
     const int c = (i - t * vec) * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = 0; j < k; ++j) {
-      const int row = row_of[t * k + j];
-      if (row < 0 || !index_in_bounds(row, n_src, status)) continue;
-      const float wt = w != nullptr ? w[t * k + j] : 1.f;
-      const V8 v = *reinterpret_cast<const V8*>(src + static_cast<size_t>(row) * H + c);
+    for (int j0 = 0; j0 < k; j0 += 4) {
+      V8 v[4];
+      float wt[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 f = unpack_bf16x2(v.w[q]);
-        acc[2 * q] += wt * f.x;
-        acc[2 * q + 1] += wt * f.y;
+      for (int e = 0; e < 4; ++e) {
+        const int row = j0 + e < k ? row_of[t * k + j0 + e] : -1;
+        const bool ok = row >= 0 && index_in_bounds(row, n_src, status);
+        wt[e] = !ok ? 0.f : w != nullptr ? w[t * k + j0 + e] : 1.f;
+        v[e].w[0] = v[e].w[1] = v[e].w[2] = v[e].w[3] = 0u;
+        if (ok) v[e] = *reinterpret_cast<const V8*>(src + static_cast<size_t>(row) * H + c);
       }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = unpack_bf16x2(v[e].w[q]);
+          acc[2 * q] += wt[e] * f.x;
+          acc[2 * q + 1] += wt[e] * f.y;
+        }
     }
     V8 o;
 #pragma unroll

@@ -245,8 +245,9 @@ class _GroupedMLPFn(torch.autograd.Function):
         E, two_i, _ = gate_up.shape
         inter = two_i // 2
         h = torch.empty((rows, inter), dtype=xp.dtype, device=xp.device)
-        # unused tiles are never written by the kernels: keep them finite
-        gu = torch.zeros((rows, two_i), dtype=xp.dtype, device=xp.device)
+        # unused tiles are written by no kernel and read by none but the elementwise passes over the same tiles: products and
+        # sums take the rows of the experts' own tiles only
+        gu = torch.empty((rows, two_i), dtype=xp.dtype, device=xp.device)
         st = _cuda.status_word(xp.device)
         _cuda.call("b200_gemm_grouped_swiglu_bf16", xp.data_ptr(), gate_up.data_ptr(), h.data_ptr(), gu.data_ptr(),
                    perm.tile_expert.data_ptr(), rows, inter, H, E, xp.stride(0), st.data_ptr(), _cuda.stream())
