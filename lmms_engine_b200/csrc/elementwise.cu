@@ -735,15 +735,23 @@ __device__ __forceinline__ bf16x4 to_bf16x4(float a, float b, float c, float d) 
   return r;
 }
 
+// four gradient elements of either type
+__device__ __forceinline__ float4 grad4(const float4& g) { return g; }
+__device__ __forceinline__ float4 grad4(const bf16x4& g) {
+  const float2 a = unpack_bf16x2(g.lo), b = unpack_bf16x2(g.hi);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename G4>
 __global__ void adamw_vec_kernel(float4* __restrict__ p32, bf16x4* __restrict__ p16, float4* __restrict__ m,
-                                 float4* __restrict__ v, const float4* __restrict__ g, long nv, float lr, float beta1,
+                                 float4* __restrict__ v, const G4* __restrict__ g, long nv, float lr, float beta1,
                                  float beta2, float eps, float wd, float bc1, float bc2, const float* gscale,
                                  const int* skip) {
   if (skip != nullptr && *skip) return;
   const float gs = gscale != nullptr ? *gscale : 1.f;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < nv;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float4 g4 = g[i];
+    const float4 g4 = grad4(g[i]);
     float4 p4 = p32[i], m4 = m[i], v4 = v[i];
     const float gi[4] = {g4.x * gs, g4.y * gs, g4.z * gs, g4.w * gs};
     float pi[4] = {p4.x, p4.y, p4.z, p4.w}, mi[4] = {m4.x, m4.y, m4.z, m4.w}, vi[4] = {v4.x, v4.y, v4.z, v4.w};
@@ -761,7 +769,8 @@ __global__ void adamw_vec_kernel(float4* __restrict__ p32, bf16x4* __restrict__ 
   }
 }
 
-__global__ void muon_momentum_vec_kernel(float4* __restrict__ mom, const float4* __restrict__ g, bf16x4* __restrict__ out,
+template <typename G4>
+__global__ void muon_momentum_vec_kernel(float4* __restrict__ mom, const G4* __restrict__ g, bf16x4* __restrict__ out,
                                          float* __restrict__ sumsq, long nv, float beta, int nesterov,
                                          const float* gscale) {
   __shared__ float red[32];
@@ -769,7 +778,7 @@ __global__ void muon_momentum_vec_kernel(float4* __restrict__ mom, const float4*
   float acc = 0.f;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < nv;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float4 g4 = g[i];
+    const float4 g4 = grad4(g[i]);
     const float4 m4 = mom[i];
     const float gi[4] = {g4.x * gs, g4.y * gs, g4.z * gs, g4.w * gs};
     float mi[4] = {m4.x, m4.y, m4.z, m4.w}, u[4];
@@ -835,6 +844,35 @@ __global__ void sumsq_part_vec_kernel(const float4* __restrict__ g, float* __res
     acc += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
   }
   if (blockIdx.x == 0 && threadIdx.x < n_tail) acc += tail[threadIdx.x] * tail[threadIdx.x];
+  acc = block_sum<256>(acc, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+}
+
+__device__ __forceinline__ float sq8(const uint4& w) {
+  const float2 a = unpack_bf16x2(w.x), b = unpack_bf16x2(w.y), c = unpack_bf16x2(w.z), d = unpack_bf16x2(w.w);
+  return (a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y) + (c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y);
+}
+// The same over bf16, eight elements a load and eight loads in flight: two CTAs per SM (the partials) need 64 KB per SM under
+// way to reach HBM's rate.
+__global__ void sumsq_part_bf16_kernel(const uint4* __restrict__ g, float* __restrict__ part, long nv, const bf16* tail, int n_tail) {
+  __shared__ float red[32];
+  float acc = 0.f;
+  const long stride = static_cast<long>(gridDim.x) * blockDim.x;
+  long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+  for (; i + 7 * stride < nv; i += 8 * stride) {
+    uint4 w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = g[i + j * stride];
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += sq8(w[j]);
+    acc += s;
+  }
+  for (; i < nv; i += stride) acc += sq8(g[i]);
+  if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < n_tail) {
+    const float t = __bfloat162float(tail[threadIdx.x]);
+    acc += t * t;
+  }
   acc = block_sum<256>(acc, red);
   if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
@@ -1172,14 +1210,22 @@ int b200_adamw(void* p32, void* p16, void* m, void* v, const void* g, int g_is_f
                float beta2, float eps, float wd, float bc1, float bc2, const void* gscale, const void* skip,
                cudaStream_t st) {
   if (n <= 0) return 0;
-  if (g_is_fp32 && n >= 4 && aligned_to(p32, 16) && aligned_to(p16, 8) && aligned_to(m, 16) && aligned_to(v, 16) && aligned_to(g, 16)) {
+  if (n >= 4 && aligned_to(p32, 16) && aligned_to(p16, 8) && aligned_to(m, 16) && aligned_to(v, 16) && aligned_to(g, g_is_fp32 ? 16 : 8)) {
     const long nv = n / 4, done = nv * 4;
-    adamw_vec_kernel<<<grid_for(nv, 256), 256, 0, st>>>((float4*)p32, (bf16x4*)p16, (float4*)m, (float4*)v, (const float4*)g, nv, lr,
-                                                        beta1, beta2, eps, wd, bc1, bc2, (const float*)gscale, (const int*)skip);
-    if (done < n)
-      adamw_kernel<float><<<1, 32, 0, st>>>((float*)p32 + done, p16 ? (bf16*)p16 + done : nullptr, (float*)m + done, (float*)v + done,
-                                            (const float*)g + done, n - done, lr, beta1, beta2, eps, wd, bc1, bc2,
-                                            (const float*)gscale, (const int*)skip);
+    bf16* tail16 = p16 ? (bf16*)p16 + done : nullptr;
+    if (g_is_fp32) {
+      adamw_vec_kernel<<<grid_for(nv, 256), 256, 0, st>>>((float4*)p32, (bf16x4*)p16, (float4*)m, (float4*)v, (const float4*)g, nv, lr,
+                                                          beta1, beta2, eps, wd, bc1, bc2, (const float*)gscale, (const int*)skip);
+      if (done < n)
+        adamw_kernel<float><<<1, 32, 0, st>>>((float*)p32 + done, tail16, (float*)m + done, (float*)v + done, (const float*)g + done,
+                                              n - done, lr, beta1, beta2, eps, wd, bc1, bc2, (const float*)gscale, (const int*)skip);
+    } else {
+      adamw_vec_kernel<<<grid_for(nv, 256), 256, 0, st>>>((float4*)p32, (bf16x4*)p16, (float4*)m, (float4*)v, (const bf16x4*)g, nv, lr,
+                                                          beta1, beta2, eps, wd, bc1, bc2, (const float*)gscale, (const int*)skip);
+      if (done < n)
+        adamw_kernel<bf16><<<1, 32, 0, st>>>((float*)p32 + done, tail16, (float*)m + done, (float*)v + done, (const bf16*)g + done,
+                                             n - done, lr, beta1, beta2, eps, wd, bc1, bc2, (const float*)gscale, (const int*)skip);
+    }
     return CHECK_LAUNCH();
   }
   int blocks = grid_for(n, 256);
@@ -1197,10 +1243,14 @@ int b200_muon_momentum(void* mom, const void* g, int g_is_fp32, void* out, void*
                        int nesterov, const void* gscale, float eps, cudaStream_t st) {
   if (n <= 0) return 0;
   cudaMemsetAsync(sumsq, 0, sizeof(float), st);
-  if (g_is_fp32 && n % 8 == 0 && aligned_to(mom, 16) && aligned_to(g, 16) && aligned_to(out, 16)) {
+  if (n % 8 == 0 && aligned_to(mom, 16) && aligned_to(g, g_is_fp32 ? 16 : 8) && aligned_to(out, 16)) {
     // whole matrices: their element counts are multiples of 8 in every supported layout
-    muon_momentum_vec_kernel<<<grid_for(n / 4, 256, 4), 256, 0, st>>>((float4*)mom, (const float4*)g, (bf16x4*)out, (float*)sumsq,
-                                                                     n / 4, beta, nesterov, (const float*)gscale);
+    if (g_is_fp32)
+      muon_momentum_vec_kernel<<<grid_for(n / 4, 256, 4), 256, 0, st>>>((float4*)mom, (const float4*)g, (bf16x4*)out, (float*)sumsq,
+                                                                       n / 4, beta, nesterov, (const float*)gscale);
+    else
+      muon_momentum_vec_kernel<<<grid_for(n / 4, 256, 4), 256, 0, st>>>((float4*)mom, (const bf16x4*)g, (bf16x4*)out, (float*)sumsq,
+                                                                       n / 4, beta, nesterov, (const float*)gscale);
     scale_by_norm_vec_kernel<<<grid_for(n / 8, 256, 4), 256, 0, st>>>((uint4*)out, (const float*)sumsq, n / 8, eps);
     return CHECK_LAUNCH();
   }
@@ -1243,6 +1293,13 @@ int b200_sumsq(const void* g, int g_is_fp32, long n, void* part, void* out, int 
     blocks = grid_for(nv, 256, 2);  // the partials scratch holds b200_num_partials() = 2 per SM
     sumsq_part_vec_kernel<<<blocks, 256, 0, st>>>((const float4*)g, (float*)part, nv, (const float*)g + nv * 4,
                                                   static_cast<int>(n - nv * 4));
+    sumsq_finish_kernel<<<1, 256, 0, st>>>((const float*)part, (float*)out, blocks, accumulate);
+    return CHECK_LAUNCH();
+  }
+  if (!g_is_fp32 && n >= 8 && aligned_to(g, 16)) {
+    const long nv = n / 8;
+    blocks = grid_for(nv, 256, 2);
+    sumsq_part_bf16_kernel<<<blocks, 256, 0, st>>>((const uint4*)g, (float*)part, nv, (const bf16*)g + nv * 8, static_cast<int>(n - nv * 8));
     sumsq_finish_kernel<<<1, 256, 0, st>>>((const float*)part, (float*)out, blocks, accumulate);
     return CHECK_LAUNCH();
   }

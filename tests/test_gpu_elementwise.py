@@ -374,3 +374,23 @@ def test_rope_in_fours(T, H, D, rot):
     b.backward(dy)
     for u, v in ((a.detach(), b.detach()), (x.grad, y.grad)):
         assert torch.allclose(u.float(), v.float(), rtol=2 ** -7, atol=2 ** -20)
+
+
+@pytest.mark.parametrize("n,shift", [(4096, 0), (4099, 0), (5, 0), (4096, 1), (4096, 4)])
+def test_bf16_gradient_passes_at_any_alignment(n, shift):
+    """16-byte passes over bf16 gradients, their remainders and the scalar passes off the boundary: the same elements."""
+    from lmms_engine_b200.ops import optim
+
+    torch.manual_seed(0)
+    g = torch.randn(n + 8, device="cuda").bfloat16()[shift:shift + n]
+    p, m, v = (torch.randn(n + 8, device="cuda").abs()[shift:shift + n] for _ in range(3))
+    want = [t.clone() for t in (p, m, v)]
+    p16 = torch.empty(n + 8, device="cuda", dtype=torch.bfloat16)[shift:shift + n]
+    optim.adamw_step(p, p16, m, v, g, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, wd=0.1, step=2)
+    optim.adamw_step(want[0], None, want[1], want[2], g.float(), lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, wd=0.1, step=2)
+    for a, b in zip((p, m, v), want):
+        assert torch.allclose(a, b, rtol=1e-6, atol=1e-7)
+    assert torch.equal(p16, p.bfloat16())
+    ss = torch.zeros(1, device="cuda")
+    optim.sumsq_(g, ss, False)
+    assert abs(float(ss) - float(g.double().pow(2).sum())) < 1e-5 * float(ss)
