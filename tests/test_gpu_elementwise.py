@@ -376,6 +376,38 @@ def test_rope_in_fours(T, H, D, rot):
         assert torch.allclose(u.float(), v.float(), rtol=2 ** -7, atol=2 ** -20)
 
 
+@pytest.mark.parametrize("rows,H", [(1, 520), (7, 1024), (9, 1032), (2500, 1152), (33, 1280), (17, 1288), (1300, 2048), (5, 8)])
+@pytest.mark.parametrize("form", ["rms", "rms_res", "layer"])
+def test_norm_backward_warp_rows(rows, H, form):
+    """One warp per row: fewer rows than CTAs and warps, several rows per warp, widths at and next to the register tiles.
+    Against fp32 autograd; dx carries one bf16 rounding, dw is an fp32 sum rounded once."""
+    from lmms_engine_b200.ops import norm
+
+    torch.manual_seed(0)
+    x, w, b, res, dy, dres = (torch.randn(s, device="cuda").bfloat16() for s in ((rows, H), (H,), (H,), (rows, H), (rows, H), (rows, H)))
+    dev = [t.clone().requires_grad_() for t in (x, w, b, res)]
+    ref = [t.float().requires_grad_() for t in (x, w, b, res)]
+    if form == "layer":
+        norm.layernorm(dev[0], dev[1], dev[2]).backward(dy)
+        norm.layernorm_ref(ref[0], ref[1], ref[2], 1e-6).backward(dy.float())
+        n = 3
+    elif form == "rms":
+        norm.rmsnorm(dev[0], dev[1]).backward(dy)
+        norm.rmsnorm_ref(ref[0], ref[1], 1e-6).backward(dy.float())
+        n = 2
+    else:
+        y, s = norm.rmsnorm(dev[0], dev[1], residual=dev[3])
+        torch.autograd.backward([y, s], [dy, dres])
+        xr = (ref[0] + ref[3])
+        xr = xr + (xr.bfloat16().float() - xr).detach()  # the sum is stored in bf16
+        z = xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-6) * ref[1]
+        torch.autograd.backward([z, xr], [dy.float(), dres.float()])
+        n = 2
+    for d, r in zip(dev[:n], ref[:n]):
+        assert torch.isfinite(d.grad).all()
+        assert (d.grad.float() - r.grad).norm() < 2 ** -7 * r.grad.norm() + 1e-5
+
+
 @pytest.mark.parametrize("n,shift", [(4096, 0), (4099, 0), (5, 0), (4096, 1), (4096, 4)])
 def test_bf16_gradient_passes_at_any_alignment(n, shift):
     """16-byte passes over bf16 gradients, their remainders and the scalar passes off the boundary: the same elements."""
