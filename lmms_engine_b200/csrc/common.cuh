@@ -332,6 +332,21 @@ __device__ __forceinline__ bool index_in_bounds(long idx, long limit, int* statu
 #define B200_DBG_INDEX(idx, limit, status) true
 #endif
 
+// ---------------------------------------------------------------- index arithmetic
+// i = q * d + r.  A 64-bit division is about a hundred instructions; flat indices nearly always fit 32 bits (`narrow`, the same
+// for the whole launch), and the passes that split one per 16 bytes were bound by it rather than by memory.
+__device__ __forceinline__ void split_index(long i, int d, bool narrow, long& q, int& r) {
+  if (narrow) {
+    const unsigned u = static_cast<unsigned>(i), v = u / static_cast<unsigned>(d);
+    q = v;
+    r = static_cast<int>(u - v * static_cast<unsigned>(d));
+  } else {
+    q = i / d;
+    r = static_cast<int>(i - q * d);
+  }
+}
+__device__ __forceinline__ bool fits32(long n) { return n < (1L << 31); }
+
 // ---------------------------------------------------------------- misc numeric helpers
 // 2^x on the special-function unit, one instruction (exp2f() adds a range fix-up for denormal results that a softmax does
 // not need): 2^-inf = +0.

@@ -592,6 +592,10 @@ __device__ __forceinline__ float group_sum(float v, int lanes) {
   for (int o = lanes >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+__device__ __forceinline__ void load_f4(const float* p, float (&v)[4]) {
+  const float4 u = *reinterpret_cast<const float4*>(p);
+  v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+}
 template <int D>
 __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
                                                                const bf16* __restrict__ wq, const bf16* __restrict__ wk,
@@ -601,16 +605,18 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __res
   constexpr int L = D / 8, HPW = 32 / L;   // lanes per head, heads per warp
   const int lane = threadIdx.x & 31, l = lane % L, heads = n_q + n_kv;
   const long total = T * heads;
+  const bool narrow = fits32(total);
   const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
   // every lane of a warp takes part in the shuffles: a group past the end computes on the last head and stores nothing
   for (long w0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * HPW; w0 < total; w0 += warps * HPW) {
     const long idx = w0 + lane / L;
     const bool live = idx < total;
     const long at = live ? idx : total - 1;
-    const long t = at / heads;
-    const int h = static_cast<int>(at - t * heads);
+    long t;
+    int h;
+    split_index(at, heads, narrow, t, h);
     const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
-    float a[4], b[4], ca[4], sa[4];
+    float a[4], b[4];
     load_w<4>(xp, a);
     load_w<4>(xp + D / 2, b);
     float ss = 0.f;
@@ -622,17 +628,19 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __res
     const bf16* w = (h < n_q ? wq : wk) + 4 * l;
     load_w<4>(w, wa);
     load_w<4>(w + D / 2, wb);
-    const float* c = cosb + t * D + 4 * l;
-    const float* s = sinb + t * D + 4 * l;
+    float c[4], s[4], c2[4], s2[4];
+    load_f4(cosb + t * D + 4 * l, c);
+    load_f4(sinb + t * D + 4 * l, s);
+    load_f4(cosb + t * D + D / 2 + 4 * l, c2);
+    load_f4(sinb + t * D + D / 2 + 4 * l, s2);
     float o1[4], o2[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       // the normalised head is a bf16 tensor of its own in the separate form: rounded here too
       const float x1 = __bfloat162float(__float2bfloat16(a[j] * r * wa[j]));
       const float x2 = __bfloat162float(__float2bfloat16(b[j] * r * wb[j]));
-      ca[j] = c[j]; sa[j] = s[j];
-      o1[j] = x1 * ca[j] - x2 * sa[j];
-      o2[j] = x2 * c[D / 2 + j] + x1 * s[D / 2 + j];
+      o1[j] = x1 * c[j] - x2 * s[j];
+      o2[j] = x2 * c2[j] + x1 * s2[j];
     }
     if (live) {
       bf16* yp = y + t * ldy + static_cast<long>(h) * D + 4 * l;
@@ -655,13 +663,15 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
   __syncthreads();
   float dw[2][8] = {};
   const long total = T * heads;
+  const bool narrow = fits32(total);
   const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
   for (long w0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * HPW; w0 < total; w0 += warps * HPW) {
     const long idx = w0 + lane / L;
     const bool live = idx < total;
     const long at = live ? idx : total - 1;
-    const long t = at / heads;
-    const int h = static_cast<int>(at - t * heads);
+    long t;
+    int h;
+    split_index(at, heads, narrow, t, h);
     const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
     bf16* dp = d + t * ldd + static_cast<long>(h) * D + 4 * l;
     float a[4], b[4], da[4], db[4], wa[4], wb[4];
@@ -673,21 +683,26 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
     const bf16* w = (is_q ? wq : wk) + 4 * l;
     load_w<4>(w, wa);
     load_w<4>(w + D / 2, wb);
-    const float* c = cosb + t * D + 4 * l;
-    const float* s = sinb + t * D + 4 * l;
+    float c[4], s[4], c2[4], s2[4];
+    load_f4(cosb + t * D + 4 * l, c);
+    load_f4(sinb + t * D + 4 * l, s);
+    load_f4(cosb + t * D + D / 2 + 4 * l, c2);
+    load_f4(sinb + t * D + D / 2 + 4 * l, s2);
     const float r = rstd[at];
     float dot = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       // transposed rotation, rounded where the separate form stores it
-      const float g1 = __bfloat162float(__float2bfloat16(da[j] * c[j] + db[j] * s[D / 2 + j]));
-      const float g2 = __bfloat162float(__float2bfloat16(db[j] * c[D / 2 + j] - da[j] * s[j]));
+      const float g1 = __bfloat162float(__float2bfloat16(da[j] * c[j] + db[j] * s2[j]));
+      const float g2 = __bfloat162float(__float2bfloat16(db[j] * c2[j] - da[j] * s[j]));
       a[j] *= r;
       b[j] *= r;
-      if (live) {
-        dw[is_q ? 0 : 1][j] += g1 * a[j];
-        dw[is_q ? 0 : 1][4 + j] += g2 * b[j];
-      }
+      // an index that depends on the head would put the sums into local memory
+      const float g1a = live ? g1 * a[j] : 0.f, g2b = live ? g2 * b[j] : 0.f;
+      dw[0][j] += is_q ? g1a : 0.f;
+      dw[0][4 + j] += is_q ? g2b : 0.f;
+      dw[1][j] += is_q ? 0.f : g1a;
+      dw[1][4 + j] += is_q ? 0.f : g2b;
       da[j] = g1 * wa[j];
       db[j] = g2 * wb[j];
       dot += da[j] * a[j] + db[j] * b[j];
@@ -1053,10 +1068,13 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ src, const int64_t* 
                                    bf16* __restrict__ out, long n_out, int H, long n_src, int* status) {
   const int vec = H / 8;
   const long total = n_out * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vec;
-    const int c = (i - r * vec) * 8;
+    long r;
+    int c;
+    split_index(i, vec, narrow, r, c);
+    c *= 8;
     const int64_t s = idx[r];
     bf16x8 v;
     v.w[0] = v.w[1] = v.w[2] = v.w[3] = 0u;
@@ -1068,10 +1086,13 @@ __global__ void scatter_rows_kernel(const bf16* __restrict__ src, const int64_t*
                                     bf16* __restrict__ out, long n_src, int H, int add, long n_out, int* status) {
   const int vec = H / 8;
   const long total = n_src * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vec;
-    const int c = (i - r * vec) * 8;
+    long r;
+    int c;
+    split_index(i, vec, narrow, r, c);
+    c *= 8;
     const int64_t d = idx[r];
     if (d < 0 || !index_in_bounds(d, n_out, status)) continue;
     float v[8];
@@ -1296,7 +1317,7 @@ int b200_rope_apply(const void* x, void* y, const void* cosb, const void* sinb, 
 }
 
 // Partial weight gradients that b200_qk_norm_rope_bwd writes: part [this][2][D] fp32.
-int b200_qk_norm_rope_parts() { return 296; }
+int b200_qk_norm_rope_parts() { return num_sms() * 3; }  // as many CTAs as its registers keep resident
 
 // q and k heads of rows x [T, >= (n_q + n_kv) * D] into y; D 64 or 128, rows on 16-byte boundaries, rstd [T, n_q + n_kv].
 int b200_qk_norm_rope_fwd(const void* x, void* y, const void* wq, const void* wk, const void* cosb, const void* sinb, void* rstd,

@@ -184,10 +184,13 @@ __global__ void moe_combine_kernel(const bf16* __restrict__ src, const int* __re
                                    long n_src, int* status) {
   const int vec = H / 8;
   const long total = static_cast<long>(T) * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long t = i / vec;
-    const int c = (i - t * vec) * 8;
+    long t;
+    int c;
+    split_index(i, vec, narrow, t, c);
+    c *= 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int j0 = 0; j0 < k; j0 += 4) {
       V8 v[4];
@@ -222,10 +225,13 @@ __global__ void moe_combine_bwd_src_kernel(const bf16* __restrict__ dout, const 
                                            long rows, int H, long n_tok, int* status) {
   const int vec = H / 8;
   const long total = rows * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vec;
-    const int c = (i - r * vec) * 8;
+    long r;
+    int c;
+    split_index(i, vec, narrow, r, c);
+    c *= 8;
     const int64_t t = token_of_row[r];
     V8 o;
     o.w[0] = o.w[1] = o.w[2] = o.w[3] = 0u;
@@ -302,10 +308,13 @@ __global__ void moe_row_scale_dot_kernel(const bf16* __restrict__ g, long ldg, c
 __global__ void swiglu_cat_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, long rows, int I) {
   const int vec = I / 8;
   const long total = rows * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vec;
-    const int c = (i - r * vec) * 8;
+    long r;
+    int c;
+    split_index(i, vec, narrow, r, c);
+    c *= 8;
     const V8 g = *reinterpret_cast<const V8*>(gu + r * 2 * I + c);
     const V8 u = *reinterpret_cast<const V8*>(gu + r * 2 * I + I + c);
     V8 o;
@@ -320,10 +329,13 @@ __global__ void swiglu_cat_fwd_kernel(const bf16* __restrict__ gu, bf16* __restr
 __global__ void swiglu_cat_bwd_kernel(const bf16* __restrict__ dh, bf16* gu, long rows, int I) {
   const int vec = I / 8;
   const long total = rows * vec;
+  const bool narrow = fits32(total);
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vec;
-    const int c = (i - r * vec) * 8;
+    long r;
+    int c;
+    split_index(i, vec, narrow, r, c);
+    c *= 8;
     const V8 g = *reinterpret_cast<const V8*>(gu + r * 2 * I + c);
     const V8 u = *reinterpret_cast<const V8*>(gu + r * 2 * I + I + c);
     const V8 d = *reinterpret_cast<const V8*>(dh + r * I + c);

@@ -196,6 +196,7 @@ def _fused_rows_ok(qkv, cos, sin, n_q, n_kv, D, wq, wk) -> bool:
             and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and D % 8 == 0 and D <= 128
             and n_q % n_kv == 0 and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
             and cos.shape == sin.shape == (qkv.shape[0], D) and not (cos.requires_grad or sin.requires_grad)
+            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0
             and (wq is None) == (wk is None) and (wq is None or (D in (64, 128) and plain(wq) and plain(wk))))
 
 
