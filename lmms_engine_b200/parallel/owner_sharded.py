@@ -529,7 +529,7 @@ class OwnerShardedRuntime:
         if self._lanes is None:
             n = 1
             if self.P.is_cuda:
-                n = max(1, int(os.environ.get("LMMS_B200_MUON_LANES", "4")))
+                n = max(1, int(os.environ.get("LMMS_B200_MUON_LANES", "2")))
             sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.P.is_cuda else 0
             self._lanes = []
             for i in range(n):
