@@ -489,6 +489,55 @@ static void colsum(const float* part, float* out, int parts, int H, int accumula
   colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(part, out, parts, H, accumulate);
 }
 
+// Column sums of a bf16 matrix (bias gradients), fp32 inside, bf16 out.  A CTA takes 256 columns and every gridDim.y-th block
+// of eight rows, four rows of a warp's loads in flight; the partials are summed by colsum_bf16_finish_kernel in a fixed order.
+// Bound by reading the matrix once (the framework's reduction: 38 us for 22.4k x 1152).  Rows may be wider than N: the last
+// 16-byte piece of a row may reach into its padding, which is read and dropped.
+__global__ void __launch_bounds__(256) colsum_bf16_kernel(const bf16* __restrict__ x, long ld, float* __restrict__ part, long rows, int N) {
+  __shared__ float sm[8][256 + 8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 256 + lane * 8;
+  float acc[8] = {};
+  if (c < N) {
+    const long step = static_cast<long>(gridDim.y) * 8;
+    long r = static_cast<long>(blockIdx.y) * 8 + warp;
+    for (; r + 3 * step < rows; r += 4 * step) {
+      float v[4][8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) load8(x + (r + k * step) * ld + c, v[k]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += (v[0][j] + v[1][j]) + (v[2][j] + v[3][j]);
+    }
+    for (; r < rows; r += step) {
+      float v[8];
+      load8(x + r * ld + c, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += v[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sm[warp][lane * 8 + j] = acc[j];
+  __syncthreads();
+  const int co = blockIdx.x * 256 + threadIdx.x;
+  float s = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s += sm[q][threadIdx.x];
+  if (co < N) part[static_cast<size_t>(blockIdx.y) * N + co] = s;
+}
+__global__ void __launch_bounds__(1024) colsum_bf16_finish_kernel(const float* __restrict__ part, bf16* __restrict__ out, int parts, int N) {
+  __shared__ float sm[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  float s = 0.f;
+  if (c < N) {
+#pragma unroll 4
+    for (int p = ty; p < parts; p += 32) s += part[static_cast<size_t>(p) * N + c];
+  }
+  sm[ty][tx] = s;
+  __syncthreads();
+  const float t = warp_sum(sm[tx][ty]);
+  const int co = blockIdx.x * 32 + ty;
+  if (tx == 0 && co < N) out[co] = __float2bfloat16(t);
+}
+
 // ------------------------------------------------------------------ rotary embedding
 // cos/sin tables [T, D] (fp32) from up to three position streams.
 // mode 0: plain (pos[0]);  mode 1: sectioned M-RoPE (frequency i uses stream by section
@@ -1288,6 +1337,23 @@ int b200_norm_bwd(const void* dy, const void* x, const void* w, const void* rstd
   colsum((const float*)dw_part, (float*)dw, parts, H, accumulate, st);
   if (db != nullptr && db_part != nullptr)
     colsum((const float*)db_part, (float*)db, parts, H, accumulate, st);
+  return CHECK_LAUNCH();
+}
+
+// Rows of partials [this, N] fp32 that b200_colsum_bf16 needs.
+int b200_colsum_parts(int rows, int N) {
+  const int cols = (N + 255) / 256;
+  int parts = num_sms() * 4 / (cols > 0 ? cols : 1);
+  const int most = (rows + 31) / 32;   // at least four rows a warp
+  if (parts > most) parts = most;
+  return parts < 1 ? 1 : parts;
+}
+// out [N] bf16 = column sums of x [rows, N] bf16, rows ld elements apart (a multiple of 8, at least N rounded up to 8), 16-byte aligned.
+int b200_colsum_bf16(const void* x, long ld, void* part, void* out, int rows, int N, int parts, cudaStream_t st) {
+  if (N <= 0) return 0;
+  if (ld % 8 || ld < (N + 7) / 8 * 8 || parts < 1 || parts > 65535) return -10;
+  colsum_bf16_kernel<<<dim3((N + 255) / 256, parts), 256, 0, st>>>((const bf16*)x, ld, (float*)part, rows, N);
+  colsum_bf16_finish_kernel<<<(N + 31) / 32, 1024, 0, st>>>((const float*)part, (bf16*)out, parts, N);
   return CHECK_LAUNCH();
 }
 

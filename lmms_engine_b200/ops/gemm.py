@@ -19,6 +19,8 @@ from . import _cuda
 # the library GEMM (torch.matmul) and only the fused epilogues use the in-tree kernel.
 LINEAR_BACKEND = "tcgen05"
 
+_cuda.register("b200_colsum_parts", "elementwise", "ii")
+_cuda.register("b200_colsum_bf16", "elementwise", "plppiii" + "s")
 _cuda.register("b200_skinny_linear", "decode", "pppp" + "iii" + "lll" + "s")
 # Products of at most this many rows are bound by reading the weights once: one kernel spreads the weight rows over the
 # whole chip (csrc/decode.cu) where a 256-column tile would leave most of it idle.
@@ -144,6 +146,18 @@ def gemm_stats(x: torch.Tensor, w: torch.Tensor, alpha: float = 1.0):
     return logits, stats
 
 
+def column_sum(t: torch.Tensor) -> torch.Tensor:
+    """``t.sum(0)`` of a matrix with an fp32 accumulator, in ``t``'s dtype (the gradient of a bias)."""
+    if _ok(t) and t.shape[0] > 0 and t.shape[1] > 0 and (t.stride(0) >= (t.shape[1] + 7) // 8 * 8):
+        rows, n = t.shape
+        parts = _cuda.fn("b200_colsum_parts")(rows, n)
+        part = torch.empty((parts, n), dtype=torch.float32, device=t.device)
+        out = torch.empty(n, dtype=t.dtype, device=t.device)
+        _cuda.call("b200_colsum_bf16", t.data_ptr(), t.stride(0), part.data_ptr(), out.data_ptr(), rows, n, parts, _cuda.stream())
+        return out
+    return t.sum(0, dtype=torch.float32).to(t.dtype)
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias):
@@ -169,7 +183,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = matmul_tn(dy2, x2)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.sum(0, dtype=torch.float32).to(dy2.dtype)
+            db = column_sum(dy2)
         return dx, dw, db
 
 

@@ -143,16 +143,12 @@ class _GatedMLPFn(torch.autograd.Function):
         dwg = _gemm.matmul_tn(dg, x2) if need[1] else None
         dwu = _gemm.matmul_tn(du, x2) if need[3] else None
         has_g, has_u, has_d = ctx.biases
-        return (dx, dwg, _column_sum(dg) if has_g and need[2] else None, dwu, _column_sum(du) if has_u and need[4] else None, dwd,
-                _column_sum(dy2) if has_d and need[6] else None)
+        return (dx, dwg, _gemm.column_sum(dg) if has_g and need[2] else None, dwu, _gemm.column_sum(du) if has_u and need[4] else None, dwd,
+                _gemm.column_sum(dy2) if has_d and need[6] else None)
 
 
 def _rows16(t):
     return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
-
-
-def _column_sum(t):
-    return t.sum(0, dtype=torch.float32).to(t.dtype)
 
 
 def _padded(wd):

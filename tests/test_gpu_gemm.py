@@ -176,3 +176,17 @@ def test_gated_mlp_any_width(P, K, inter, N, biases):
     for t, f in zip(dev, first):
         if t is not None:
             assert torch.equal(t.grad, f + f)
+
+
+@pytest.mark.parametrize("rows,N,ld", [(1, 8, 8), (31, 256, 256), (33, 260, 264), (1000, 1152, 1152), (4097, 3420, 3424), (7, 1, 8)])
+def test_column_sum(rows, N, ld):
+    """Remainders of the row and column tiles; rows wider than N hold NaN that may not reach a sum.  fp32 sums, one rounding."""
+    from lmms_engine_b200.ops import gemm
+
+    torch.manual_seed(0)
+    x = torch.full((rows, ld), float("nan"), device="cuda", dtype=torch.bfloat16)
+    x[:, :N] = torch.randn(rows, N, device="cuda").bfloat16()
+    want = x[:, :N].double().sum(0)
+    got = gemm.column_sum(x[:, :N])
+    assert got.shape == (N,) and got.dtype == torch.bfloat16
+    assert ((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * rows).all()
