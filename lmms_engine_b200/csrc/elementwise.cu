@@ -789,6 +789,105 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
   for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) part[static_cast<long>(blockIdx.x) * 2 * D + i] = (&sw[0][0])[i];
 }
 
+// ------------------------------------------------------------------ gated per-head RMSNorm (output of linear attention)
+// y = bf16(rmsnorm(o) * w) * silu(z): o [T, heads, D] dense, z rows of contiguous heads at stride ldz (a column range of the
+// projection), D = 8 L.  L lanes hold a head.  As framework operations the gate took seven passes over the rows, four of them in
+// fp32, and the gate's columns were copied out first; bound by memory, each tensor is read or written once here.
+template <int L>
+__global__ void __launch_bounds__(256) gated_norm_fwd_kernel(const bf16* __restrict__ o, const bf16* __restrict__ z,
+                                                             const bf16* __restrict__ w, bf16* __restrict__ y,
+                                                             float* __restrict__ rstd_out, long rows, int heads, long ldz, float eps) {
+  constexpr int D = 8 * L, HPW = 32 / L;
+  const int lane = threadIdx.x & 31, c = (lane % L) * 8;
+  const bool narrow = fits32(rows);
+  const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
+  float wv[8];
+  load8(w + c, wv);
+  for (long w0 = (static_cast<long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * HPW; w0 < rows; w0 += warps * HPW) {
+    const long r = w0 + lane / L;
+    const bool live = r < rows;   // a group past the end takes part in the shuffles on the last row
+    const long at = live ? r : rows - 1;
+    long t;
+    int h;
+    split_index(at, heads, narrow, t, h);
+    float v[8], zv[8], out[8];
+    load8(o + at * D + c, v);
+    load8(z + t * ldz + static_cast<long>(h) * D + c, zv);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    const float rstd = rsqrtf(group_sum(ss, L) / D + eps);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[j] = __bfloat162float(__float2bfloat16(v[j] * rstd * wv[j])) * (zv[j] / (1.f + expf(-zv[j])));
+    if (live) {
+      store8(y + at * D + c, out);
+      if (lane % L == 0) rstd_out[at] = rstd;
+    }
+  }
+}
+template <int L>
+__global__ void __launch_bounds__(256) gated_norm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ o,
+                                                             const bf16* __restrict__ z, const bf16* __restrict__ w,
+                                                             const float* __restrict__ rstd_in, bf16* __restrict__ d_o,
+                                                             bf16* __restrict__ dz, float* __restrict__ part, long rows, int heads,
+                                                             long ldz) {
+  constexpr int D = 8 * L, HPW = 32 / L;
+  __shared__ float sw[8][D];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (lane % L) * 8;
+  const bool narrow = fits32(rows);
+  const long warps = static_cast<long>(gridDim.x) * 8;
+  float wv[8], dw[8];
+  load8(w + c, wv);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) dw[j] = 0.f;
+  for (long w0 = (static_cast<long>(blockIdx.x) * 8 + warp) * HPW; w0 < rows; w0 += warps * HPW) {
+    const long r = w0 + lane / L;
+    const bool live = r < rows;
+    const long at = live ? r : rows - 1;
+    long t;
+    int h;
+    split_index(at, heads, narrow, t, h);
+    float g[8], v[8], zv[8], gz[8];
+    load8(dy + at * D + c, g);
+    load8(o + at * D + c, v);
+    load8(z + t * ldz + static_cast<long>(h) * D + c, zv);
+    const float rstd = rstd_in[at];
+    float dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float sig = 1.f / (1.f + expf(-zv[j])), si = zv[j] * sig;
+      v[j] *= rstd;
+      const float n = __bfloat162float(__float2bfloat16(v[j] * wv[j]));
+      gz[j] = g[j] * n * (sig * (1.f + zv[j] * (1.f - sig)));
+      const float dn = __bfloat162float(__float2bfloat16(g[j] * si));   // a bf16 tensor in the separate form
+      if (live) dw[j] += dn * v[j];
+      g[j] = dn * wv[j];
+      dot += g[j] * v[j];
+    }
+    dot = group_sum(dot, L) / D;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] = rstd * (g[j] - v[j] * dot);
+    if (live) {
+      store8(d_o + at * D + c, g);
+      store8(dz + at * D + c, gz);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    for (int k = L; k < 32; k <<= 1) dw[j] += __shfl_xor_sync(0xffffffffu, dw[j], k);
+  if (lane < L) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sw[warp][c + j] = dw[j];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += 256) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += sw[q][i];
+    part[static_cast<long>(blockIdx.x) * D + i] = s;
+  }
+}
+
 // ------------------------------------------------------------------ SwiGLU
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ g, const bf16* __restrict__ u, bf16* __restrict__ h,
                                   long n8) {
@@ -1409,6 +1508,35 @@ int b200_qk_norm_rope_bwd(void* d, const void* x, const void* wq, const void* wk
   else
     qk_norm_rope_bwd_kernel<64><<<blocks, 256, 0, st>>>((bf16*)d, (const bf16*)x, (const bf16*)wq, (const bf16*)wk, (const float*)cosb,
                                                         (const float*)sinb, (const float*)rstd, (float*)part, T, n_q, n_kv, ldx, ldd);
+  return CHECK_LAUNCH();
+}
+
+// o, y [rows, D] dense with rows = T * heads, z [T, >= heads * D] at row stride ldz (a multiple of 8), w [D]; D = 64, 128 or 256.
+int b200_gated_norm_fwd(const void* o, const void* z, const void* w, void* y, void* rstd, long rows, int heads, int D, long ldz, float eps,
+                        cudaStream_t st) {
+  if (rows <= 0) return 0;
+  if (heads <= 0 || ldz % 8) return -10;
+  const int blocks = grid_for(rows * (D / 8), 256);
+#define GATED(L) gated_norm_fwd_kernel<L><<<blocks, 256, 0, st>>>((const bf16*)o, (const bf16*)z, (const bf16*)w, (bf16*)y, (float*)rstd, rows, heads, ldz, eps)
+  if (D == 64) GATED(8);
+  else if (D == 128) GATED(16);
+  else if (D == 256) GATED(32);
+  else return -11;
+#undef GATED
+  return CHECK_LAUNCH();
+}
+// Rows of partial weight gradients [this, D] fp32 that the backward pass writes.
+int b200_gated_norm_parts() { return num_sms() * 4; }
+int b200_gated_norm_bwd(const void* dy, const void* o, const void* z, const void* w, const void* rstd, void* d_o, void* dz, void* part,
+                        long rows, int heads, int D, long ldz, cudaStream_t st) {
+  if (heads <= 0 || ldz % 8 || rows <= 0) return -10;
+  const int blocks = b200_gated_norm_parts();
+#define GATED(L) gated_norm_bwd_kernel<L><<<blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)o, (const bf16*)z, (const bf16*)w, (const float*)rstd, (bf16*)d_o, (bf16*)dz, (float*)part, rows, heads, ldz)
+  if (D == 64) GATED(8);
+  else if (D == 128) GATED(16);
+  else if (D == 256) GATED(32);
+  else return -11;
+#undef GATED
   return CHECK_LAUNCH();
 }
 

@@ -104,7 +104,7 @@ class FlaGatedDeltaNet(nn.Module):
             w_all = F.pad(w_all, (0, 0, 0, pad))
         proj = gemm_ops.linear(x, w_all, None)
         sizes = [self.key_dim, self.key_dim, self.value_dim, self.hv, self.hv] + ([self.value_dim] if self.use_gate else [])
-        cols = torch.split(proj[:, : sum(sizes)], sizes, -1)
+        cols = torch.split(proj, sizes + ([pad] if pad else []), -1)
         q, k, v, a, b = cols[:5]
         lengths, pos_in_doc, chunks = gdn_ops.plan_for(ctx, x.device)
         live = int(pos_in_doc.numel())
@@ -122,9 +122,10 @@ class FlaGatedDeltaNet(nn.Module):
         o = gdn_ops.chunk_gated_delta_rule_packed(q, k, v, g, beta, lengths, chunks)
         if o.shape[0] < T:
             o = torch.cat([o, o.new_zeros((T - o.shape[0], self.hv, self.dv))], 0)
-        o = norm_ops.rmsnorm(o.reshape(-1, self.dv).to(x.dtype), self.o_norm.weight, self.eps)
         if self.use_gate:
-            o = (o.float() * F.silu(cols[5].reshape(-1, self.dv).float())).to(x.dtype)
+            o = norm_ops.gated_head_norm(o.reshape(T, self.hv, self.dv).to(x.dtype), cols[5], self.o_norm.weight, self.eps)
+        else:
+            o = norm_ops.rmsnorm(o.reshape(-1, self.dv).to(x.dtype), self.o_norm.weight, self.eps)
         return gemm_ops.linear(o.reshape(T, self.value_dim), _w(self.o_proj.weight), None)
 
 

@@ -164,8 +164,8 @@ class GatedDeltaNet(nn.Module):
             w_all = F.pad(w_all, (0, 0, 0, pad))
         proj = gemm_ops.linear(x, w_all, None)
         c = 2 * self.key_dim + self.value_dim
-        mixed, z = proj[:, :c], proj[:, c:c + self.value_dim]
-        b, a = proj[:, c + self.value_dim:c + self.value_dim + self.hv], proj[:, c + self.value_dim + self.hv:c + self.value_dim + 2 * self.hv]
+        # one split: its backward writes the projection's gradient once (every slice would add a zero-filled one of its own)
+        mixed, z, b, a = torch.split(proj, [c, self.value_dim, self.hv, self.hv] + ([pad] if pad else []), -1)[:4]
         A_log, dt_bias, conv_w = self.A_log, self.dt_bias, self.conv1d.weight[:, 0]
         hk, hv = self.hk, self.hv
         if getattr(ctx, "kv_cache", None) is not None:
@@ -198,12 +198,16 @@ class GatedDeltaNet(nn.Module):
         lengths, pos_in_doc, chunks = plan
         live = int(pos_in_doc.numel())  # rows after it are the padding of a sequence-parallel split
         # causal depthwise convolution inside every document, then SiLU
-        seg = gdn_ops.causal_conv_silu_packed(mixed[:live], conv_w, pos_in_doc)
+        if live < mixed.shape[0]:
+            mixed_l, g, beta = mixed[:live], g[:live], beta[:live]
+        else:
+            mixed_l = mixed
+        seg = gdn_ops.causal_conv_silu_packed(mixed_l, conv_w, pos_in_doc)
         q, k, v = torch.split(seg, [hk * self.dk, hk * self.dk, hv * self.dv], -1)
         q, k, v = q.reshape(-1, hk, self.dk), k.reshape(-1, hk, self.dk), v.reshape(-1, hv, self.dv)
         if hv // hk > 1:
             q, k = q.repeat_interleave(hv // hk, 1), k.repeat_interleave(hv // hk, 1)
-        o = gdn_ops.chunk_gated_delta_rule_packed(q, k, v, g[:live], beta[:live], lengths, chunks)
+        o = gdn_ops.chunk_gated_delta_rule_packed(q, k, v, g, beta, lengths, chunks)
         if o.shape[0] < mixed.shape[0]:
             o = torch.cat([o, o.new_zeros((mixed.shape[0] - o.shape[0], hv, self.dv))], 0)
         if ctx.sp_size > 1:
@@ -272,8 +276,7 @@ class GatedDeltaNet(nn.Module):
 
     def _finish(self, o, z, x, T):
         # RMSNorm over the head dim, gated by SiLU(z)
-        o = norm_ops.rmsnorm(o.reshape(-1, self.dv).to(x.dtype), self.norm.weight, self.eps)
-        o = (o.float() * F.silu(z.reshape(-1, self.dv).float())).to(x.dtype).reshape(T, self.value_dim)
+        o = norm_ops.gated_head_norm(o.reshape(T, self.hv, self.dv).to(x.dtype), z, self.norm.weight, self.eps)
         return gemm_ops.linear(o, _w(self.out_proj.weight), None)
 
 
@@ -294,7 +297,8 @@ class GatedAttention(nn.Module):
     def forward(self, x, ctx: PackedContext):
         T, D = x.shape[0], self.head_dim
         qg = gemm_ops.linear(x, _w(self.q_proj.weight), _w(self.q_proj.bias)).view(T, self.n_q, 2 * D)
-        q, gate = qg[..., :D], qg[..., D:].reshape(T, self.n_q * D)
+        q, gate = torch.split(qg, D, -1)
+        gate = gate.reshape(T, self.n_q * D)
         k = gemm_ops.linear(x, _w(self.k_proj.weight), _w(self.k_proj.bias)).view(T, self.n_kv, D)
         v = gemm_ops.linear(x, _w(self.v_proj.weight), _w(self.v_proj.bias)).view(T, self.n_kv, D)
         q = self.q_norm(q.reshape(-1, D)).view(T, self.n_q, D)

@@ -14,6 +14,10 @@ import torch
 
 from . import _cuda
 
+_cuda.register("b200_gated_norm_parts", "elementwise", "")
+_cuda.register("b200_gated_norm_fwd", "elementwise", "ppppp" + "liil" + "f" + "s")
+_cuda.register("b200_gated_norm_bwd", "elementwise", "pppppppp" + "liil" + "s")
+
 
 def rmsnorm_ref(x, w, eps: float, offset: float = 0.0, residual=None):
     xf = x.float()
@@ -100,3 +104,43 @@ def layernorm(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], eps: 
     if _native_ok(x, w):
         return _NormFn.apply(x, None, w, b, eps, 0.0, True)
     return layernorm_ref(x, w, b, eps)
+
+
+class _GatedNormFn(torch.autograd.Function):
+    """``rmsnorm(o) * silu(z)`` per head in one kernel per direction; the gate is read where it lies in the projection."""
+
+    @staticmethod
+    def forward(ctx, o, z, w, eps):
+        T, heads, D = o.shape
+        o = o if o.is_contiguous() and o.data_ptr() % 16 == 0 else o.clone(memory_format=torch.contiguous_format)
+        y = torch.empty((T, heads * D), dtype=o.dtype, device=o.device)
+        rstd = torch.empty(T * heads, dtype=torch.float32, device=o.device)
+        _cuda.call("b200_gated_norm_fwd", o.data_ptr(), z.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), T * heads, heads, D,
+                   z.stride(0), float(eps), _cuda.stream())
+        ctx.save_for_backward(o, z, w, rstd)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        o, z, w, rstd = ctx.saved_tensors
+        T, heads, D = o.shape
+        dy = dy if dy.is_contiguous() and dy.data_ptr() % 16 == 0 else dy.clone(memory_format=torch.contiguous_format)
+        d_o = torch.empty_like(o)
+        dz = torch.empty((T, heads * D), dtype=z.dtype, device=z.device)
+        part = torch.empty((_cuda.fn("b200_gated_norm_parts")(), D), dtype=torch.float32, device=o.device)
+        _cuda.call("b200_gated_norm_bwd", dy.data_ptr(), o.data_ptr(), z.data_ptr(), w.data_ptr(), rstd.data_ptr(), d_o.data_ptr(),
+                   dz.data_ptr(), part.data_ptr(), T * heads, heads, D, z.stride(0), _cuda.stream())
+        return d_o, dz, part.sum(0).to(w.dtype), None
+
+
+def gated_head_norm(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    """``rmsnorm(o [T, heads, D]) * silu(z [T, heads * D])`` -> ``[T, heads * D]``: the norm rounds to ``o``'s dtype, the gate is
+    evaluated in fp32."""
+    T, heads, D = o.shape
+    native = (o.is_cuda and o.dtype == z.dtype == w.dtype == torch.bfloat16 and z.is_cuda and w.is_cuda and T > 0 and D in (64, 128, 256)
+              and z.dim() == 2 and z.shape == (T, heads * D) and z.stride(1) == 1 and z.stride(0) % 8 == 0 and z.data_ptr() % 16 == 0
+              and type(w) in (torch.Tensor, torch.nn.Parameter) and w.shape == (D,) and w.is_contiguous() and w.data_ptr() % 16 == 0)
+    if native:
+        return _GatedNormFn.apply(o, z, w, eps)
+    n = rmsnorm(o.reshape(-1, D), w, eps)
+    return (n.float() * torch.nn.functional.silu(z.reshape(-1, D).float())).to(o.dtype).reshape(T, heads * D)

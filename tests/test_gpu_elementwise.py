@@ -426,3 +426,25 @@ def test_bf16_gradient_passes_at_any_alignment(n, shift):
     ss = torch.zeros(1, device="cuda")
     optim.sumsq_(g, ss, False)
     assert abs(float(ss) - float(g.double().pow(2).sum())) < 1e-5 * float(ss)
+
+
+@pytest.mark.parametrize("T,heads,D,wide", [(1, 1, 128, 0), (37, 3, 64, 24), (130, 32, 128, 8), (9, 5, 256, 0)])
+def test_gated_head_norm(T, heads, D, wide):
+    """Gate read from a column range of wider rows, odd numbers of heads (groups past the end): against fp32 autograd of the
+    same formula; the result and the gradients carry two bf16 roundings, 2^-7 of the 2-norm bounds them."""
+    from lmms_engine_b200.ops import _cuda, norm
+
+    torch.manual_seed(0)
+    base = torch.randn(T, heads * D + wide, device="cuda").bfloat16()
+    o, w, dy = torch.randn(T, heads, D, device="cuda").bfloat16(), torch.randn(D, device="cuda").bfloat16(), torch.randn(T, heads * D, device="cuda").bfloat16()
+    dev = [t.clone().requires_grad_() for t in (o, base, w)]
+    n0 = _cuda.launch_count
+    y = norm.gated_head_norm(dev[0], dev[1][:, wide:], dev[2], 1e-6)
+    y.backward(dy)
+    assert _cuda.launch_count == n0 + 2
+    ref = [t.float().requires_grad_() for t in (o, base, w)]
+    want = norm.rmsnorm_ref(ref[0].reshape(-1, D), ref[2], 1e-6).view(T, -1) * torch.nn.functional.silu(ref[1][:, wide:])
+    want.backward(dy.float())
+    for a, b in [(y.detach(), want.detach())] + [(d.grad, r.grad) for d, r in zip(dev, ref)]:
+        assert torch.isfinite(a).all()
+        assert (a.float() - b).norm() < 2 ** -7 * b.norm()
