@@ -634,16 +634,17 @@ __global__ void rope_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__
 
 // ------------------------------------------------------------------ per-head RMSNorm + rotary embedding
 // The q and k heads of a projection row [T, n_q + n_kv (+ ...), D] (row stride ldx): y = rope(rmsnorm(x) * w), the rotation over
-// the whole head; D = 64 or 128.  D / 8 lanes share a head and hold four columns of each half, so both the norm's sum and the
-// rotation's partner stay inside a lane group.  As separate passes a head was copied out of its strided row, normalised and
-// rotated (six reads and writes of q and k); here it is read and written once.  Bound by memory.
+// the whole head; D = 64 or 128.  D / 8 lanes share a head, eight columns each; the rotation's partner comes from the lane half
+// a head away.  Sums run in the order of the separate norm kernels and every value is rounded where they store it, so that both
+// forms give the same bits (a model of 28 layers amplifies any other rounding).  As separate passes a head was copied out of its
+// strided row, normalised and rotated (six reads and writes of q and k); here it is read and written once.  Bound by memory.
 __device__ __forceinline__ float group_sum(float v, int lanes) {
   for (int o = lanes >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ void load_f4(const float* p, float (&v)[4]) {
-  const float4 u = *reinterpret_cast<const float4*>(p);
-  v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+__device__ __forceinline__ void load_f8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 template <int D>
 __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
@@ -652,7 +653,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __res
                                                                float* __restrict__ rstd, long T, int n_q, int n_kv, long ldx,
                                                                long ldy, float eps) {
   constexpr int L = D / 8, HPW = 32 / L;   // lanes per head, heads per warp
-  const int lane = threadIdx.x & 31, l = lane % L, heads = n_q + n_kv;
+  const int lane = threadIdx.x & 31, c = (lane % L) * 8, heads = n_q + n_kv;
+  const bool lower = c < D / 2;
   const long total = T * heads;
   const bool narrow = fits32(total);
   const long warps = static_cast<long>(gridDim.x) * (blockDim.x >> 5);
@@ -664,38 +666,23 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_kernel(const bf16* __res
     long t;
     int h;
     split_index(at, heads, narrow, t, h);
-    const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
-    float a[4], b[4];
-    load_w<4>(xp, a);
-    load_w<4>(xp + D / 2, b);
+    float v[8], wv[8], cs[8], sn[8], o[8];
+    load8(x + t * ldx + static_cast<long>(h) * D + c, v);
+    load8((h < n_q ? wq : wk) + c, wv);
+    load_f8(cosb + t * D + c, cs);
+    load_f8(sinb + t * D + c, sn);
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ss += a[j] * a[j] + b[j] * b[j];
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
     const float r = rsqrtf(group_sum(ss, L) / D + eps);
-    if (live && l == 0) rstd[at] = r;
-    float wa[4], wb[4];
-    const bf16* w = (h < n_q ? wq : wk) + 4 * l;
-    load_w<4>(w, wa);
-    load_w<4>(w + D / 2, wb);
-    float c[4], s[4], c2[4], s2[4];
-    load_f4(cosb + t * D + 4 * l, c);
-    load_f4(sinb + t * D + 4 * l, s);
-    load_f4(cosb + t * D + D / 2 + 4 * l, c2);
-    load_f4(sinb + t * D + D / 2 + 4 * l, s2);
-    float o1[4], o2[4];
+    if (live && lane % L == 0) rstd[at] = r;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // the normalised head is a bf16 tensor of its own in the separate form: rounded here too
-      const float x1 = __bfloat162float(__float2bfloat16(a[j] * r * wa[j]));
-      const float x2 = __bfloat162float(__float2bfloat16(b[j] * r * wb[j]));
-      o1[j] = x1 * c[j] - x2 * s[j];
-      o2[j] = x2 * c2[j] + x1 * s2[j];
+    for (int j = 0; j < 8; ++j) {
+      const float n = __bfloat162float(__float2bfloat16(v[j] * r * wv[j]));
+      const float m = __shfl_xor_sync(0xffffffffu, n, L / 2);
+      o[j] = lower ? n * cs[j] - m * sn[j] : n * cs[j] + m * sn[j];
     }
-    if (live) {
-      bf16* yp = y + t * ldy + static_cast<long>(h) * D + 4 * l;
-      store_w<4>(yp, o1);
-      store_w<4>(yp + D / 2, o2);
-    }
+    if (live) store8(y + t * ldy + static_cast<long>(h) * D + c, o);
   }
 }
 // d [T, heads, D] (row stride ldd): gradient of y on entry, of x on exit; part [gridDim.x][2][D] partial weight gradients.
@@ -707,7 +694,9 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
                                                                long ldd) {
   constexpr int L = D / 8, HPW = 32 / L;
   __shared__ float sw[2][D];
-  const int lane = threadIdx.x & 31, l = lane % L, heads = n_q + n_kv;
+  const int lane = threadIdx.x & 31, l = lane % L, c = l * 8, heads = n_q + n_kv;
+  const bool lower = c < D / 2;
+  const int other = lower ? c + D / 2 : c - D / 2;
   for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&sw[0][0])[i] = 0.f;
   __syncthreads();
   float dw[2][8] = {};
@@ -721,52 +710,34 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
     long t;
     int h;
     split_index(at, heads, narrow, t, h);
-    const bf16* xp = x + t * ldx + static_cast<long>(h) * D + 4 * l;
-    bf16* dp = d + t * ldd + static_cast<long>(h) * D + 4 * l;
-    float a[4], b[4], da[4], db[4], wa[4], wb[4];
-    load_w<4>(xp, a);
-    load_w<4>(xp + D / 2, b);
-    load_w<4>(dp, da);
-    load_w<4>(dp + D / 2, db);
+    bf16* dp = d + t * ldd + static_cast<long>(h) * D + c;
+    float v[8], g[8], wv[8], cs[8], sn[8];
+    load8(x + t * ldx + static_cast<long>(h) * D + c, v);
+    load8(dp, g);
     const bool is_q = h < n_q;
-    const bf16* w = (is_q ? wq : wk) + 4 * l;
-    load_w<4>(w, wa);
-    load_w<4>(w + D / 2, wb);
-    float c[4], s[4], c2[4], s2[4];
-    load_f4(cosb + t * D + 4 * l, c);
-    load_f4(sinb + t * D + 4 * l, s);
-    load_f4(cosb + t * D + D / 2 + 4 * l, c2);
-    load_f4(sinb + t * D + D / 2 + 4 * l, s2);
+    load8((is_q ? wq : wk) + c, wv);
+    load_f8(cosb + t * D + c, cs);
+    load_f8(sinb + t * D + other, sn);
     const float r = rstd[at];
     float dot = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 8; ++j) {
       // transposed rotation, rounded where the separate form stores it
-      const float g1 = __bfloat162float(__float2bfloat16(da[j] * c[j] + db[j] * s2[j]));
-      const float g2 = __bfloat162float(__float2bfloat16(db[j] * c2[j] - da[j] * s[j]));
-      a[j] *= r;
-      b[j] *= r;
+      const float m = __shfl_xor_sync(0xffffffffu, g[j], L / 2);
+      const float dy = __bfloat162float(__float2bfloat16(lower ? g[j] * cs[j] + m * sn[j] : g[j] * cs[j] - m * sn[j]));
+      v[j] *= r;
       // an index that depends on the head would put the sums into local memory
-      const float g1a = live ? g1 * a[j] : 0.f, g2b = live ? g2 * b[j] : 0.f;
-      dw[0][j] += is_q ? g1a : 0.f;
-      dw[0][4 + j] += is_q ? g2b : 0.f;
-      dw[1][j] += is_q ? 0.f : g1a;
-      dw[1][4 + j] += is_q ? 0.f : g2b;
-      da[j] = g1 * wa[j];
-      db[j] = g2 * wb[j];
-      dot += da[j] * a[j] + db[j] * b[j];
+      const float s = live ? dy * v[j] : 0.f;
+      dw[0][j] += is_q ? s : 0.f;
+      dw[1][j] += is_q ? 0.f : s;
+      g[j] = dy * wv[j];
+      dot += g[j] * v[j];
     }
-    const float m = group_sum(dot, L) / D;
+    dot = group_sum(dot, L) / D;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      da[j] = r * (da[j] - a[j] * m);
-      db[j] = r * (db[j] - b[j] * m);
-    }
+    for (int j = 0; j < 8; ++j) g[j] = r * (g[j] - v[j] * dot);
     __syncwarp();   // a group past the end read the last head: it must have before that head is rewritten
-    if (live) {
-      store_w<4>(dp, da);
-      store_w<4>(dp + D / 2, db);
-    }
+    if (live) store8(dp, g);
   }
   // the groups of a warp in a fixed order, then the warps one after the other: the same sum on every run
 #pragma unroll
@@ -779,10 +750,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(bf16* d, const bf
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          sw[k][4 * l + j] += dw[k][j];
-          sw[k][D / 2 + 4 * l + j] += dw[k][4 + j];
-        }
+        for (int j = 0; j < 8; ++j) sw[k][c + j] += dw[k][j];
     }
     __syncthreads();
   }

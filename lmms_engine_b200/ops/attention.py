@@ -191,7 +191,7 @@ def _fused_rows_ok(qkv, cos, sin, n_q, n_kv, D, wq, wk) -> bool:
     tables of exactly these rows; with norms, heads of 64 or 128 (a lane group owns a head)."""
     def plain(w):
         return (type(w) in (torch.Tensor, torch.nn.Parameter) and w.is_cuda and w.dtype == torch.bfloat16 and w.shape == (D,)
-                and w.is_contiguous() and w.data_ptr() % 8 == 0)
+                and w.is_contiguous() and w.data_ptr() % 16 == 0)
     return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.shape[0] > 0 and qkv.shape[1] == (n_q + 2 * n_kv) * D
             and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and D % 8 == 0 and D <= 128
             and n_q % n_kv == 0 and cos.dtype == sin.dtype == torch.float32 and cos.is_cuda and sin.is_cuda
