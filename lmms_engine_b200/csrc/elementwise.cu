@@ -403,7 +403,7 @@ norm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, co
       const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
       v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
     };
-    float dot = 0.f, gsum = 0.f;
+    float dots[8] = {}, gsums[8] = {};   // of 256 columns each
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * 32 + lane) * 8;
@@ -417,13 +417,20 @@ norm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, co
           const float xh = (v[j] - mean) * rstd, g = d[j] * (wv[j] + w_offset);
           dw[i][j] += d[j] * xh;
           if (LN) db[i][j] += d[j];
-          dot += g * xh;
-          gsum += g;
+          dots[i] += g * xh;
+          if (LN) gsums[i] += g;
         }
       }
     }
-    dot = warp_sum(dot) / H;
-    gsum = LN ? warp_sum(gsum) / H : 0.f;
+    // the order of a CTA per row with a warp per 256 columns, which rows above 2048 columns and the forward passes have: the
+    // gradient does not depend on which of the kernels ran
+    auto total = [](float (&s)[8]) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) s[i] = warp_sum(s[i]);
+      return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+    };
+    const float dot = total(dots) / H;
+    const float gsum = LN ? total(gsums) / H : 0.f;
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const int c = (i * 32 + lane) * 8;
