@@ -253,9 +253,10 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_kernel(const __grid_cons
 }
 
 // ------------------------------------------------------------------------------------------------ row norm
-__global__ void __launch_bounds__(256) row_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                       bf16* __restrict__ y, int K, long ldx, long ldy, float eps,
-                                                       float off) {
+// The kernel in front may still write `x` when this one starts, so `x` is not declared __restrict__: the compiler could then
+// read it through the non-coherent path or above the wait.  Only the weight is unchanged for the whole launch.
+__global__ void __launch_bounds__(256) row_norm_kernel(const bf16* x, const bf16* __restrict__ w, bf16* y, int K, long ldx,
+                                                       long ldy, float eps, float off) {
   __shared__ float red[8];
   pdl_go();
   pdl_wait();

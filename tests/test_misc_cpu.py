@@ -584,3 +584,22 @@ def test_public_class_names_of_the_reference_resolve():
         {"input_ids": torch.arange(1, 6), "labels": torch.arange(1, 6), "pixel_values": torch.ones(1, 5, 2, 2, 2), "use_audio_in_video": False}])
     assert batch["pixel_values"].shape == (2, 5, 2, 2, 2) and batch["pixel_values"][0, 3:].abs().sum() == 0
     assert batch["use_audio_in_video"] is False and batch["attention_mask"].sum(1).tolist() == [3, 5]
+
+
+def test_early_started_kernels_promise_nothing_about_what_their_predecessor_writes():
+    """A kernel that starts before the one in front of it has finished (``pdl_wait``) may declare only weights ``__restrict__``:
+    for ``const __restrict__`` data the compiler may use non-coherent loads and move them above the wait."""
+    import re
+
+    from lmms_engine_b200 import _native
+
+    found = 0
+    for src in _native.cuda_sources():
+        text = src.read_text()
+        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\(([^{]*?)\)\s*\{", text):
+            body = text[m.end():text.find("\n}\n", m.end())]
+            if "pdl_wait()" in body:
+                found += 1
+                promised = re.findall(r"__restrict__\s+(\w+)", m.group(2))
+                assert set(promised) <= {"w"}, f"{src.name}: {m.group(1)} promises that nobody writes {promised}"
+    assert found == 4
