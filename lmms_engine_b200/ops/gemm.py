@@ -76,6 +76,8 @@ def gemm(
         raise TypeError("bad output tensor")
     if cin is not None and not _ok(cin):
         raise TypeError("bad cin tensor")
+    if bias is not None and bias.numel() != N:
+        raise ValueError(f"{bias.numel()} bias entries for {N} outputs")
     if M <= SKINNY_ROWS and not (a_mn_major or b_mn_major or symmetric) and alpha == 1.0 and cin is None and (N | K) % 8 == 0:
         _cuda.call("b200_skinny_linear", a.data_ptr(), b.data_ptr(), _cuda.ptr(bias), out.data_ptr(), M, N, K, a.stride(0),
                    b.stride(0), out.stride(0), _cuda.stream())
@@ -113,6 +115,11 @@ def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, store_gu: b
         raise TypeError("gemm_swiglu needs contiguous CUDA bf16 operands")
     M, K = x.shape
     inter = wg.shape[0]
+    # the kernel takes one width and one row stride for both weights and bounds its reads by K and by the number of outputs
+    if wg.shape != (inter, K) or wu.shape != (inter, K) or wu.stride(0) != wg.stride(0):
+        raise ValueError(f"gate {tuple(wg.shape)} and up {tuple(wu.shape)} do not match rows of {K}")
+    if any(b is not None and b.numel() != inter for b in (bg, bu)):
+        raise ValueError(f"the biases need {inter} entries")
     ld = (inter + 7) // 8 * 8
     h = torch.empty((M, ld), dtype=torch.bfloat16, device=x.device)
     g = torch.empty_like(h) if store_gu else None

@@ -168,11 +168,11 @@ def gated_mlp(x, wg, bg, wu, bu, wd, bd) -> torch.Tensor:
     plain = (torch.Tensor, torch.nn.Parameter)
     native = (
         _gemm.LINEAR_BACKEND == "tcgen05" and x.is_cuda and x.dtype == torch.bfloat16 and x.numel() > 0 and wg.shape == wu.shape
-        and x.shape[-1] % 8 == 0 and wd.shape[0] % 8 == 0 and wd.shape[1] == wg.shape[0]
+        and x.shape[-1] % 8 == 0 and wg.shape[1] == x.shape[-1] and wd.shape[0] % 8 == 0 and wd.shape[1] == wg.shape[0]
         and all(type(w) in plain and w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0
                 for w in (wg, wu, wd))
-        and all(b is None or (type(b) in plain and b.is_cuda and b.dtype == torch.bfloat16 and b.is_contiguous())
-                for b in (bg, bu, bd))
+        and all(b is None or (type(b) in plain and b.is_cuda and b.dtype == torch.bfloat16 and b.is_contiguous() and b.shape == (w.shape[0],))
+                for b, w in ((bg, wg), (bu, wu), (bd, wd)))
     )
     if native:
         return _GatedMLPFn.apply(x, wg, bg, wu, bu, wd, bd)

@@ -178,6 +178,30 @@ def test_gated_mlp_any_width(P, K, inter, N, biases):
             assert torch.equal(t.grad, f + f)
 
 
+@pytest.mark.parametrize("inter", [36, 40])
+@pytest.mark.parametrize("wrong", ["gate", "up", "both", "bias", "down"])
+def test_gated_mlp_refuses_shapes_that_do_not_match(inter, wrong):
+    """Weights narrower or wider than the rows and short biases are refused on the host, as three linears refuse them: the
+    kernel takes one width for all and would read past the end."""
+    from lmms_engine_b200.ops import swiglu
+
+    K, N = 64, 64
+    for d in (-8, 8):
+        wg, bg, wu, bu, wd, bd = _rand(inter, K), _rand(inter), _rand(inter, K), _rand(inter), _rand(N, inter), _rand(N)
+        if wrong == "gate":
+            wg = _rand(inter, K + d)
+        elif wrong == "up":
+            wu = _rand(inter, K + d)
+        elif wrong == "both":
+            wg, wu = _rand(inter, K + d), _rand(inter, K + d)
+        elif wrong == "bias":
+            bu = _rand(inter + d)
+        else:
+            wd = _rand(N, inter + d)
+        with pytest.raises((ValueError, RuntimeError)):
+            swiglu.gated_mlp(_rand(130, K), wg, bg, wu, bu, wd, bd)
+
+
 @pytest.mark.parametrize("rows,N,ld", [(1, 8, 8), (31, 256, 256), (33, 260, 264), (1000, 1152, 1152), (4097, 3420, 3424), (7, 1, 8)])
 def test_column_sum(rows, N, ld):
     """Remainders of the row and column tiles; rows wider than N hold NaN that may not reach a sum.  fp32 sums, one rounding."""
