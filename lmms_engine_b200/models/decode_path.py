@@ -3,8 +3,9 @@
 ``decode_layers`` takes the place of the layer loop when a forward pass against a ``PackedKVCache`` feeds at most one token
 to each of at most 64 sequences, without gradients, on plain bf16 CUDA weights of the dense decoder layers
 (``decoder_lm.DecoderLayer``) or the hybrid ones (``qwen3_5.Qwen35Layer``).  Everything else - prompts, sparse MLPs, sharded
-weights, modules with forward hooks, other head dims - returns ``None`` and runs layer by layer.  The numbers are those of
-the layer loop up to the order of fp32 sums: every intermediate is rounded to bf16 at the same place.
+weights, subclassed, patched, parametrised or hooked modules, norms of different eps, other head dims - returns ``None`` and
+runs layer by layer.  The numbers are those of the layer loop up to the order of fp32 sums: every intermediate is rounded to
+bf16 at the same place.
 """
 from __future__ import annotations
 
@@ -15,6 +16,7 @@ import torch
 
 from ..ops import _cuda
 from ..ops import gemm as gemm_ops
+from .plain_call import global_hooks, own_call
 
 _cuda.register("b200_decode_layers", "decode", "ppi" + "pppp" + "fff" + "ppppp" + "p" + "l" + "pp" + "s")
 
@@ -26,9 +28,9 @@ class _Unfit(Exception):
     pass
 
 
-def _plain(module) -> dict:
-    """Parameters of a module whose call is only its arithmetic."""
-    if module._forward_hooks or module._forward_pre_hooks:
+def _plain(module, cls) -> dict:
+    """Parameters of a module whose call is only the arithmetic of its class."""
+    if not own_call(module, cls):
         raise _Unfit
     return module._parameters
 
@@ -46,54 +48,64 @@ def _opt(w, shape) -> int:
     return 0 if w is None else _at(w, shape)
 
 
-def _norm(module, cfg, H) -> int:
-    if module.eps != cfg.rms_norm_eps:
+def _norm(module, cls, cfg, width) -> int:
+    own = _plain(module, cls)
+    if module.eps != cfg.rms_norm_eps:  # one eps for all norms of the call
         raise _Unfit
-    return _at(_plain(module)["weight"], (H,))
+    return _at(own.get("weight"), (width,))
 
 
-def _mlp(rec, mlp, H, I):
+def _weight(module, shape, cls=torch.nn.Linear) -> int:
+    """Weight of a projection.  Its layer reads the weight and never calls the module, so hooks on it do not matter, but a
+    subclass may compute its weight on access."""
+    if type(module) is not cls:
+        raise _Unfit
+    return _at(module._parameters.get("weight"), shape)
+
+
+def _mlp(rec, mlp, cls, H, I):
+    _plain(mlp, cls)
     if mlp.tp_group is not None:
         raise _Unfit
-    _plain(mlp)
     m = mlp._modules
-    rec[13] = _at(_plain(m["gate_proj"])["weight"], (I, H))
-    rec[14] = _at(_plain(m["up_proj"])["weight"], (I, H))
-    rec[15] = _at(_plain(m["down_proj"])["weight"], (H, I))
+    rec[13] = _weight(m["gate_proj"], (I, H))
+    rec[14] = _weight(m["up_proj"], (I, H))
+    rec[15] = _weight(m["down_proj"], (H, I))
 
 
-def _attention(rec, att, cache, dev, H, nq, nkv, D, gated):
+def _attention(rec, att, cls, norm_cls, cfg, cache, dev, H, nq, nkv, D, gated):
+    _plain(att, cls)
     m = att._modules
-    _plain(att)
     if getattr(att, "nsa", None) is not None or getattr(att, "window", (-1, -1))[0] != cache.decode_window:
         raise _Unfit
     rows = nq * D * (2 if gated else 1)
     for i, (name, n) in enumerate((("q_proj", rows), ("k_proj", nkv * D), ("v_proj", nkv * D))):
-        p = _plain(m[name])
-        rec[1 + i] = _at(p["weight"], (n, H))
-        rec[5 + i] = _opt(p["bias"], (n,))
-    if "q_norm" in m:
-        rec[9] = _at(_plain(m["q_norm"])["weight"], (D,))
-        rec[10] = _at(_plain(m["k_norm"])["weight"], (D,))
-    p = _plain(m["o_proj"])
-    rec[11] = _at(p["weight"], (H, nq * D))
-    rec[19] = _opt(p["bias"], (H,))
+        rec[1 + i] = _weight(m[name], (n, H))
+        rec[5 + i] = _opt(m[name]._parameters.get("bias"), (n,))
+    if gated or att.cfg.qk_norm:
+        rec[9] = _norm(m["q_norm"], norm_cls, cfg, D)
+        rec[10] = _norm(m["k_norm"], norm_cls, cfg, D)
+    rec[11] = _weight(m["o_proj"], (H, nq * D))
+    rec[19] = _opt(m["o_proj"]._parameters.get("bias"), (H,)) if gated else 0  # the ungated layer adds none
     k, v = cache.slabs(att.layer_idx, nkv, D, _BF16, dev)
     if k.dtype is not _BF16 or k.device != dev or k.shape[1:] != (nkv, D):
         raise _Unfit
     rec[16], rec[17] = k.data_ptr(), v.data_ptr()
 
 
-def _delta(rec, net, H):
+def _delta(rec, net, cls, cfg, H):
+    own = _plain(net, cls)
     m = net._modules
-    own = _plain(net)
+    # the gated output norm is a weight without a call of its own; its eps stands at the layer
+    if net.eps != cfg.rms_norm_eps or type(m["norm"]) is not torch.nn.Module:
+        raise _Unfit
     key, val, hv = net.key_dim, net.value_dim, net.hv
     for i, (name, n) in enumerate((("in_proj_qkv", 2 * key + val), ("in_proj_z", val), ("in_proj_b", hv), ("in_proj_a", hv))):
-        rec[1 + i] = _at(_plain(m[name])["weight"], (n, H))
-    rec[9] = _at(_plain(m["conv1d"])["weight"], (2 * key + val, 1, net.kernel))
-    rec[10], rec[16] = _at(own["A_log"], (hv,)), _at(own["dt_bias"], (hv,))
-    rec[17] = _at(m["norm"]._parameters["weight"], (net.dv,))
-    rec[11] = _at(_plain(m["out_proj"])["weight"], (H, val))
+        rec[1 + i] = _weight(m[name], (n, H))
+    rec[9] = _weight(m["conv1d"], (2 * key + val, 1, net.kernel), torch.nn.Conv1d)
+    rec[10], rec[16] = _at(own.get("A_log"), (hv,)), _at(own.get("dt_bias"), (hv,))
+    rec[17] = _at(m["norm"]._parameters.get("weight"), (net.dv,))
+    rec[11] = _weight(m["out_proj"], (H, val))
 
 
 def _delta_state(store, net, seqs, device):
@@ -106,6 +118,9 @@ def _delta_state(store, net, seqs, device):
             tail = torch.zeros((net.kernel - 1, 2 * net.key_dim + net.value_dim), dtype=_BF16, device=device)
         if S is None:
             S = torch.zeros((net.hv, net.dk, net.dv), dtype=torch.float32, device=device)
+        if tail.shape != (net.kernel - 1, 2 * net.key_dim + net.value_dim) or S.shape != (net.hv, net.dk, net.dv) \
+                or tail.device != device or S.device != device:
+            raise _Unfit
         if not (tail.is_contiguous() and S.is_contiguous() and tail.dtype is _BF16 and S.dtype is torch.float32 and S.data_ptr() % 16 == 0):
             tail, S = tail.to(_BF16).contiguous(), S.float().clone()
         out = torch.empty_like(tail)
@@ -118,7 +133,7 @@ def decode_layers(backbone, embeds: torch.Tensor, ctx) -> Optional[torch.Tensor]
     cache = ctx.kv_cache
     M = embeds.shape[0]
     if (M > MAX_SEQS or not embeds.is_cuda or embeds.dtype is not _BF16 or torch.is_grad_enabled() or not ctx.causal
-            or ctx.sp_size > 1 or ctx.tp_size > 1 or ctx.deepstack is not None or gemm_ops.LINEAR_BACKEND != "tcgen05"):
+            or ctx.sp_size > 1 or ctx.tp_size > 1 or ctx.deepstack is not None or gemm_ops.LINEAR_BACKEND != "tcgen05" or global_hooks()):
         return None
     seqs = [i for i, n in enumerate(cache.new_lens) if n]
     if len(seqs) != M or any(cache.new_lens[i] != 1 for i in seqs):
@@ -139,58 +154,43 @@ def _run(backbone, embeds, ctx, cache, seqs):
     rot = ctx.cos.shape[-1]
     if rot % 2 or rot > D or ctx.cos.dtype is not torch.float32 or ctx.cos.shape[0] != M:
         raise _Unfit
-    norm_off = 0.0
     cache.decode_window = -1
     layers = backbone.layers._modules
-    first = next(iter(layers.values()))
+    first = next(iter(layers.values()), None)
     if type(first) is DecoderLayer:
-        cache.decode_window = first.self_attn.window[0]
-        hybrid = None
+        cache.decode_window = getattr(first.self_attn, "window", (-1, -1))[0]
+        hybrid, layer_cls, att_cls, norm_cls, norm_off = None, DecoderLayer, Attention, RMSNorm, 0.0
     else:
         from . import qwen3_5 as hybrid
 
         if type(first) is not hybrid.Qwen35Layer:
             raise _Unfit
-        norm_off = 1.0
+        layer_cls, att_cls, norm_cls, norm_off = hybrid.Qwen35Layer, hybrid.GatedAttention, hybrid.ZRMSNorm, 1.0
     table, types, nets = array("Q"), array("i"), []
     rec0 = [0] * 24
     hk = hv = taps = 0
     for layer in layers.values():
         rec = rec0[:]
-        _plain(layer)
+        _plain(layer, layer_cls)
         m = layer._modules
-        mlp = m["mlp"]
-        if type(mlp) is not SwiGLUMLP:
-            raise _Unfit
-        if hybrid is None:
-            att = m["self_attn"]
-            if type(layer) is not DecoderLayer or type(att) is not Attention or type(m["input_layernorm"]) is not RMSNorm:
+        if hybrid is not None and "linear_attn" in m:
+            net = m["linear_attn"]
+            _delta(rec, net, hybrid.GatedDeltaNet, cfg, H)
+            if net.dk != 128 or net.dv != 128 or net.hv % 8 or net.hv % net.hk or not 2 <= net.kernel <= 8:
                 raise _Unfit
-            _attention(rec, att, cache, dev, H, nq, nkv, D, False)
-            types.append(0)
+            hk, hv, taps = net.hk, net.hv, net.kernel
+            nets.append(net)
+            types.append(2)
         else:
-            if type(layer) is not hybrid.Qwen35Layer:
-                raise _Unfit
-            if "linear_attn" in m:
-                net = m["linear_attn"]
-                if type(net) is not hybrid.GatedDeltaNet or net.dk != 128 or net.dv != 128 or net.hv % 8 or net.hv % net.hk or not 2 <= net.kernel <= 8:
-                    raise _Unfit
-                _delta(rec, net, H)
-                hk, hv, taps = net.hk, net.hv, net.kernel
-                nets.append(net)
-                types.append(2)
-            else:
-                if type(m["self_attn"]) is not hybrid.GatedAttention:
-                    raise _Unfit
-                _attention(rec, m["self_attn"], cache, dev, H, nq, nkv, D, True)
-                types.append(1)
+            _attention(rec, m["self_attn"], att_cls, norm_cls, cfg, cache, dev, H, nq, nkv, D, hybrid is not None)
+            types.append(0 if hybrid is None else 1)
         for at, name in ((0, "input_layernorm"), (12, "post_attention_layernorm")):
-            rec[at] = _norm(m[name], cfg, H)
-        _mlp(rec, mlp, H, I)
+            rec[at] = _norm(m[name], norm_cls, cfg, H)
+        _mlp(rec, m["mlp"], SwiGLUMLP, H, I)
         table.extend(rec)
-    final = _norm(backbone._modules["norm"], cfg, H)
+    final = _norm(backbone._modules["norm"], norm_cls, cfg, H)
 
-    # nothing below declines: the states are replaced only here
+    # the states are replaced after the call: what declines here leaves them as they were
     gdn, news = array("Q"), []
     for net in nets:
         store = cache.state.setdefault(net.layer_idx, {})

@@ -90,3 +90,76 @@ def test_native_path_is_taken_and_hooks_keep_the_layer_loop():
         assert "b200_decode_layers" not in seen
     finally:
         _cuda.call = real
+
+
+class _ScaledLinear(torch.nn.Linear):
+    """Computes its weight on access, as a quantised or adapted projection does."""
+
+    @property
+    def weight(self):
+        return self._parameters["weight"] * 1.5
+
+
+class _Twice(torch.nn.Module):
+    def forward(self, w):
+        return 2 * w
+
+
+def _negated(cls):
+    return type("Negated" + cls.__name__, (cls,), {"forward": lambda self, *a: cls.forward(self, *(-x for x in a))})
+
+
+def _change(model, what, monkeypatch):
+    from torch.nn.utils import parametrize
+
+    from lmms_engine_b200.models import decoder_lm
+
+    layer = model.model.layers[1]
+    if what == "parametrized":
+        parametrize.register_parametrization(layer.self_attn.o_proj, "weight", _Twice())
+    elif what == "computed weight":
+        layer.mlp.up_proj.__class__ = _ScaledLinear
+    elif what in ("q_norm eps", "k_norm eps"):
+        getattr(layer.self_attn, what[:6]).eps = 0.5
+    elif what == "post norm eps":
+        layer.post_attention_layernorm.eps = 0.5
+    elif what == "q_norm subclass":
+        layer.self_attn.q_norm.__class__ = _negated(type(layer.self_attn.q_norm))
+    elif what == "post norm subclass":
+        layer.post_attention_layernorm.__class__ = _negated(type(layer.post_attention_layernorm))
+    elif what == "final norm subclass":
+        model.model.norm.__class__ = _negated(type(model.model.norm))
+    elif what == "instance forward":
+        layer.mlp.forward = lambda x: 0.5 * x
+    elif what == "class forward":
+        monkeypatch.setattr(decoder_lm.SwiGLUMLP, "forward", lambda self, x: 0.5 * x)
+    elif what == "global hook":
+        return torch.nn.modules.module.register_module_forward_hook(lambda m, a, out: 0.5 * out if m is layer.mlp else None).remove
+    elif what == "delta eps":
+        model.model.layers[0].linear_attn.eps = 0.5
+    elif what == "delta projection":
+        model.model.layers[0].linear_attn.in_proj_z.__class__ = _ScaledLinear
+    return lambda: None
+
+
+@pytest.mark.parametrize("kind,what", [("normed", w) for w in (
+    "parametrized", "computed weight", "q_norm eps", "k_norm eps", "post norm eps", "q_norm subclass", "post norm subclass",
+    "final norm subclass", "instance forward", "class forward", "global hook")] + [("hybrid", "delta eps"), ("hybrid", "delta projection")])
+def test_modules_that_are_more_than_their_weights_keep_the_layer_loop(kind, what, monkeypatch):
+    """Whatever a call of the module would do beyond its class's arithmetic on plain parameters has to happen: the pass runs
+    layer by layer, which is what it is compared with (bit by bit: it is the same code)."""
+    from lmms_engine_b200.ops import _cuda
+
+    model = _model(kind)
+    before = _go(model, [10], 2, False)
+    undo = _change(model, what, monkeypatch)
+    try:
+        want = _go(model, [10], 2, False)
+        seen, real = [], _cuda.call
+        monkeypatch.setattr(_cuda, "call", lambda name, *a: (seen.append(name), real(name, *a))[1])
+        got = _go(model, [10], 2, True)
+    finally:
+        undo()
+    assert not torch.equal(want, before), "the change has no effect on the output"
+    assert torch.equal(got, want)
+    assert "b200_decode_layers" not in seen
