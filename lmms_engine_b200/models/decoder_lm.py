@@ -33,6 +33,7 @@ from ..ops import swiglu as swiglu_ops
 from ..parallel import fused_ops, tp_ops
 from ..parallel.sequence_parallel import ulysses as sp
 from . import decode_path
+from .plain_call import global_hooks, own_call
 
 IGNORE_INDEX = -100
 
@@ -143,8 +144,7 @@ class Attention(nn.Module):
         if not self.cfg.qk_norm:
             return None
         q, k = self.q_norm, self.k_norm
-        if type(q) is not RMSNorm or type(k) is not RMSNorm or q.eps != k.eps or q._forward_hooks or k._forward_hooks \
-                or q._forward_pre_hooks or k._forward_pre_hooks:
+        if not (own_call(q, RMSNorm) and own_call(k, RMSNorm)) or q.eps != k.eps or global_hooks():
             return False
         return q.weight, k.weight, q.eps
 

@@ -603,3 +603,42 @@ def test_early_started_kernels_promise_nothing_about_what_their_predecessor_writ
                 promised = re.findall(r"__restrict__\s+(\w+)", m.group(2))
                 assert set(promised) <= {"w"}, f"{src.name}: {m.group(1)} promises that nobody writes {promised}"
     assert found == 4
+
+
+@pytest.mark.parametrize("what", ["plain", "backward hook", "backward pre hook", "forward hook", "global forward", "global backward", "instance",
+                                  "class", "subclass", "eps"])
+def test_head_norms_are_read_only_where_a_call_does_nothing_else(what, monkeypatch):
+    """The fused per-head norm reads weights instead of calling ``q_norm`` and ``k_norm``; hooks of every kind and replaced
+    forwards need the calls."""
+    from torch.nn.modules import module as nn_module
+
+    from lmms_engine_b200.models import decoder_lm
+
+    att = decoder_lm.Attention(decoder_lm.DecoderConfig(hidden_size=32, num_attention_heads=4, num_key_value_heads=2, head_dim=8, qk_norm=True), 0)
+    k, undo = att.k_norm, lambda: None
+    if what == "backward hook":
+        k.register_full_backward_hook(lambda m, gi, go: None)
+    elif what == "backward pre hook":
+        k.register_full_backward_pre_hook(lambda m, go: None)
+    elif what == "forward hook":
+        k.register_forward_hook(lambda m, a, o: None)
+    elif what == "global forward":
+        undo = nn_module.register_module_forward_pre_hook(lambda m, a: None).remove
+    elif what == "global backward":
+        undo = nn_module.register_module_full_backward_hook(lambda m, gi, go: None).remove
+    elif what == "instance":
+        k.forward = lambda x, residual=None: x
+    elif what == "class":
+        monkeypatch.setattr(decoder_lm.RMSNorm, "forward", lambda self, x, residual=None: x)
+    elif what == "subclass":
+        k.__class__ = type("Other", (decoder_lm.RMSNorm,), {})
+    elif what == "eps":
+        k.eps = 1e-3
+    try:
+        got = att._head_norms()
+    finally:
+        undo()
+    if what == "plain":
+        assert got[0] is att.q_norm.weight and got[1] is k.weight
+    else:
+        assert got is False
