@@ -110,7 +110,10 @@ class PackedKVCache:
             self.k[layer][lo:hi].copy_(k)
             self.v[layer][lo:hi].copy_(v)
             if self.had[i]:
-                return self.k[layer][self.base[i]:hi], self.v[layer][self.base[i]:hi], cu_k, max_k
+                k_all, v_all = self.k[layer][self.base[i]:hi], self.v[layer][self.base[i]:hi]
+                if torch.is_grad_enabled():  # the backward pass reads them after a later pass has written into the slab
+                    k_all, v_all = k_all.clone(), v_all.clone()
+                return k_all, v_all, cu_k, max_k
         else:
             self.k[layer].index_copy_(0, write, k)
             self.v[layer].index_copy_(0, write, v)

@@ -165,3 +165,36 @@ def test_flow_grpo_trainer_samples_scores_and_replays_image_generation(tmp_path)
                                    "reward": "latent_brightness", "boi_token_id": 126, "eoi_token_id": 127, "beta": 0.01, "clip_range": [1e-3, 1e-3]})
     assert "rl/reward_mean" in hist[0] and hist[0]["rl/recorded_steps"] > 0 and "rl/policy_loss" in hist[0]
     assert runner.trainer.ref_model is not None
+
+
+def _small_cached_model():
+    from lmms_engine_b200.mapping_func import create_model_from_config
+
+    torch.manual_seed(0)
+    cfg = dict(vocab_size=64, hidden_size=32, intermediate_size=64, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=4, head_dim=8)
+    return create_model_from_config("qwen3", dict(cfg, model_type="qwen3"))
+
+
+def test_cached_passes_can_be_differentiated_after_later_passes():
+    """With gradients a pass keeps the rows that it attended to: a later pass writes into the same slab, so what the backward
+    pass reads must not be the slab itself."""
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    model = _small_cached_model()
+    ids = torch.randint(0, 64, (9,))
+
+    def go(late):
+        model.zero_grad(set_to_none=True)
+        cache, losses = PackedKVCache(2, [16]), []
+        for a, b in ((0, 4), (4, 7), (7, 9)):
+            pos = cache.advance([b - a])
+            h = model(input_ids=ids[a:b], cu_seqlens=torch.tensor([0, b - a], dtype=torch.int32), position_ids=pos, kv_cache=cache)["hidden_states"]
+            losses.append(h.square().sum())
+            if not late:
+                losses[-1].backward()
+        if late:
+            sum(losses).backward()
+        return [p.grad.clone() for p in model.parameters() if p.grad is not None]
+
+    for x, y in zip(go(True), go(False)):
+        assert torch.allclose(x, y, rtol=1e-4, atol=1e-6)
