@@ -104,6 +104,10 @@ class PackedKVCache:
         if self.k[layer] is None:
             self.k[layer] = k.new_empty((self.base[-1],) + tuple(k.shape[1:]))
             self.v[layer] = v.new_empty((self.base[-1],) + tuple(v.shape[1:]))
+        for new, slab in ((k, self.k[layer]), (v, self.v[layer])):  # copying into a slice would cast and broadcast
+            if new.dtype != slab.dtype or new.shape[1:] != slab.shape[1:] or new.device != slab.device:
+                raise RuntimeError(f"rows of {tuple(new.shape[1:])} {new.dtype} on {new.device} for a cache of {tuple(slab.shape[1:])} "
+                                   f"{slab.dtype} on {slab.device}")
         if sum(1 for n in self.new_lens if n) == 1:
             i = next(i for i, n in enumerate(self.new_lens) if n)
             lo, hi = self.base[i] + self.had[i], self.base[i] + self.lens[i]

@@ -198,3 +198,24 @@ def test_cached_passes_can_be_differentiated_after_later_passes():
 
     for x, y in zip(go(True), go(False)):
         assert torch.allclose(x, y, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("seqs", [1, 2])
+def test_cache_refuses_rows_of_another_kind(seqs):
+    """Rows of another type, width or head count are an error for one sequence as for several, and leave the cache as it was."""
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    cache = PackedKVCache(1, [8] * seqs)
+    cache.advance([2] * seqs)
+    rows = torch.randn(2 * seqs, 2, 4)
+    cache.extend(0, rows, rows)
+    cache.advance([1] * seqs)
+    good = torch.randn(seqs, 2, 4)
+    for bad in (good.double(), good[:, :1], good[..., :1]):
+        before = cache.k[0][: 2].clone()
+        for k, v in ((bad, good), (good, bad)):
+            with pytest.raises(RuntimeError):
+                cache.extend(0, k, v)
+        assert torch.equal(cache.k[0][: 2], before)
+    keys = cache.extend(0, good, good)[0]
+    assert torch.equal(keys.reshape(seqs, 3, 2, 4)[:, 2], good)
