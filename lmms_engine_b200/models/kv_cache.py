@@ -56,10 +56,11 @@ class PackedKVCache:
         live = [(s, n) for s, n in zip(starts, self.new_lens) if n]
         if len(live) == 1:
             return torch.arange(live[0][0], live[0][0] + live[0][1], device=self.device)
+        # on the host whatever the default device is: pinned memory is host memory
         if max(self.new_lens) == 1:
-            host = torch.tensor([s for s, _ in live])
+            host = torch.tensor([s for s, _ in live], device="cpu")
         else:
-            host = torch.cat([torch.arange(s, s + n) for s, n in live])
+            host = torch.cat([torch.arange(s, s + n, device="cpu") for s, n in live])
         if self.device is None or torch.device(self.device).type != "cuda":
             return host.to(self.device)
         # from pinned memory: a pageable copy waits for everything queued on the device, once per generated token

@@ -163,3 +163,14 @@ def test_modules_that_are_more_than_their_weights_keep_the_layer_loop(kind, what
     assert not torch.equal(want, before), "the change has no effect on the output"
     assert torch.equal(got, want)
     assert "b200_decode_layers" not in seen
+
+
+def test_cache_advances_under_a_default_device():
+    """``torch.set_default_device("cuda")`` and ``with torch.device("cuda")`` make factory calls return device tensors."""
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    with torch.device("cuda"):
+        cache = PackedKVCache(1, [8, 8, 8], device=torch.device("cuda", 0))
+        assert cache.advance([3, 0, 2]).tolist() == [0, 1, 2, 0, 1]
+        assert cache.advance([1, 1, 1]).tolist() == [3, 0, 2]
+        assert cache.advance([0, 2, 0]).tolist() == [1, 2]
