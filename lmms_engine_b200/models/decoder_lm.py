@@ -356,16 +356,26 @@ class DecoderBackbone(nn.Module):
         self.register_buffer("inv_freq", rope_ops.inv_freq(cfg.head_dim, cfg.rope_theta), persistent=False)
 
     def _frequencies(self, dim: int, device) -> torch.Tensor:
-        """Rotary frequencies in fp32.  Casting a model to bf16 casts the buffer too; the fp32 values are then computed
-        once per device and kept (they are constants of the configuration)."""
+        """Rotary frequencies in fp32.  Casting a model to bf16 casts the buffer too; the fp32 values (constants of the
+        configuration) are then computed, and kept for the stream that they were computed on: another stream would have to
+        wait for them.  What a capture or a trace computes belongs to it and is not kept."""
         invf = self.inv_freq
         if invf.dtype == torch.float32 and invf.device == device:
             return invf
-        kept = self.__dict__.setdefault("_fp32_frequencies", {})
-        key = (dim, float(self.cfg.rope_theta), device)
-        if key not in kept:
-            kept[key] = rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
-        return kept[key]
+        kept, key = None, None
+        if torch.device(device).type == "cuda" and not torch.cuda.is_current_stream_capturing():
+            kept = self.__dict__.setdefault("_fp32_frequencies", {})
+            key = (dim, float(self.cfg.rope_theta), device, torch.cuda.current_stream(device).cuda_stream)
+            if key in kept:
+                return kept[key]
+        fresh = rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
+        if kept is not None and type(fresh) is torch.Tensor:
+            kept[key] = fresh
+        return fresh
+
+    def __getstate__(self):
+        # a copy of the model computes its own: copies are made on other streams
+        return {k: v for k, v in self.__dict__.items() if k != "_fp32_frequencies"}
 
     def rope_tables(self, position_ids: torch.Tensor):
         cfg = self.cfg

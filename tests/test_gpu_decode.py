@@ -174,3 +174,29 @@ def test_cache_advances_under_a_default_device():
         assert cache.advance([3, 0, 2]).tolist() == [0, 1, 2, 0, 1]
         assert cache.advance([1, 1, 1]).tolist() == [3, 0, 2]
         assert cache.advance([0, 2, 0]).tolist() == [1, 2]
+
+
+def test_rotary_frequencies_are_kept_per_stream_and_not_from_a_capture():
+    """The first pass may be a capture, a trace or on another stream: none of them leaves values behind that a later pass
+    reads before they exist."""
+    import copy
+
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from lmms_engine_b200.ops import rope
+
+    backbone = _model("grouped").model
+    pos = torch.arange(5, device="cuda")
+    want = rope.rope_table(pos, rope.inv_freq(128, backbone.cfg.rope_theta, device=pos.device))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        backbone.rope_tables(pos)
+    with FakeTensorMode():
+        backbone._frequencies(128, pos.device)
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(backbone.rope_tables(pos), want))
+    here = backbone._frequencies(128, pos.device)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        there = backbone._frequencies(128, pos.device)
+    assert there is not here and backbone._frequencies(128, pos.device) is here
+    assert not hasattr(copy.deepcopy(backbone), "_fp32_frequencies")
