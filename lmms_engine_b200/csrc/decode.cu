@@ -16,6 +16,8 @@
 //
 // Reference counterpart: the same modules run one by one through transformers' generate
 // (src/lmms_engine/models/aero_realtime/modeling_aero_realtime.py:700-1385 for the streaming loop).
+#include <atomic>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -711,18 +713,36 @@ static int launch_k(void (*k)(const P), dim3 grid, int threads, size_t smem, cud
   return cudaLaunchKernelEx(&cfg, k, p) == cudaSuccess ? 0 : -4;
 }
 
+// Dynamic shared memory beyond the default limit has to be asked for once per kernel and device.  The amount is always the
+// kernel's largest, so that threads with different sizes do not lower it for one another; two that come first at the same time
+// ask for the same.
+struct SmemOptIn {
+  std::atomic<unsigned long long> done{0};   // a bit per device
+  template <typename K>
+  int ask(K kernel, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return -3;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) != cudaSuccess) return -3;
+    done.fetch_or(bit, std::memory_order_release);
+    return 0;
+  }
+};
+
+constexpr size_t kNormRowsBytes = 96 * 1024;   // most that the rows of the fused norm may take
+static bool norm_fits(int M, int K) { return M <= kSkNormRows && static_cast<size_t>(M) * (K + 8) * 2 <= kNormRowsBytes; }
+
 template <int RT, int MT, int MODE, bool NORM>
 static int launch_skinny(const SkinnyParams& p, cudaStream_t st, bool early) {
-  size_t smem = static_cast<size_t>(kSkWarps) * MT * 16 * RT * 8 * 4;
+  constexpr size_t kParts = static_cast<size_t>(kSkWarps) * MT * 16 * RT * 8 * 4;
+  size_t smem = kParts;
   if (NORM) {
     const size_t xs = static_cast<size_t>(p.M) * (p.K + 8) * 2;
     if (xs > smem) smem = xs;
   }
-  static size_t set = 48 * 1024;
-  if (smem > set) {
-    if (cudaFuncSetAttribute(skinny_kernel<RT, MT, MODE, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) return -3;
-    set = smem;
-  }
+  static SmemOptIn opt;
+  if (opt.ask(skinny_kernel<RT, MT, MODE, NORM>, NORM && kNormRowsBytes > kParts ? kNormRowsBytes : kParts) != 0) return -3;
   const int per = MODE == SK_SWIGLU ? RT * 4 : RT * 8;
   return launch_k(skinny_kernel<RT, MT, MODE, NORM>, dim3((p.N + per - 1) / per), kSkWarps * 32, smem, st, p, early);
 }
@@ -746,8 +766,6 @@ static int skinny(const SkinnyParams& p, cudaStream_t st, bool early = true) {
   return wide<4, MODE>(p, st, early);
 }
 
-static bool norm_fits(int M, int K) { return M <= kSkNormRows && static_cast<size_t>(M) * (K + 8) * 2 <= 96 * 1024; }
-
 static int row_norm(const bf16* x, const bf16* w, bf16* y, int M, int K, float eps, float off, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(M);
@@ -765,11 +783,8 @@ template <int D, int QROWS>
 static int launch_dec_attn(const DecAttnParams& p, int n_seq, cudaStream_t st) {
   constexpr size_t smem = (16 * D + D + 4 * 2 * 16 * D) * 2 + 4 * QROWS * 2 * 4 + 16;
   static_assert(4 * QROWS * D * 4 <= 4 * 2 * 16 * D * 2, "outputs of the warps reuse the value tiles");
-  static bool set = false;
-  if (!set) {
-    if (cudaFuncSetAttribute(dec_attn_kernel<D, QROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) return -3;
-    set = true;
-  }
+  static SmemOptIn opt;
+  if (opt.ask(dec_attn_kernel<D, QROWS>, smem) != 0) return -3;
   return launch_k(dec_attn_kernel<D, QROWS>, dim3(p.splits, p.n_kv, n_seq), 128, smem, st, p, true);
 }
 

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 DENSE = dict(vocab_size=512, hidden_size=256, intermediate_size=520, num_hidden_layers=2, rms_norm_eps=1e-6)
 
 
-def _model(kind):
+def _model(kind, **sizes):
     from lmms_engine_b200.mapping_func import create_model_from_config
 
     torch.manual_seed(3)
@@ -20,7 +20,7 @@ def _model(kind):
         heads, kv, dim, extra = {"grouped": (14, 2, 128, {}), "normed": (4, 2, 128, dict(attention_bias=False, qk_norm=True)),
                                  "narrow": (4, 4, 64, {}), "wide_group": (12, 1, 128, {}),
                                  "window": (4, 2, 128, dict(sliding_window=70, use_sliding_window=True))}[kind]
-        m = create_model_from_config("qwen2", dict(DENSE, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, **extra))
+        m = create_model_from_config("qwen2", dict(DENSE, num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, **{**extra, **sizes}))
     m = m.to("cuda", torch.bfloat16).eval()
     with torch.no_grad():
         for n, p in m.named_parameters():
@@ -31,33 +31,39 @@ def _model(kind):
     return m
 
 
-def _go(model, prompts, steps, native):
-    from lmms_engine_b200.models import decode_path
+def _run_tokens(model, prompts, steps):
     from lmms_engine_b200.models.kv_cache import PackedKVCache
-    from lmms_engine_b200.ops import _cuda
 
     gen = torch.Generator(device="cuda").manual_seed(5)
-    n = len(prompts)
+    n, out = len(prompts), []
     cache = PackedKVCache(len(model.model.layers), [p + steps for p in prompts], device=torch.device("cuda", 0))
     ids = torch.randint(0, 512, (sum(prompts),), device="cuda", generator=gen)
-    keep, out = decode_path.MAX_SEQS, []
+    with torch.no_grad():
+        pos = cache.advance(prompts)
+        cu = torch.tensor([0] + torch.tensor(prompts).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        model(input_ids=ids, cu_seqlens=cu, position_ids=pos, kv_cache=cache)
+        for s in range(steps):
+            live = [1 if (i + s) % 3 or n == 1 else 0 for i in range(n)]  # sequences pause and resume
+            pos = cache.advance(live)
+            m = sum(live)
+            tok = torch.randint(0, 512, (m,), device="cuda", generator=gen)
+            cu = torch.arange(m + 1, dtype=torch.int32, device="cuda")
+            out.append(model(input_ids=tok, cu_seqlens=cu, position_ids=pos, kv_cache=cache)["hidden_states"])
+    return torch.cat(out).float()
+
+
+def _go(model, prompts, steps, native):
+    from lmms_engine_b200.models import decode_path
+    from lmms_engine_b200.ops import _cuda
+
+    keep = decode_path.MAX_SEQS
     decode_path.MAX_SEQS = keep if native else 0
     try:
-        with torch.no_grad():
-            pos = cache.advance(prompts)
-            cu = torch.tensor([0] + torch.tensor(prompts).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
-            model(input_ids=ids, cu_seqlens=cu, position_ids=pos, kv_cache=cache)
-            for s in range(steps):
-                live = [1 if (i + s) % 3 or n == 1 else 0 for i in range(n)]  # sequences pause and resume
-                pos = cache.advance(live)
-                m = sum(live)
-                tok = torch.randint(0, 512, (m,), device="cuda", generator=gen)
-                cu = torch.arange(m + 1, dtype=torch.int32, device="cuda")
-                out.append(model(input_ids=tok, cu_seqlens=cu, position_ids=pos, kv_cache=cache)["hidden_states"])
+        out = _run_tokens(model, prompts, steps)
         _cuda.check_status()
     finally:
         decode_path.MAX_SEQS = keep
-    return torch.cat(out).float()
+    return out
 
 
 @pytest.mark.parametrize("kind,prompts", [("grouped", [1]), ("grouped", [63, 64, 65, 700]), ("normed", [2100]), ("normed", [5] * 7 + [130] * 11),
@@ -200,3 +206,37 @@ def test_rotary_frequencies_are_kept_per_stream_and_not_from_a_capture():
         there = backbone._frequencies(128, pos.device)
     assert there is not here and backbone._frequencies(128, pos.device) is here
     assert not hasattr(copy.deepcopy(backbone), "_fp32_frequencies")
+
+
+@pytest.mark.parametrize("seqs,hidden", [(6, 6136), (4, 8184), (6, 6144), (6, 12280), (6, 12288)])
+def test_rows_of_the_fused_norm_at_the_edges_of_shared_memory(seqs, hidden):
+    """Of six sequences four have a token in a pass, of four up to three.  Rows that fill shared memory up to the limit without an opt-in (which covers a kernel's static part too), one step past
+    it, up to the largest that the fused norm takes, and one past that."""
+    model = _model("grouped", hidden_size=hidden)
+    prompts = [5, 9, 1, 7, 3, 2][:seqs]
+    want, got = _go(model, prompts, 2, False), _go(model, prompts, 2, True)
+    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -7
+
+
+def test_threads_with_different_row_sizes():
+    """Host threads that generate with models of different widths: neither lowers the other's shared-memory limit."""
+    import threading
+
+    models = [_model("grouped", hidden_size=h) for h in (6400, 12000)]
+    prompts, errors = [3, 4, 5, 6, 1, 2], []
+
+    def work(m):
+        try:
+            for _ in range(8):
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    assert torch.isfinite(_run_tokens(m, prompts, 3)).all()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(m,)) for m in models]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors[0]
