@@ -618,7 +618,8 @@ struct GdnStepParams {
   long ldo;
   const bf16* tail_in[kDecSeqs];   // [taps - 1, conv_dim] rows that went into the convolution before this token
   bf16* tail_out[kDecSeqs];        // another buffer: heads that share key channels read the old rows
-  float* state[kDecSeqs];          // [hv, 128, 128] updated in place
+  const float* state_in[kDecSeqs]; // [hv, 128, 128]
+  float* state_out[kDecSeqs];      // another buffer: whoever holds the state before this token keeps it
 };
 
 // One CTA per (value head, sequence); thread (half, v) keeps 64 rows of column v of the state in registers, so the state
@@ -627,7 +628,9 @@ __global__ void __launch_bounds__(256) gdn_step_kernel(const __grid_constant__ G
   __shared__ float sq[kGdnD], sk[kGdnD], sv[kGdnD], part[2][kGdnD], part2[2][kGdnD], red[8];
   const int vh = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x;
   const int col = tid & (kGdnD - 1), half = tid >> 7;
-  float* S = p.state[seq] + (static_cast<size_t>(vh) * kGdnD + half * 64) * kGdnD + col;
+  const size_t at = (static_cast<size_t>(vh) * kGdnD + half * 64) * kGdnD + col;
+  const float* S = p.state_in[seq] + at;
+  float* So = p.state_out[seq] + at;
   pdl_go();
   pdl_wait();
   float st[64];
@@ -679,7 +682,7 @@ __global__ void __launch_bounds__(256) gdn_step_kernel(const __grid_constant__ G
   for (int i = 0; i < 64; ++i) {
     st[i] += sk[half * 64 + i] * kn * delta;
     oo += sq[half * 64 + i] * st[i];
-    S[i * kGdnD] = st[i];
+    So[i * kGdnD] = st[i];
   }
   part2[half][col] = oo * qn;
   __syncthreads();
@@ -823,7 +826,7 @@ static size_t up256(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
 //          12 post norm | 13 gate | 14 up | 15 down | 16 key slab | 17 value slab |
 //          19 output bias | (linear attention) 9 conv weight | 10 A_log | 16 dt_bias | 17 gated norm weight
 //   lt     per layer: 0 attention, 1 attention with an output gate, 2 Gated-DeltaNet
-//   gdn    per linear-attention layer and sequence: tail in, tail out, state
+//   gdn    per linear-attention layer and sequence: tail in, tail out, state in, state out
 //   dims   0 M 1 H 2 heads 3 kv heads 4 head dim 5 rotary dim 6 intermediate 7 window 8 splits
 //          9 key heads 10 value heads 11 taps (linear attention)
 int b200_decode_layers(const unsigned long long* lw, const int* lt, int n_layers, const int* dims, const int* base,
@@ -898,10 +901,11 @@ int b200_decode_layers(const unsigned long long* lw, const int* lt, int n_layers
       q.eps = eps;
       q.out = mix; q.ldo = val_dim;
       for (int s = 0; s < M; ++s) {
-        const unsigned long long* e = gdn + (static_cast<size_t>(gi) * M + s) * 3;
+        const unsigned long long* e = gdn + (static_cast<size_t>(gi) * M + s) * 4;
         q.tail_in[s] = reinterpret_cast<const bf16*>(e[0]);
         q.tail_out[s] = reinterpret_cast<bf16*>(e[1]);
-        q.state[s] = reinterpret_cast<float*>(e[2]);
+        q.state_in[s] = reinterpret_cast<const float*>(e[2]);
+        q.state_out[s] = reinterpret_cast<float*>(e[3]);
       }
       ++gi;
       if ((rc = launch_k(gdn_step_kernel, dim3(hv, M), 256, 0, st, q, true)) != 0) return rc;

@@ -109,8 +109,9 @@ def _delta(rec, net, cls, cfg, H):
 
 
 def _delta_state(store, net, seqs, device):
-    """Tail and state buffers of every live sequence: ``(pointers, new store entries)``; the old tail is read and a new one
-    written, because value heads that share key channels read the same old rows."""
+    """Tail and state buffers of every live sequence: ``(pointers, new store entries)``; the old ones are read and new ones
+    written, as in the layer loop: value heads that share key channels read the same old rows, and a caller may hold the state
+    of an earlier token."""
     ptrs, new = [], []
     for i in seqs:
         tail, S = store.get(i, (None, None))
@@ -122,10 +123,10 @@ def _delta_state(store, net, seqs, device):
                 or tail.device != device or S.device != device:
             raise _Unfit
         if not (tail.is_contiguous() and S.is_contiguous() and tail.dtype is _BF16 and S.dtype is torch.float32 and S.data_ptr() % 16 == 0):
-            tail, S = tail.to(_BF16).contiguous(), S.float().clone()
-        out = torch.empty_like(tail)
-        ptrs += (tail.data_ptr(), out.data_ptr(), S.data_ptr())
-        new.append((i, tail, out, S))
+            tail, S = tail.to(_BF16).contiguous(), S.float().clone(memory_format=torch.contiguous_format)
+        tail_out, S_out = torch.empty_like(tail), torch.empty_like(S)
+        ptrs += (tail.data_ptr(), tail_out.data_ptr(), S.data_ptr(), S_out.data_ptr())
+        new.append((i, tail, S, (tail_out, S_out)))
     return ptrs, new
 
 
@@ -220,6 +221,6 @@ def _run(backbone, embeds, ctx, cache, seqs):
                float(cfg.rms_norm_eps), norm_off, D ** -0.5, cos.data_ptr(), sin.data_ptr(), res.data_ptr(), hidden.data_ptr(), final,
                work.data_ptr(), work.numel(), shares.data_ptr(), count.data_ptr(), _cuda.stream())
     for store, new in news:
-        for i, _, tail, S in new:
-            store[i] = (tail, S)
+        for i, _, _, entry in new:
+            store[i] = entry
     return hidden

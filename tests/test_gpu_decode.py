@@ -240,3 +240,28 @@ def test_threads_with_different_row_sizes():
         t.join()
     torch.cuda.synchronize()
     assert not errors, errors[0]
+
+
+def test_an_earlier_recurrent_state_stays_as_it_was():
+    """A caller that keeps the entries of ``PackedKVCache.state`` can go back to them: a token replaces them and writes into
+    none."""
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    model = _model("hybrid")
+    cache = PackedKVCache(len(model.model.layers), [40], device=torch.device("cuda", 0))
+    one = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+
+    def token(t):
+        return model(input_ids=torch.tensor([t], device="cuda"), cu_seqlens=one, position_ids=cache.advance([1]), kv_cache=cache)["hidden_states"]
+
+    with torch.no_grad():
+        cu = torch.tensor([0, 30], dtype=torch.int32, device="cuda")
+        model(input_ids=torch.arange(30, device="cuda"), cu_seqlens=cu, position_ids=cache.advance([30]), kv_cache=cache)
+        token(3)
+        held = {layer: dict(entries) for layer, entries in cache.state.items()}
+        copies = {layer: {i: tuple(t.clone() for t in e) for i, e in entries.items()} for layer, entries in held.items()}
+        first = token(7)
+        token(9)
+        assert held and all(torch.equal(a, b) for layer in held for i in held[layer] for a, b in zip(held[layer][i], copies[layer][i]))
+        cache.state, cache.lens = {layer: dict(e) for layer, e in held.items()}, [31]
+        assert torch.equal(token(7), first)
