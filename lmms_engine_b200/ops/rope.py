@@ -94,29 +94,36 @@ def _apply_native(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, conj: b
 
 class _RopeFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, cos, sin):
+    def forward(ctx, x, cos, sin, conj):
         ctx.save_for_backward(cos, sin)
-        return _apply_native(x, cos, sin, False, False)
+        ctx.conj = conj
+        return _apply_native(x, cos, sin, conj, False)
 
     @staticmethod
     def backward(ctx, dy):
+        # the transposed rotation as the same function: a second derivative goes through it
         cos, sin = ctx.saved_tensors
-        return _apply_native(dy, cos, sin, True, False), None, None
+        return _RopeFn.apply(dy, cos, sin, not ctx.conj), None, None, None
+
+
+def _transformed() -> bool:
+    """Inside ``torch.func`` transforms or forward-mode differentiation, which a kernel call on raw pointers cannot follow."""
+    return torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
 
 
 def rope_apply(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """Rotate ``x [T, H, D]`` by the per-token table; differentiable."""
     if (x.is_cuda and x.dtype == torch.bfloat16 and cos.shape[-1] % 16 == 8 and x.shape[-1] % 8 == 0 and x.dim() == 3
             and cos.shape[-1] <= x.shape[-1] and cos.shape == sin.shape == (x.shape[0], cos.shape[-1]) and cos.is_cuda and sin.is_cuda
-            and cos.dtype == sin.dtype == torch.float32 and not (cos.requires_grad or sin.requires_grad)):
-        return _RopeFn.apply(x, cos.contiguous(), sin.contiguous())  # any other table of such a width takes the form below
+            and cos.dtype == sin.dtype == torch.float32 and not (cos.requires_grad or sin.requires_grad) and not _transformed()):
+        return _RopeFn.apply(x, cos.contiguous(), sin.contiguous(), False)  # any other table of such a width takes the form below
     if x.is_cuda and x.dtype == torch.bfloat16 and cos.shape[-1] % 16 == 0 and x.shape[-1] % 8 == 0:
         if cos.dtype != torch.float32 or sin.dtype != torch.float32:
             # the kernel reads the tables as fp32; a table that some wrapper cast down would be read past its end
             raise TypeError(f"rotary tables must be float32, got {cos.dtype} / {sin.dtype}")
         if cos.shape[0] < x.shape[0]:
             raise ValueError(f"rotary table has {cos.shape[0]} rows for {x.shape[0]} tokens")
-        return _RopeFn.apply(x, cos.contiguous(), sin.contiguous())
+        return _RopeFn.apply(x, cos.contiguous(), sin.contiguous(), False)
     return rope_apply_ref(x, cos, sin)
 
 

@@ -376,6 +376,34 @@ def test_rope_in_fours(T, H, D, rot):
         assert torch.allclose(u.float(), v.float(), rtol=2 ** -7, atol=2 ** -20)
 
 
+def test_rope_in_fours_under_transforms():
+    """Second derivatives, ``vmap``, forward mode and a table that needs a gradient: what the framework form of such a width
+    gives (up to one bf16 step where the kernel ran)."""
+    from lmms_engine_b200.ops import rope
+
+    torch.manual_seed(0)
+    x, dy, v = (torch.randn(9, 2, 72, device="cuda").bfloat16() for _ in range(3))
+    ang = torch.randn(9, 36, device="cuda").repeat(1, 2)
+    cos, sin = ang.cos(), ang.sin()
+
+    def second(f):  # gradient of <df(x)/dx . dy, v> with respect to dy
+        xs, g = x.clone().requires_grad_(), dy.clone().requires_grad_()
+        dx, = torch.autograd.grad(f(xs, cos, sin), xs, g, create_graph=True)
+        return torch.autograd.grad(dx, g, v)[0]
+
+    assert torch.allclose(second(rope.rope_apply).float(), second(rope.rope_apply_ref).float(), rtol=2 ** -7, atol=2 ** -8)
+    batch = torch.stack([x, dy])
+    assert torch.equal(torch.vmap(lambda t: rope.rope_apply(t, cos, sin))(batch), torch.vmap(lambda t: rope.rope_apply_ref(t, cos, sin))(batch))
+    for f in (lambda t: torch.func.jvp(lambda u: t(u, cos, sin), (x,), (v,))[1], lambda t: torch.func.vjp(lambda u: t(u, cos, sin), x)[1](dy)[0]):
+        assert torch.equal(f(rope.rope_apply), f(rope.rope_apply_ref))
+    grads = []
+    for f in (rope.rope_apply, rope.rope_apply_ref):
+        c = cos.clone().requires_grad_()
+        f(x, c, sin).backward(dy)
+        grads.append(c.grad)
+    assert torch.equal(*grads)
+
+
 @pytest.mark.parametrize("rows,H", [(1, 520), (7, 1024), (9, 1032), (2500, 1152), (33, 1280), (17, 1288), (1300, 2048), (5, 8)])
 @pytest.mark.parametrize("form", ["rms", "rms_res", "layer"])
 def test_norm_backward_warp_rows(rows, H, form):
