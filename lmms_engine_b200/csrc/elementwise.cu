@@ -422,8 +422,8 @@ norm_bwd_rows_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, co
         }
       }
     }
-    // the order of a CTA per row with a warp per 256 columns, which rows above 2048 columns and the forward passes have: the
-    // gradient does not depend on which of the kernels ran
+    // the order of a CTA per row with a warp per 256 columns, which rows above 2048 columns and the forward passes have: dx
+    // does not depend on which of the kernels ran (the weight gradients are summed per warp here, in another order)
     auto total = [](float (&s)[8]) {
 #pragma unroll
       for (int i = 0; i < VEC; ++i) s[i] = warp_sum(s[i]);
@@ -1373,7 +1373,7 @@ int b200_norm_bwd(const void* dy, const void* x, const void* w, const void* rstd
     parts = blocks * 8;
     norm_bwd_warp_kernel<<<blocks, 256, 0, st>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd,
                                                  (bf16*)dx, (float*)dw_part, rows, H, w_offset);
-  } else if (H <= 2048) {
+  } else if (H <= 2048 && !(ln && dres_in != nullptr)) {  // a LayerNorm with a residual's gradient has no caller among the layers
     // one row of partials per CTA; above 1024 columns the registers of a row leave one CTA per SM
     parts = H <= 1024 ? num_sms() * 2 : num_sms();
     if (parts > (rows + 7) / 8) parts = (rows + 7) / 8;
@@ -1383,8 +1383,7 @@ int b200_norm_bwd(const void* dy, const void* x, const void* w, const void* rstd
                                                        (float*)db_part, rows, H, w_offset)
 #define NORM_BWD_V(V)                       \
   do {                                      \
-    if (ln && dres_in) NORM_BWD(V, true, true);   \
-    else if (ln) NORM_BWD(V, true, false);  \
+    if (ln) NORM_BWD(V, true, false);       \
     else if (dres_in) NORM_BWD(V, false, true);   \
     else NORM_BWD(V, false, false);         \
   } while (0)
