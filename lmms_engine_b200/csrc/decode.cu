@@ -1,11 +1,14 @@
 // Token-by-token generation: a few rows of activations against weights and cached keys / values that are read once.
 //
 // Every product here is bound by reading its weights, every attention by reading the cached rows, and a small model by
-// the number of launches, so the path has five kernels per layer and each of them
-//   * starts loading weights BEFORE it waits for the kernel in front of it (programmatic dependent launch: weights never
-//     depend on that kernel), so that launch, ramp-up and DRAM latency of one kernel hide behind the tail of another;
-//   * reads weights straight from global memory into mma.sync fragments (no shared-memory staging, see skinny_kernel);
-//   * rounds to bf16 where the layer-by-layer path does (projection outputs, normalised rows, the residual stream), so
+// the number of launches, so the path has five kernels per layer (seven above four rows, where the norms do not fit the
+// products' prologue) and they
+//   * start before the kernel in front of them has finished (programmatic dependent launch).  The products ask for their first
+//     weights BEFORE they wait for it (weights never depend on it) and the attention for cached rows of earlier passes, so that
+//     launch, ramp-up and DRAM latency of one kernel hide behind the tail of another; the row norm and the Gated-DeltaNet step
+//     have nothing that they could load early and only launch early;
+//   * read weights straight from global memory into mma.sync fragments (no shared-memory staging, see skinny_kernel);
+//   * round to bf16 where the layer-by-layer path does (projection outputs, normalised rows, the residual stream), so
 //     both paths compute the same numbers up to the order of fp32 sums.
 //
 //   skinny_kernel   y[M, N] = x[M, K] w[N, K]^T for M <= 64 rows, RMSNorm of x in its prologue (M <= 4), bias /
@@ -86,8 +89,9 @@ struct SkinnyParams {
 // so lane (g = lane / 4, t = lane % 4) loads 16 contiguous bytes of row g at k0 + 8 t and k0 + 32 + 8 t: full 128-byte
 // lines of eight rows per warp and step, straight into fragments.
 // RT = 1 below 17 rows: N / 8 CTAs are enough to fill the chip from N = 1024 on, and a row's slice of K per warp is short.
-// From 17 rows on the activations (M x K) that every CTA reads from L2 outweigh eight weight rows, so RT grows - as long as
-// the grid still has a CTA for every SM (RT = 4 left 32 CTAs for the 1024 output rows of a narrow model).
+// From 17 rows on the activations (M x K) that every CTA reads from L2 outweigh eight weight rows, so RT grows to 2 (17 to 32
+// rows) and 4 (33 rows and more), each as long as the grid still has a CTA for every SM (RT = 4 left 32 CTAs for the 1024
+// output rows of a narrow model).
 template <int RT, int MT, int MODE, bool NORM>
 __global__ void __launch_bounds__(kSkWarps * 32) skinny_kernel(const __grid_constant__ SkinnyParams p) {
   extern __shared__ __align__(16) uint8_t dyn[];
@@ -750,12 +754,26 @@ static int launch_skinny(const SkinnyParams& p, cudaStream_t st, bool early) {
   return launch_k(skinny_kernel<RT, MT, MODE, NORM>, dim3((p.N + per - 1) / per), kSkWarps * 32, smem, st, p, early);
 }
 
+static int num_sms() {
+  static std::atomic<int> sms{0};
+  int n = sms.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    sms.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <int MT, int MODE>
 static int wide(const SkinnyParams& p, cudaStream_t st, bool early) {
   constexpr int per = MODE == SK_SWIGLU ? 4 : 8;   // output rows per weight tile
-  constexpr int kSms = 148;
-  if (MT > 2 && p.N >= kSms * per * 4) return launch_skinny<4, MT, MODE, false>(p, st, early);
-  if (MODE == SK_SWIGLU || p.N >= kSms * per * 2) return launch_skinny<2, MT, MODE, false>(p, st, early);
+  const int sms = num_sms();
+  if constexpr (MT > 2) {
+    if (p.N >= sms * per * 4) return launch_skinny<4, MT, MODE, false>(p, st, early);
+  }
+  if (MODE == SK_SWIGLU || p.N >= sms * per * 2) return launch_skinny<2, MT, MODE, false>(p, st, early);
   return launch_skinny<MODE == SK_SWIGLU ? 2 : 1, MT, MODE, false>(p, st, early);
 }
 

@@ -10,6 +10,7 @@ bf16 at the same place.
 from __future__ import annotations
 
 from array import array
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -26,6 +27,11 @@ _BF16 = torch.bfloat16
 
 class _Unfit(Exception):
     pass
+
+
+@lru_cache(maxsize=None)
+def _sms(dev) -> int:
+    return torch.cuda.get_device_properties(dev).multi_processor_count
 
 
 def _plain(module, cls) -> dict:
@@ -205,7 +211,7 @@ def _run(backbone, embeds, ctx, cache, seqs):
         longest = min(longest, cache.decode_window + 1)
     # shares of a key head: enough to fill the chip about twice or 512 keys each (a batch waits for its longest sequence),
     # whichever are more, and at least 64 keys each
-    splits = max(1, min(max(-(-296 // (nkv * M)), -(-longest // 512)), -(-longest // 64), 64))
+    splits = max(1, min(max(-(-2 * _sms(dev) // (nkv * M)), -(-longest // 512)), -(-longest // 64), 64))
     has_attn = any(t != 2 for t in types)
     np_ = max(nq * D * 2 + 2 * nkv * D if has_attn else 0, (2 * hk + 2 * hv) * 128 + 2 * hv)
     work = torch.empty(2 * M * (np_ + max(nq * D, hv * 128) + I + H) + 4096, dtype=torch.uint8, device=dev)
