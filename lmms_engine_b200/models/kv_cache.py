@@ -41,6 +41,8 @@ class PackedKVCache:
         new_lens = [int(n) for n in new_lens]
         if len(new_lens) != len(self.lens):
             raise ValueError(f"{len(new_lens)} lengths for a cache of {len(self.lens)} sequences")
+        if any(n < 0 for n in new_lens):
+            raise RuntimeError(f"new token counts {new_lens}: a pass adds tokens, it takes none away")
         self.new_lens, self.had = new_lens, list(self.lens)
         for i, n in enumerate(new_lens):
             if self.lens[i] + n > self.capacities[i]:

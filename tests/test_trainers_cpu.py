@@ -219,3 +219,14 @@ def test_cache_refuses_rows_of_another_kind(seqs):
         assert torch.equal(cache.k[0][: 2], before)
     keys = cache.extend(0, good, good)[0]
     assert torch.equal(keys.reshape(seqs, 3, 2, 4)[:, 2], good)
+
+
+def test_cache_refuses_negative_token_counts():
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    cache = PackedKVCache(1, [8, 8])
+    cache.advance([3, 2])
+    for bad in ([-1, 1], [1, -2], [-1, -1]):
+        with pytest.raises(RuntimeError):
+            cache.advance(bad)
+    assert cache.lens == [3, 2] and cache.advance([1, 1]).tolist() == [3, 2]
