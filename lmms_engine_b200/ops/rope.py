@@ -101,9 +101,10 @@ class _RopeFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        # the transposed rotation as the same function: a second derivative goes through it
+        # the transposed rotation; as the same function where a second derivative is to go through it
         cos, sin = ctx.saved_tensors
-        return _RopeFn.apply(dy, cos, sin, not ctx.conj), None, None, None
+        dx = _RopeFn.apply(dy, cos, sin, not ctx.conj) if torch.is_grad_enabled() else _apply_native(dy, cos, sin, not ctx.conj, False)
+        return dx, None, None, None
 
 
 def _transformed() -> bool:
