@@ -69,11 +69,18 @@ def _go(model, prompts, steps, native):
 @pytest.mark.parametrize("kind,prompts", [("grouped", [1]), ("grouped", [63, 64, 65, 700]), ("normed", [2100]), ("normed", [5] * 7 + [130] * 11),
                                           ("narrow", [17, 300]), ("wide_group", [129, 40]), ("window", [50, 200]), ("hybrid", [100]),
                                           ("hybrid", [64, 1, 130]), ("normed", list(range(1, 41))), ("normed", list(range(1, 65)))])
-def test_one_call_matches_layer_loop(kind, prompts):
+def test_one_call_matches_layer_loop(kind, prompts, monkeypatch):
     """Both paths round every intermediate to bf16 at the same place, so only elements whose fp32 sums land on either side of
     a rounding boundary differ, by one bf16 step (2^-8); two layers carry a few of those into an output of rms 1."""
+    from lmms_engine_b200.ops import _cuda
+
     model = _model(kind)
-    want, got = _go(model, prompts, 5, False), _go(model, prompts, 5, True)
+    seen, real = [], _cuda.call
+    monkeypatch.setattr(_cuda, "call", lambda name, *a: (seen.append(name), real(name, *a))[1])
+    want = _go(model, prompts, 5, False)
+    assert "b200_decode_layers" not in seen
+    got = _go(model, prompts, 5, True)
+    assert seen.count("b200_decode_layers") == 5
     assert torch.isfinite(got).all()
     rel = ((got - want).norm() / want.norm()).item()
     assert rel < 2.0 ** -7, rel
@@ -210,12 +217,15 @@ def test_rotary_frequencies_are_kept_per_stream_and_not_from_a_capture():
 
 @pytest.mark.parametrize("seqs,hidden", [(6, 6136), (4, 8184), (6, 6144), (6, 12280), (6, 12288)])
 def test_rows_of_the_fused_norm_at_the_edges_of_shared_memory(seqs, hidden):
-    """Of six sequences four have a token in a pass, of four up to three.  Rows that fill shared memory up to the limit without an opt-in (which covers a kernel's static part too), one step past
-    it, up to the largest that the fused norm takes, and one past that."""
+    """Of six sequences four have a token in a pass, of four up to three.  Rows that fill shared memory up to the limit without
+    an opt-in (which covers a kernel's static part too), one step past it, up to the largest that the fused norm takes, and one
+    past that.  Against the same weights in fp32: no further off than the layer loop, whose roundings are as many (a few per
+    cent apart over some ten thousand values)."""
     model = _model("grouped", hidden_size=hidden)
     prompts = [5, 9, 1, 7, 3, 2][:seqs]
-    want, got = _go(model, prompts, 2, False), _go(model, prompts, 2, True)
-    assert ((got - want).norm() / want.norm()).item() < 2.0 ** -7
+    loop, got = _go(model, prompts, 2, False), _go(model, prompts, 2, True)
+    want = _go(model.float(), prompts, 2, False)
+    assert (got - want).norm() < 1.15 * (loop - want).norm()
 
 
 def test_threads_with_different_row_sizes():
