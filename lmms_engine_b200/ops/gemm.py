@@ -22,9 +22,24 @@ LINEAR_BACKEND = "tcgen05"
 _cuda.register("b200_colsum_parts", "elementwise", "ii")
 _cuda.register("b200_colsum_bf16", "elementwise", "plppiii" + "s")
 _cuda.register("b200_skinny_linear", "decode", "pppp" + "iii" + "lll" + "s")
-# Products of at most this many rows are bound by reading the weights once: one kernel spreads the weight rows over the
-# whole chip (csrc/decode.cu) where a 256-column tile would leave most of it idle.
+# Products of at most this many rows have two kernels.  The tcgen05 one takes a tile of 256 weight rows per CTA: below about
+# 37k weight rows part of the chip is idle and its time is the latency of one tile (17 us at K = 1024, 32 at 3584).  The one
+# of csrc/decode.cu takes eight to thirty-two weight rows per CTA, which fills the chip at any width, but every CTA reads
+# all activations from L2, so its rate falls with the rows: 5.6 TB/s of weights at one row, 2.2 at 64.
 SKINNY_ROWS = 64
+
+
+def few_rows_kernel(M: int, N: int, K: int) -> bool:
+    """Whether ``[M, K] x [N, K]^T`` runs on the kernel for few rows.  The lines lie where both measured the same (K 512 to 8192,
+    weights out of L2), us, tcgen05 / few rows: 4 rows, N 16384: 19.5 / 17.4 (K 1024), 28672: 23.6 / 23.5; K 3584, N 152064:
+    210 / 190; 16 rows, N 12288: 19.5 / 16.4, 40 / 37; 18944: 19.5 / 20.5, 46 / 50; 32 rows, N 8192: 17.4 / 15.2, 36 / 33; 10240:
+    17.4 / 18.5, 38 / 43; 48 rows, N 4096: 17.3 / 12.3, 32 / 28; 6144: 17.3 / 17.4, 34 / 39; 64 rows, N 2048: 15.4 / 13.3,
+    32 / 26; 4096: 17.4 / 15.3, 32 / 37.  Far past the lines it is up to three times slower (64 rows, N 151936, K 1024: 62 / 185)."""
+    if M > SKINNY_ROWS:
+        return False
+    if M <= 4:  # up to four rows, weights stream at the memory rate in both; short rows of weights favour the larger tile
+        return N <= 16384 or (K >= 2048 and (M == 1 or K <= 4096))
+    return N <= (12288 if M <= 16 else 8192 if M <= 32 else 4096 if M <= 48 else 3584)
 
 
 def _ok(t: torch.Tensor) -> bool:
@@ -78,7 +93,7 @@ def gemm(
         raise TypeError("bad cin tensor")
     if bias is not None and bias.numel() != N:
         raise ValueError(f"{bias.numel()} bias entries for {N} outputs")
-    if M <= SKINNY_ROWS and not (a_mn_major or b_mn_major or symmetric) and alpha == 1.0 and cin is None and (N | K) % 8 == 0:
+    if not (a_mn_major or b_mn_major or symmetric) and alpha == 1.0 and cin is None and (N | K) % 8 == 0 and few_rows_kernel(M, N, K):
         _cuda.call("b200_skinny_linear", a.data_ptr(), b.data_ptr(), _cuda.ptr(bias), out.data_ptr(), M, N, K, a.stride(0),
                    b.stride(0), out.stride(0), _cuda.stream())
         return out

@@ -147,6 +147,23 @@ def test_few_rows(M, N, K):
         assert ((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4 * K ** 0.5).all()
 
 
+@pytest.mark.parametrize("M,N,K,few", [(1, 16384, 64, True), (1, 16392, 64, False), (1, 16392, 2048, True), (4, 16392, 8192, False),
+                                       (5, 12288, 64, True), (16, 12296, 64, False), (17, 8192, 64, True), (32, 8200, 64, False),
+                                       (33, 4096, 64, True), (48, 4104, 64, False), (49, 3584, 64, True), (64, 3592, 64, False),
+                                       (65, 64, 64, False)])
+def test_few_rows_take_the_kernel_that_is_faster(M, N, K, few, monkeypatch):
+    """Both sides of every line of the rule; either kernel gives fp32 sums rounded once."""
+    from lmms_engine_b200.ops import gemm, _cuda
+
+    seen, real = [], _cuda.call
+    monkeypatch.setattr(_cuda, "call", lambda name, *a: (seen.append(name), real(name, *a))[1])
+    x, w, b = _rand(M, K), _rand(N, K, scale=0.05), _rand(N)
+    y = gemm.matmul_nt(x, w, b)
+    assert ("b200_skinny_linear" in seen) == few
+    want = x.float() @ w.float().t() + b.float()
+    assert ((y.float() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4 * K ** 0.5).all()
+
+
 @pytest.mark.parametrize("P,K,inter,N,biases", [(1, 64, 36, 64, True), (65, 72, 100, 136, True), (300, 128, 130, 64, False),
                                                (257, 1280, 3420, 1280, True), (129, 64, 3, 8, True)])
 def test_gated_mlp_any_width(P, K, inter, N, biases):
