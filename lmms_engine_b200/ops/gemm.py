@@ -123,9 +123,10 @@ def matmul_tn(dy: torch.Tensor, x: torch.Tensor, out=None, cin=None, beta: float
 
 
 def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, store_gu: bool = True, bg: Optional[torch.Tensor] = None,
-                bu: Optional[torch.Tensor] = None):
+                bu: Optional[torch.Tensor] = None, whole_rows: bool = False):
     """``h = silu(x wg^T + bg) * (x wu^T + bu)`` in one kernel; also returns gate/up when asked.  A width that is no multiple
-    of 8 gets rows padded to one: the results are views ``[M, width]`` of them, and nothing writes the padding."""
+    of 8 gets rows padded to one: the results are views ``[M, width]`` of them (the buffers themselves with ``whole_rows``),
+    and nothing writes the padding."""
     if not (_ok(x) and _ok(wg) and _ok(wu)):
         raise TypeError("gemm_swiglu needs contiguous CUDA bf16 operands")
     M, K = x.shape
@@ -145,7 +146,7 @@ def gemm_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, store_gu: b
         x.data_ptr(), wg.data_ptr(), wu.data_ptr(), h.data_ptr(), _cuda.ptr(g), _cuda.ptr(u), M, inter, K,
         x.stride(0), wg.stride(0), ld, int(store_gu), _cuda.ptr(bg), _cuda.ptr(bu), st.data_ptr(), _cuda.stream(),
     )
-    if ld != inter:
+    if ld != inter and not whole_rows:
         h, g, u = h[:, :inter], (g[:, :inter] if store_gu else None), (u[:, :inter] if store_gu else None)
     return h, g, u
 

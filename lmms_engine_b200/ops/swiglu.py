@@ -113,8 +113,10 @@ class _GatedMLPFn(torch.autograd.Function):
     def forward(ctx, x, wg, bg, wu, bu, wd, bd):
         shp = x.shape
         x2 = _rows16(x.reshape(-1, shp[-1]))
-        h, g, u = _gemm.gemm_swiglu(x2, wg, wu, True, bg, bu)
-        y = _gemm.gemm(h, _padded(wd), bias=bd)
+        # whole padded rows are saved: a hook on saved tensors (offloading) copies a view without its padding, which the
+        # elementwise pass of the backward would read past
+        h, g, u = _gemm.gemm_swiglu(x2, wg, wu, True, bg, bu, whole_rows=True)
+        y = _gemm.gemm(h[:, :wg.shape[0]], _padded(wd), bias=bd)
         ctx.save_for_backward(x2, wg, wu, wd, g, u)
         ctx.shp, ctx.biases = shp, (bg is not None, bu is not None, bd is not None)
         return y.view(*shp[:-1], wd.shape[0])

@@ -1,4 +1,6 @@
 """tcgen05 GEMM against an fp32 PyTorch reference (all operand layouts and epilogues)."""
+import contextlib
+
 import pytest
 import torch
 
@@ -193,6 +195,24 @@ def test_gated_mlp_any_width(P, K, inter, N, biases):
     for t, f in zip(dev, first):
         if t is not None:
             assert torch.equal(t.grad, f + f)
+
+
+@pytest.mark.parametrize("inter", [36, 40])
+def test_gated_mlp_under_saved_tensor_hooks(inter):
+    """Activations that are moved to the host and back between the passes come back without the strides of a view."""
+    from lmms_engine_b200.ops import swiglu
+
+    torch.manual_seed(0)
+    raw = [_rand(130, 64), _rand(inter, 64, scale=0.1), _rand(inter), _rand(inter, 64, scale=0.1), _rand(inter), _rand(72, inter, scale=0.1), _rand(72)]
+    dy, grads = _rand(130, 72), []
+    for hooked in (False, True):
+        leaves = [t.clone().requires_grad_() for t in raw]
+        with torch.autograd.graph.save_on_cpu(pin_memory=True) if hooked else contextlib.nullcontext():
+            y = swiglu._GatedMLPFn.apply(*leaves)
+        y.backward(dy)
+        grads.append([t.grad for t in leaves])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("inter", [36, 40])
