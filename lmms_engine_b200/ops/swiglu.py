@@ -117,26 +117,26 @@ class _GatedMLPFn(torch.autograd.Function):
         # elementwise pass of the backward would read past
         h, g, u = _gemm.gemm_swiglu(x2, wg, wu, True, bg, bu, whole_rows=True)
         y = _gemm.gemm(h[:, :wg.shape[0]], _padded(wd), bias=bd)
-        ctx.save_for_backward(x2, wg, wu, wd, g, u)
+        # h too, as three linears keep it: computing it again is a pass over all three
+        ctx.save_for_backward(x2, wg, wu, wd, g, u, h)
         ctx.shp, ctx.biases = shp, (bg is not None, bu is not None, bd is not None)
         return y.view(*shp[:-1], wd.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        x2, wg, wu, wd, g, u = ctx.saved_tensors
+        x2, wg, wu, wd, g, u, h = ctx.saved_tensors
         need = ctx.needs_input_grad
         dy2 = _rows16(dy.reshape(-1, dy.shape[-1]))
         M, inter = x2.shape[0], wg.shape[0]
         ld = (inter + 7) // 8 * 8
-        # elementwise passes run over whole padded rows: the padding holds anything and is not read again
-        h, dg, du = (torch.empty((M, ld), dtype=g.dtype, device=g.device) for _ in range(3))
-        _cuda.call("b200_swiglu_fwd", g.data_ptr(), u.data_ptr(), h.data_ptr(), M * ld, _cuda.stream())
+        # the elementwise pass runs over whole padded rows: the padding holds anything and is not read again
+        dh, dg, du = (torch.empty((M, ld), dtype=g.dtype, device=g.device) for _ in range(3))
         dwd = None
         if need[5]:
             dwd = torch.empty((wd.shape[0], ld), dtype=wd.dtype, device=wd.device)[:, :inter]
             _gemm.matmul_tn(dy2, h[:, :inter], out=dwd)
-        _gemm.matmul_nn(dy2, _padded(wd), out=h[:, :inter])
-        _cuda.call("b200_swiglu_bwd", h.data_ptr(), g.data_ptr(), u.data_ptr(), dg.data_ptr(), du.data_ptr(), M * ld, _cuda.stream())
+        _gemm.matmul_nn(dy2, _padded(wd), out=dh[:, :inter])
+        _cuda.call("b200_swiglu_bwd", dh.data_ptr(), g.data_ptr(), u.data_ptr(), dg.data_ptr(), du.data_ptr(), M * ld, _cuda.stream())
         dg, du = dg[:, :inter], du[:, :inter]
         dx = None
         if need[0]:
