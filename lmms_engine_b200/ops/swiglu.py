@@ -162,14 +162,22 @@ def _padded(wd):
     return torch.empty((n, (i + 7) // 8 * 8), dtype=wd.dtype, device=wd.device)[:, :i].copy_(wd)
 
 
+# Rows x width x inner width from which an inner width that is no multiple of 8 takes the fused function: below, host time decides,
+# and the library's three linears launch less.  Forward + backward, us, linears / fused: 100 x 1280 x 3420 360 / 515, 2000 x 256 x
+# 516 375 / 503, 22000 x 256 x 516 (2.9e9) 700 / 683, 2000 x 1280 x 3420 (8.8e9) 854 / 508, 22000 x 1280 x 3420 6540 / 1640.
+UNALIGNED_MIN = 1 << 31
+
+
 def gated_mlp(x, wg, bg, wu, bu, wd, bd) -> torch.Tensor:
     """``(silu(x wg^T + bg) * (x wu^T + bu)) wd^T + bd``; any of the biases may be ``None``.
 
-    One fused function for every width: as three linears, an inner width that is no multiple of 8 went to the library's
-    unaligned kernels (49 of the 94 device ms of an eight-block tower with 3420 over 21.9k patches, forward + backward)."""
+    One fused function: as three linears, an inner width that is no multiple of 8 went to the library's unaligned kernels (49 of
+    the 94 device ms of an eight-block tower with 3420 over 21.9k patches, forward + backward).  Such a width takes the linears
+    where the products are small (``UNALIGNED_MIN``)."""
     plain = (torch.Tensor, torch.nn.Parameter)
     native = (
         _gemm.LINEAR_BACKEND == "tcgen05" and x.is_cuda and x.dtype == torch.bfloat16 and x.numel() > 0 and wg.shape == wu.shape
+        and (wg.shape[0] % 8 == 0 or x.numel() * wg.shape[0] >= UNALIGNED_MIN)
         and x.shape[-1] % 8 == 0 and wg.shape[1] == x.shape[-1] and wd.shape[0] % 8 == 0 and wd.shape[1] == wg.shape[0]
         and all(type(w) in plain and w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0
                 for w in (wg, wu, wd))

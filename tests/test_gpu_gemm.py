@@ -197,6 +197,21 @@ def test_gated_mlp_any_width(P, K, inter, N, biases):
             assert torch.equal(t.grad, f + f)
 
 
+@pytest.mark.parametrize("P,K,inter,N,biases", [(1, 64, 36, 64, True), (65, 72, 100, 136, True), (300, 128, 130, 64, False),
+                                               (257, 1280, 3420, 1280, True), (129, 64, 3, 8, True)])
+def test_gated_mlp_fused_at_small_sizes(P, K, inter, N, biases, monkeypatch):
+    """Unaligned widths below the line run as linears; the fused function has to hold there too."""
+    from lmms_engine_b200.ops import swiglu, _cuda
+
+    seen, real = [], _cuda.call
+    monkeypatch.setattr(_cuda, "call", lambda name, *a: (seen.append(name), real(name, *a))[1])
+    test_gated_mlp_any_width(P, K, inter, N, biases)
+    assert "b200_gemm_swiglu_bf16" not in seen
+    monkeypatch.setattr(swiglu, "UNALIGNED_MIN", 0)
+    test_gated_mlp_any_width(P, K, inter, N, biases)
+    assert "b200_gemm_swiglu_bf16" in seen
+
+
 @pytest.mark.parametrize("inter", [36, 40])
 def test_gated_mlp_under_saved_tensor_hooks(inter):
     """Activations that are moved to the host and back between the passes come back without the strides of a view."""
