@@ -17,12 +17,13 @@ import torch
 
 from ..ops import _cuda
 from ..ops import gemm as gemm_ops
-from .plain_call import global_hooks, own_call
+from .plain_call import global_hooks, own_forward
 
 _cuda.register("b200_decode_layers", "decode", "ppi" + "pppp" + "fff" + "ppppp" + "p" + "l" + "pp" + "s")
 
 MAX_SEQS = 64  # kDecSeqs of the kernels: per-sequence tables travel as kernel arguments
 _BF16 = torch.bfloat16
+_PARAM = torch.nn.Parameter
 
 
 class _Unfit(Exception):
@@ -35,98 +36,84 @@ def _sms(dev) -> int:
 
 
 def _plain(module, cls) -> dict:
-    """Parameters of a module whose call is only the arithmetic of its class."""
-    if not own_call(module, cls):
+    """Parameters of a module whose call is only the arithmetic of its class (``plain_call.own_call`` with the part that is the
+    same for all modules of a class done once per pass, and without backward hooks: there is no backward pass)."""
+    d = module.__dict__
+    if type(module) is not cls or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
         raise _Unfit
-    return module._parameters
+    return d["_parameters"]
 
 
-def _at(w, shape) -> int:
-    if w is None or w.dtype is not _BF16 or type(w) is not torch.nn.Parameter or not w.is_cuda or w.shape != shape or not w.is_contiguous():
-        raise _Unfit
-    p = w.data_ptr()
-    if p & 15:
-        raise _Unfit
-    return p
+def _fill(rec, items) -> None:
+    """``rec[slot]`` = address of every plain bf16 weight ``(slot, weight, shape)``."""
+    for slot, w, shape in items:
+        if type(w) is not _PARAM or w.dtype is not _BF16 or w.shape != shape or not (w.is_cuda and w.is_contiguous()):
+            raise _Unfit
+        p = w.data_ptr()
+        if p & 15:
+            raise _Unfit
+        rec[slot] = p
 
 
-def _opt(w, shape) -> int:
-    return 0 if w is None else _at(w, shape)
-
-
-def _norm(module, cls, cfg, width) -> int:
-    own = _plain(module, cls)
-    if module.eps != cfg.rms_norm_eps:  # one eps for all norms of the call
-        raise _Unfit
-    return _at(own.get("weight"), (width,))
-
-
-def _weight(module, shape, cls=torch.nn.Linear) -> int:
-    """Weight of a projection.  Its layer reads the weight and never calls the module, so hooks on it do not matter, but a
-    subclass may compute its weight on access."""
+def _own(module, cls=torch.nn.Linear) -> dict:
+    """Parameters of a projection.  Its layer reads the weight and never calls the module, so hooks on it do not matter, but a
+    subclass (a parametrisation makes one) may compute its weight on access."""
     if type(module) is not cls:
         raise _Unfit
-    return _at(module._parameters.get("weight"), shape)
+    return module.__dict__["_parameters"]
 
 
-def _mlp(rec, mlp, cls, H, I):
-    _plain(mlp, cls)
-    if mlp.tp_group is not None:
+def _norm(module, cls, eps):
+    own = _plain(module, cls)
+    if module.__dict__.get("eps") != eps:  # one eps for all norms of the call
         raise _Unfit
-    m = mlp._modules
-    rec[13] = _weight(m["gate_proj"], (I, H))
-    rec[14] = _weight(m["up_proj"], (I, H))
-    rec[15] = _weight(m["down_proj"], (H, I))
+    return own.get("weight")
 
 
-def _attention(rec, att, cls, norm_cls, cfg, cache, dev, H, nq, nkv, D, gated):
+def _attention(items, att, cls, norm_cls, eps, window, shapes, gated):
     _plain(att, cls)
-    m = att._modules
-    if getattr(att, "nsa", None) is not None or getattr(att, "window", (-1, -1))[0] != cache.decode_window:
+    m = att.__dict__["_modules"]
+    if getattr(att, "nsa", None) is not None or getattr(att, "window", (-1, -1))[0] != window:
         raise _Unfit
-    rows = nq * D * (2 if gated else 1)
-    for i, (name, n) in enumerate((("q_proj", rows), ("k_proj", nkv * D), ("v_proj", nkv * D))):
-        rec[1 + i] = _weight(m[name], (n, H))
-        rec[5 + i] = _opt(m[name]._parameters.get("bias"), (n,))
+    q_shape, kv_shape, q_bias, kv_bias, head, o_shape, o_bias = shapes
+    q, k, v, o = _own(m["q_proj"]), _own(m["k_proj"]), _own(m["v_proj"]), _own(m["o_proj"])
+    items += ((1, q.get("weight"), q_shape), (2, k.get("weight"), kv_shape), (3, v.get("weight"), kv_shape), (11, o.get("weight"), o_shape))
+    for slot, own, shape in ((5, q, q_bias), (6, k, kv_bias), (7, v, kv_bias)):
+        if own.get("bias") is not None:
+            items.append((slot, own["bias"], shape))
+    if gated and o.get("bias") is not None:  # the ungated layer adds none
+        items.append((19, o["bias"], o_bias))
     if gated or att.cfg.qk_norm:
-        rec[9] = _norm(m["q_norm"], norm_cls, cfg, D)
-        rec[10] = _norm(m["k_norm"], norm_cls, cfg, D)
-    rec[11] = _weight(m["o_proj"], (H, nq * D))
-    rec[19] = _opt(m["o_proj"]._parameters.get("bias"), (H,)) if gated else 0  # the ungated layer adds none
-    k, v = cache.slabs(att.layer_idx, nkv, D, _BF16, dev)
-    if k.dtype is not _BF16 or k.device != dev or k.shape[1:] != (nkv, D):
-        raise _Unfit
-    rec[16], rec[17] = k.data_ptr(), v.data_ptr()
+        items += ((9, _norm(m["q_norm"], norm_cls, eps), head), (10, _norm(m["k_norm"], norm_cls, eps), head))
 
 
-def _delta(rec, net, cls, cfg, H):
+def _delta(items, net, cls, eps, H):
     own = _plain(net, cls)
-    m = net._modules
+    m = net.__dict__["_modules"]
     # the gated output norm is a weight without a call of its own; its eps stands at the layer
-    if net.eps != cfg.rms_norm_eps or type(m["norm"]) is not torch.nn.Module:
+    if net.eps != eps or type(m["norm"]) is not torch.nn.Module:
         raise _Unfit
     key, val, hv = net.key_dim, net.value_dim, net.hv
     for i, (name, n) in enumerate((("in_proj_qkv", 2 * key + val), ("in_proj_z", val), ("in_proj_b", hv), ("in_proj_a", hv))):
-        rec[1 + i] = _weight(m[name], (n, H))
-    rec[9] = _weight(m["conv1d"], (2 * key + val, 1, net.kernel), torch.nn.Conv1d)
-    rec[10], rec[16] = _at(own.get("A_log"), (hv,)), _at(own.get("dt_bias"), (hv,))
-    rec[17] = _at(m["norm"]._parameters.get("weight"), (net.dv,))
-    rec[11] = _weight(m["out_proj"], (H, val))
+        items.append((1 + i, _own(m[name]).get("weight"), (n, H)))
+    items += ((9, _own(m["conv1d"], torch.nn.Conv1d).get("weight"), (2 * key + val, 1, net.kernel)), (10, own.get("A_log"), (hv,)),
+              (16, own.get("dt_bias"), (hv,)), (17, m["norm"]._parameters.get("weight"), (net.dv,)),
+              (11, _own(m["out_proj"]).get("weight"), (H, val)))
 
 
-def _delta_state(store, net, seqs, device):
+def _delta_state(store, net, seqs, where):
     """Tail and state buffers of every live sequence: ``(pointers, new store entries)``; the old ones are read and new ones
     written, as in the layer loop: value heads that share key channels read the same old rows, and a caller may hold the state
     of an earlier token."""
     ptrs, new = [], []
+    at, tail_shape, state_shape = where.get_device(), (net.kernel - 1, 2 * net.key_dim + net.value_dim), (net.hv, net.dk, net.dv)
     for i in seqs:
         tail, S = store.get(i, (None, None))
         if tail is None:
-            tail = torch.zeros((net.kernel - 1, 2 * net.key_dim + net.value_dim), dtype=_BF16, device=device)
+            tail = torch.zeros(tail_shape, dtype=_BF16, device=where.device)
         if S is None:
-            S = torch.zeros((net.hv, net.dk, net.dv), dtype=torch.float32, device=device)
-        if tail.shape != (net.kernel - 1, 2 * net.key_dim + net.value_dim) or S.shape != (net.hv, net.dk, net.dv) \
-                or tail.device != device or S.device != device:
+            S = torch.zeros(state_shape, dtype=torch.float32, device=where.device)
+        if tail.shape != tail_shape or S.shape != state_shape or tail.get_device() != at or S.get_device() != at:
             raise _Unfit
         if not (tail.is_contiguous() and S.is_contiguous() and tail.dtype is _BF16 and S.dtype is torch.float32 and S.data_ptr() % 16 == 0):
             tail, S = tail.to(_BF16).contiguous(), S.float().clone(memory_format=torch.contiguous_format)
@@ -173,35 +160,53 @@ def _run(backbone, embeds, ctx, cache, seqs):
         if type(first) is not hybrid.Qwen35Layer:
             raise _Unfit
         layer_cls, att_cls, norm_cls, norm_off = hybrid.Qwen35Layer, hybrid.GatedAttention, hybrid.ZRMSNorm, 1.0
+    if not all(map(own_forward, (layer_cls, att_cls, norm_cls, SwiGLUMLP))) or (hybrid is not None and not own_forward(hybrid.GatedDeltaNet)):
+        raise _Unfit
     table, types, nets = array("Q"), array("i"), []
     rec0 = [0] * 24
     hk = hv = taps = 0
+    gated, eps, window = hybrid is not None, cfg.rms_norm_eps, cache.decode_window
+    q_rows = nq * D * (2 if gated else 1)
+    shapes = ((q_rows, H), (nkv * D, H), (q_rows,), (nkv * D,), (D,), (H, nq * D), (H,))
+    row, wide, narrow = (H,), (I, H), (H, I)
     for layer in layers.values():
-        rec = rec0[:]
         _plain(layer, layer_cls)
-        m = layer._modules
-        if hybrid is not None and "linear_attn" in m:
+        m = layer.__dict__["_modules"]
+        rec, items, mlp = rec0[:], [], m["mlp"]
+        _plain(mlp, SwiGLUMLP)
+        if mlp.tp_group is not None:
+            raise _Unfit
+        if gated and "linear_attn" in m:
             net = m["linear_attn"]
-            _delta(rec, net, hybrid.GatedDeltaNet, cfg, H)
+            _delta(items, net, hybrid.GatedDeltaNet, eps, H)
             if net.dk != 128 or net.dv != 128 or net.hv % 8 or net.hv % net.hk or not 2 <= net.kernel <= 8:
                 raise _Unfit
             hk, hv, taps = net.hk, net.hv, net.kernel
             nets.append(net)
             types.append(2)
         else:
-            _attention(rec, m["self_attn"], att_cls, norm_cls, cfg, cache, dev, H, nq, nkv, D, hybrid is not None)
-            types.append(0 if hybrid is None else 1)
-        for at, name in ((0, "input_layernorm"), (12, "post_attention_layernorm")):
-            rec[at] = _norm(m[name], norm_cls, cfg, H)
-        _mlp(rec, m["mlp"], SwiGLUMLP, H, I)
+            att = m["self_attn"]
+            _attention(items, att, att_cls, norm_cls, eps, window, shapes, gated)
+            k, v = cache.slabs(att.layer_idx, nkv, D, _BF16, dev)
+            if k.dtype is not _BF16 or k.device != dev or k.shape[1:] != (nkv, D):
+                raise _Unfit
+            rec[16], rec[17] = k.data_ptr(), v.data_ptr()
+            types.append(1 if gated else 0)
+        mm = mlp.__dict__["_modules"]
+        items += ((0, _norm(m["input_layernorm"], norm_cls, eps), row), (12, _norm(m["post_attention_layernorm"], norm_cls, eps), row),
+                  (13, _own(mm["gate_proj"]).get("weight"), wide), (14, _own(mm["up_proj"]).get("weight"), wide),
+                  (15, _own(mm["down_proj"]).get("weight"), narrow))
+        _fill(rec, items)
         table.extend(rec)
-    final = _norm(backbone._modules["norm"], norm_cls, cfg, H)
+    last = [0]
+    _fill(last, ((0, _norm(backbone._modules["norm"], norm_cls, eps), row),))
+    final = last[0]
 
     # the states are replaced after the call: what declines here leaves them as they were
     gdn, news = array("Q"), []
     for net in nets:
         store = cache.state.setdefault(net.layer_idx, {})
-        ptrs, new = _delta_state(store, net, seqs, dev)
+        ptrs, new = _delta_state(store, net, seqs, embeds)
         gdn.extend(ptrs)
         news.append((store, new))
     have = array("i", [cache.had[i] for i in seqs])

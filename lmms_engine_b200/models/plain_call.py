@@ -14,11 +14,16 @@ def global_hooks() -> bool:
     return bool(_nn._global_forward_hooks or _nn._global_forward_pre_hooks or _nn._global_backward_hooks or _nn._global_backward_pre_hooks)
 
 
+def own_forward(cls) -> bool:
+    """Whether ``cls.forward`` is the one that the class was written with."""
+    fwd = cls.forward
+    return getattr(fwd, "__qualname__", "") == cls.__qualname__ + ".forward" and fwd.__module__ == cls.__module__
+
+
 def own_call(module, cls) -> bool:
     """Whether calling ``module`` runs ``cls.forward`` as ``cls`` defines it and nothing else (apart from ``global_hooks``)."""
     if type(module) is not cls:
         return False
     d = module.__dict__
-    fwd = cls.forward
-    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d
-                or getattr(fwd, "__qualname__", "") != cls.__qualname__ + ".forward" or fwd.__module__ != cls.__module__)
+    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d) \
+        and own_forward(cls)

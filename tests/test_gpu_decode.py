@@ -80,7 +80,7 @@ def test_one_call_matches_layer_loop(kind, prompts, monkeypatch):
     want = _go(model, prompts, 5, False)
     assert "b200_decode_layers" not in seen
     got = _go(model, prompts, 5, True)
-    assert seen.count("b200_decode_layers") == 5
+    assert seen.count("b200_decode_layers") == 5 + all(n == 1 for n in prompts)  # prompts of one token are such a pass too
     assert torch.isfinite(got).all()
     rel = ((got - want).norm() / want.norm()).item()
     assert rel < 2.0 ** -7, rel
