@@ -153,24 +153,39 @@ __device__ __forceinline__ void load_unit(float* dst, float* rs, const T* x, lon
     st4(dst + r * LB + lane * 4, scaled(scaled(v, inv), scale));
   }
 }
-// Cumulated log decays and write strengths of a chunk; ends with a barrier.
+// A cumulated log decay as the unevaluated sum of two floats.  Decays are exponentials of differences of these sums, so the error
+// of a sum in 32 bits (2^-24 of its size, which is many times the difference) shows in every one of them; a scan over lanes
+// rounds neighbours independently, which left the outputs 1.3 times as far from the exact rule as a sum in order (2.0e-6 against
+// 1.5e-6 of the 2-norm at decays of up to 16; 2.2e-7 this way).
+struct LogDecay {
+  float hi, lo;
+  __device__ __forceinline__ float minus(const LogDecay& o) const { return (hi - o.hi) + (lo - o.lo); }
+};
+
+// Cumulated log decays (summed in 64 bits) and write strengths of a chunk; ends with a barrier.
 template <typename T>
-__device__ __forceinline__ void load_gates(const ChunkStream<T>& p, long* rowmap, float* sG, float* sB, int chunk, int h) {
+__device__ __forceinline__ void load_gates(const ChunkStream<T>& p, long* rowmap, LogDecay* sG, float* sB, int chunk, int h) {
+  __shared__ double first_half;
   const int tid = threadIdx.x, lane = tid & 31;
+  double gv = 0.0;
   if (tid < CC) {
     const long row = chunk_row(p.src, p.rows, chunk, tid);
     rowmap[tid] = row;
-    float gv = row >= 0 ? p.g[row * p.H + h] : 0.f;
+    gv = row >= 0 ? static_cast<double>(p.g[row * p.H + h]) : 0.0;
     sB[tid] = row >= 0 ? p.beta[row * p.H + h] : 0.f;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, gv, o);
+      const double up = __shfl_up_sync(0xffffffffu, gv, o);
       if (lane >= o) gv += up;
     }
-    sG[tid] = gv;
+    if (tid == 31) first_half = gv;
   }
   __syncthreads();
-  if (tid >= 32 && tid < CC) sG[tid] += sG[31];
+  if (tid < CC) {
+    if (tid >= 32) gv += first_half;
+    const float hi = static_cast<float>(gv);
+    sG[tid] = {hi, fabsf(hi) < INFINITY ? static_cast<float>(gv - hi) : 0.f};
+  }
   __syncthreads();
 }
 
@@ -228,21 +243,22 @@ chunk_fwd_kernel(const ChunkStream<T> p, float* __restrict__ w, float* __restric
   float* sX = sK + CC * LB;      // queries, later values
   float* sA = sX + CC * LB;
   float* sT = sA + CC * LS;
-  __shared__ float sG[CC], sB[CC], sE[CC], rs[CC];
+  __shared__ LogDecay sG[CC];
+  __shared__ float sB[CC], sE[CC], rs[CC];
   __shared__ long rowmap[CC];
   const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const long at = static_cast<long>(h) * p.n + chunk;
   load_gates(p, rowmap, sG, sB, chunk, h);
   load_unit(sK, rs, p.k, p.ldk, rowmap, h, 1.f);
   load_unit(sX, rs, p.q, p.ldq, rowmap, h, p.scale);
-  const float g_last = sG[CC - 1];
-  if (tid < CC) sE[tid] = expf(sG[tid]);
-  if (tid == 0) gamma[at] = expf(g_last);
+  const LogDecay g_last = sG[CC - 1];
+  if (tid < CC) sE[tid] = expf(sG[tid].hi);
+  if (tid == 0) gamma[at] = expf(g_last.hi);
   __syncthreads();
   for (int i = tid; i < CC * CD / 4; i += CT) {
     const int r = i >> 5, c = (i & 31) * 4;
     st4(qt + at * CC * CD + i * 4, scaled(ld4(sX + r * LB + c), sE[r]));
-    st4(kt + at * CC * CD + i * 4, scaled(ld4(sK + r * LB + c), expf(g_last - sG[r])));
+    st4(kt + at * CC * CD + i * 4, scaled(ld4(sK + r * LB + c), expf(g_last.minus(sG[r]))));
   }
   {
     float kk[4][4] = {}, qk[4][4] = {};
@@ -253,7 +269,7 @@ chunk_fwd_kernel(const ChunkStream<T> p, float* __restrict__ w, float* __restric
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const int i = ty + 16 * a, j = tx + 16 * b;
-        const float d = i >= j ? expf(sG[i] - sG[j]) : 0.f;
+        const float d = i >= j ? expf(sG[i].minus(sG[j])) : 0.f;
         const float av = i > j ? kk[a][b] * sB[i] * d : 0.f;
         sA[i * LS + j] = av;
         sT[i * LS + j] = 0.f;
@@ -305,18 +321,19 @@ chunk_bwd_kernel(const ChunkStream<T> p, const float* __restrict__ w, const floa
   float* B1 = B0 + CC * LB;
   float* s0 = B1 + CC * LB;
   float* s1 = s0 + CC * LS;
-  __shared__ float sG[CC], sB[CC], sE[CC], rq[CC], rk[CC], row_g[CC], row_t[CC], row_b[CC], col_e[CT / 32][CC];
+  __shared__ LogDecay sG[CC];
+  __shared__ float sB[CC], sE[CC], rq[CC], rk[CC], row_g[CC], row_t[CC], row_b[CC], col_e[CT / 32][CC];
   __shared__ long rowmap[CC];
   const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const long at = static_cast<long>(h) * p.n + chunk;
   const long big = at * CC * CD, small = at * CC * CC;
   const long ldo = static_cast<long>(p.H) * CD;   // gradients of the stream are dense [rows, H, 128]
   load_gates(p, rowmap, sG, sB, chunk, h);
-  if (tid < CC) sE[tid] = expf(sG[tid]);
+  if (tid < CC) sE[tid] = expf(sG[tid].hi);
   load_small(s0, Tinv + small);
   load_big(B0, du + big);
   __syncthreads();
-  const float g_last = sG[CC - 1];
+  const LogDecay g_last = sG[CC - 1];
 
   // d(b v) = T^T du, d(b e^G k) = T^T dw, dA = -(d(b v) u^T + d(b e^G k) w^T)
   float dA[4][4] = {};
@@ -368,7 +385,7 @@ chunk_bwd_kernel(const ChunkStream<T> p, const float* __restrict__ w, const floa
         const int j = tx + 16 * b;
         float m = 0.f, nn = 0.f, e = 0.f;
         if (i >= j) {
-          const float d = expf(sG[i] - sG[j]);
+          const float d = expf(sG[i].minus(sG[j]));
           const float da = dattn[small + i * CC + j];
           nn = da * d;
           e = da * attn[small + i * CC + j];
@@ -447,7 +464,7 @@ chunk_bwd_kernel(const ChunkStream<T> p, const float* __restrict__ w, const floa
   for (int a = 0; a < 4; ++a) {
     const int r = 4 * ty + a;
     const long row = rowmap[r];
-    const float fall = expf(g_last - sG[r]);
+    const float fall = expf(g_last.minus(sG[r]));
     float ts = 0.f, bs = 0.f, kd = 0.f;
     float4 kh[2];
 #pragma unroll
@@ -484,7 +501,7 @@ chunk_bwd_kernel(const ChunkStream<T> p, const float* __restrict__ w, const floa
     float lo = row_g[tid], hi = row_g[tid + 32];
 #pragma unroll
     for (int wv = 0; wv < CT / 32; ++wv) { lo -= col_e[wv][tid]; hi -= col_e[wv][tid + 32]; }
-    const float last = warp_sum(row_t[tid] + row_t[tid + 32]) + dgamma[at] * expf(g_last);
+    const float last = warp_sum(row_t[tid] + row_t[tid + 32]) + dgamma[at] * expf(g_last.hi);
     if (tid == 31) hi += last;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -210,3 +210,36 @@ def test_fused_chunk_kernels_match_64_bit_rule(lengths, heads, dtype, strided):
         print(f"{name}: fused {err:.3e} framework ops {was:.3e}")
         assert err < tol, name
         assert err < 1.5 * was + 1e-6, f"{name}: {err} against {was}"
+
+
+@pytest.mark.parametrize("decay", [0.01, 1.0, 4.0, 16.0])
+def test_fused_chunk_kernels_are_as_close_as_framework_ops(decay):
+    """fp32 streams at weak to strong decays: outputs and gradients of the fused kernels against the rule in 64 bits, no further
+    off than the framework-op form (sums of some thousand terms in two orders: a tenth between them is chance)."""
+    from lmms_engine_b200.ops import gdn
+
+    torch.manual_seed(2)
+    lengths, heads = [300, 65], 4
+    T = sum(lengths)
+    q, k, v, go = (torch.randn(T, heads, 128) for _ in range(4))
+    g, beta = -decay * torch.rand(T, heads), torch.rand(T, heads)
+    ref = [t.double().requires_grad_() for t in (q, k, v, g, beta)]
+    want = _rule64(*ref, lengths)
+    (want * go.double()).sum().backward()
+
+    def run(fused):
+        leaves = [t.cuda().requires_grad_() for t in (q, k, v, g, beta)]
+        keep = gdn.chunk_kernels_cover
+        if not fused:
+            gdn.chunk_kernels_cover = lambda *a: False
+        try:
+            out = gdn.chunk_gated_delta_rule_packed(*leaves, lengths)
+            out.backward(go.cuda())
+        finally:
+            gdn.chunk_kernels_cover = keep
+        return [out.detach()] + [t.grad for t in leaves]
+
+    for name, a, o, b in zip(("out", "q", "k", "v", "g", "beta"), run(True), run(False), [want] + [r.grad for r in ref]):
+        b = b.detach()
+        err, was = ((t.cpu().double() - b).norm() / b.norm() for t in (a, o))
+        assert err < 1.1 * was, f"{name}: {err:.3e} against {was:.3e}"
