@@ -1269,9 +1269,12 @@ int b200_gemm_grouped_wgrad_bf16(const void* A, const void* B, void* dW, const v
   if (M <= 0 || N <= 0 || E <= 0) return 0;
   if ((lda | ldb) & 7) return -10;
   CUtensorMap tA, tB, tC;
-  // CTA pairs (256 x 256 tiles) wherever the shape allows, like the plain products: the tiles of an expert do not depend on
-  // its row count, so nothing is wasted.  128 experts of 576 rows, 1536 x 2048 and 2048 x 768: 0.95 PFLOP/s on single CTAs.
-  const bool pair = pair_shape_ok(M, N);
+  // CTA pairs (256 x 256 tiles) where the shape allows it and an expert's rows are many enough: below about 512 rows a tile is
+  // a few K steps and the time is that of writing dW, which twice as many smaller tiles spread better.  us, single CTAs / pairs,
+  // rows per expert 256, 384, 512, 640: 128 experts of 1536 x 2048 255 / 339, 316 / 359, 423 / 437, 526 / 473; of 2048 x 768
+  // 168 / 223, 194 / 244, 254 / 210, 254 / 231; 64 of 768 x 768 40 / 46, 43 / 49, 49 / 51, 57 / 54.  `rows` counts up to 64 unused
+  // rows an expert on average.
+  const bool pair = pair_shape_ok(M, N) && rows >= 576L * E;
   int a3d = M % 64 == 0 && lda >= M, b3d = N % 64 == 0 && ldb >= N;
   if (a3d && make_map_mn3d(&tA, A, rows, M, lda, 2) != 0) a3d = 0;
   if (b3d && make_map_mn3d(&tB, B, rows, N, ldb, pair ? 2 : BN / 64) != 0) b3d = 0;
