@@ -128,6 +128,19 @@ def is_muon_param(name: str, p: torch.Tensor) -> bool:
     return p.ndim == 2 and not any(pat in name for pat in MUON_EXCLUDE_PATTERNS)
 
 
+def muon_lanes(shapes, steps: int, sms: int) -> int:
+    """How many chains of matrices run side by side, each confined to its share of the SMs.
+
+    A chain alone leaves SMs idle where its symmetric products have fewer 256 x 256 tiles than the chip has CTA pairs, so the
+    narrower the matrices the more lanes; side by side, chains of wide matrices compete for L2 (a 3584 x 18944 matrix is larger
+    than it).  Step of the optimizer in ms, two / four lanes, one B200 (74 CTA pairs): 512 units (3 tiles) 8.1 / 4.6, 1024 (10)
+    42.0 / 33.8, 2048 (36) 32.8 / 27.8, 2560 (55) 31.6 / 29.7, 3072 (78) 25.4 / 24.2, 3328 (91) 29.7 / 29.8, 3584 (105) 28.6 /
+    30.9.  The line lies behind 3328: five quarters of the pairs.  More lanes than matrices would leave SMs unused."""
+    work = [(ns_flops(s, steps), (min(s) + 255) // 256) for s in shapes]
+    wide = sum(c for c, t in work if t * (t + 1) // 2 > sms // 2 * 5 // 4)
+    return max(1, min(len(work), 2 if 2 * wide > sum(c for c, _ in work) else 4))
+
+
 def ns_flops(shape, steps: int = 5) -> float:
     m, n = shape
     k, big = (n, m) if m > n else (m, n)

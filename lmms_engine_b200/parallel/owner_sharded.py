@@ -464,7 +464,7 @@ class OwnerShardedRuntime:
     def _muon_update(self, lr: float, gscale: torch.Tensor) -> None:
         """Momentum, Newton-Schulz and the update of every matrix this rank owns.
 
-        On CUDA the matrices are dealt by cost to ``muon_lanes`` streams and every GEMM of a lane
+        On CUDA the matrices are dealt by cost to ``ops.muon.muon_lanes`` streams and every GEMM of a lane
         is confined to ``SMs / lanes`` CTAs: the symmetric products of one matrix have too few tiles
         for the whole GPU (210 upper-triangle tiles for a 3584 x 3584 product, 5 for a 512-row KV
         projection), so running several chains side by side on part of the SMs each removes most of
@@ -502,7 +502,7 @@ class OwnerShardedRuntime:
         far; the lanes start after what is queued on the current stream and the current stream waits for them.  Dealt in
         turn, two of a layer's three wide matrices often met on one lane while another had none (two 3584-wide layers on four
         lanes: 24.5 units of work on the longest against 14 on the shortest)."""
-        lanes = self._muon_lanes()
+        lanes = self._muon_lanes(matrices)
         n_l = len(lanes)
         main = torch.cuda.current_stream() if n_l > 1 else None
         if n_l > 1:
@@ -525,12 +525,14 @@ class OwnerShardedRuntime:
 
     PUBLISH_BLOCKS = int(os.environ.get("LMMS_B200_PUBLISH_BLOCKS", "32"))
 
-    def _muon_lanes(self):
+    def _muon_lanes(self, matrices):
         if self._lanes is None:
-            n = 1
+            n = sms = 0
             if self.P.is_cuda:
-                n = max(1, int(os.environ.get("LMMS_B200_MUON_LANES", "2")))
-            sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.P.is_cuda else 0
+                sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+                n = int(os.environ.get("LMMS_B200_MUON_LANES", "0")) or muon_ops.muon_lanes(
+                    [tuple(s.shape) for s in matrices], self.muon["ns_steps"], sms)
+            n = max(1, n)
             self._lanes = []
             for i in range(n):
                 self._lanes.append({

@@ -642,3 +642,17 @@ def test_head_norms_are_read_only_where_a_call_does_nothing_else(what, monkeypat
         assert got[0] is att.q_norm.weight and got[1] is k.weight
     else:
         assert got is False
+
+
+@pytest.mark.parametrize("widths,lanes", [((512, 1408, 256), 4), ((1024, 3072, 1024), 4), ((2560, 9728, 1024), 4), ((3328, 13312, 256), 4),
+                                          ((3584, 18944, 512), 2), ((5120, 27648, 1024), 2)])
+def test_muon_lanes_follow_the_tiles_of_the_matrices(widths, lanes):
+    """Narrow matrices leave a chip idle on two lanes, wide ones compete for L2 on four; a rank with few matrices opens no more
+    lanes than it has matrices."""
+    from lmms_engine_b200.ops.muon import muon_lanes
+
+    h, inter, kv = widths
+    layer = [(h, h), (kv, h), (kv, h), (h, h), (inter, h), (inter, h), (h, inter)]
+    assert muon_lanes(layer * 3, 5, 148) == lanes
+    assert muon_lanes(layer[-1:], 5, 148) == 1 and muon_lanes(layer[-2:], 5, 148) == 2
+    assert muon_lanes([], 5, 148) == 1
