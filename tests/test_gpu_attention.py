@@ -187,5 +187,47 @@ def test_head_norm_rotation_attention(lens, n_q, n_kv, D):
     with torch.no_grad():
         q2, k2 = attention.rope_heads(dev[0], cos.cuda(), sin.cuda(), n_q, n_kv, D, (dev[1], dev[2], 1e-6))
         q1 = rope.rope_apply(norm.rmsnorm(dev[0][:, :n_q * D].reshape(-1, D), dev[1], 1e-6).view(T, n_q, D), cos.cuda(), sin.cuda())
-    # the separate kernels sum a head's squares in another order: one bf16 step
-    assert torch.allclose(q2.float(), q1.float(), rtol=2 ** -7, atol=2 ** -8) and k2.shape == (T, n_kv, D)
+    assert torch.equal(q2, q1) and k2.shape == (T, n_kv, D)  # the sums run in the order of the separate kernels
+
+
+@pytest.mark.parametrize("D,heads,kv", [(64, 6, 2), (128, 5, 1), (128, 4, 4)])
+@pytest.mark.parametrize("lens", [(1,), (130, 7, 64)])
+def test_fused_head_norm_gives_the_bits_of_the_separate_passes(D, heads, kv, lens):
+    """An attention layer with the per-head norms read by the fused kernels and with the norms called (a hook asks for that):
+    outputs and all gradients but the two norm weights' are equal bit by bit; those are fp32 sums over the rows in another
+    order, rounded once."""
+    from lmms_engine_b200.models.decoder_lm import Attention, DecoderConfig, PackedContext
+    from lmms_engine_b200.ops import _cuda
+
+    torch.manual_seed(5)
+    T, H = sum(lens), 256
+    cfg = DecoderConfig(hidden_size=H, num_attention_heads=heads, num_key_value_heads=kv, head_dim=D, qk_norm=True, attention_bias=True)
+    with torch.device("cuda"):
+        layer = Attention(cfg, 0).to(torch.bfloat16)
+        with torch.no_grad():
+            layer.q_norm.weight.add_(0.3 * torch.randn(D))
+            layer.k_norm.weight.add_(0.3 * torch.randn(D))
+        ang = torch.randn(T, D // 2).repeat(1, 2)
+        cu = torch.tensor([0] + torch.tensor(lens, device="cpu").cumsum(0).tolist(), dtype=torch.int32)
+        x, dy = torch.randn(T, H).bfloat16(), torch.randn(T, H).bfloat16()
+    ctx = PackedContext(cu, max(lens), ang.cos(), ang.sin(), True)
+
+    def run():
+        layer.zero_grad(set_to_none=True)
+        xs, n0 = x.clone().requires_grad_(), _cuda.launch_count
+        y = layer(xs, ctx)
+        y.backward(dy)
+        return _cuda.launch_count - n0, {"y": y.detach(), "x": xs.grad, **{n: p.grad.clone() for n, p in layer.named_parameters()}}
+
+    fused_launches, fused = run()
+    hooks = [m.register_forward_hook(lambda *a: None) for m in (layer.q_norm, layer.k_norm)]
+    separate_launches, separate = run()
+    for h in hooks:
+        h.remove()
+    assert fused_launches < separate_launches
+    for name, a in fused.items():
+        b = separate[name]
+        if "norm" in name:
+            assert ((a.float() - b.float()).abs() <= 2 ** -8 * b.float().abs() + 1e-6 * T ** 0.5).all(), name
+        else:
+            assert torch.equal(a, b), name

@@ -112,6 +112,40 @@ def test_moe_block_forward_backward(T, H, I, E, k):
     assert rel(gate.grad, gr.grad) < 6e-2
 
 
+@pytest.mark.parametrize("T,H,I", [(3000, 256, 128), (200, 256, 128), (3000, 256, 64), (3000, 128, 128)])
+def test_stale_memory_and_experts_without_rows(T, H, I):
+    """Tiles that no expert owns are written by no kernel: whatever their memory held may not reach a result.  Experts without
+    rows get weight gradients of zero, on CTA pairs (576 rows an expert and more, both sides at least 128 and the first above)
+    and on single CTAs."""
+    from lmms_engine_b200.ops import moe, _cuda
+
+    E, k = 8, 2
+    torch.manual_seed(0)
+    x, gu, dn, dy = _rand(T, H), _rand(E, 2 * I, H, scale=0.05), _rand(E, H, I, scale=0.05), _rand(T, H)
+    idx = torch.tensor([[2, 5]], dtype=torch.int32, device="cuda").repeat(T, 1)
+    w = torch.rand(T, k, device="cuda")
+    counts = torch.bincount(idx.flatten().long(), minlength=E).int()
+
+    def run(fill):
+        leaves = [t.clone().requires_grad_() for t in (x, gu, dn)]
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        stale = [torch.full((1 << 20,), fill, device="cuda", dtype=torch.bfloat16) for _ in range(64)]
+        del stale  # stays with the allocator, which hands it out again as it is
+        perm = moe.build_permutation(idx, w, counts)
+        y = moe.combine(moe.grouped_mlp(moe.dispatch(leaves[0], perm), leaves[1], leaves[2], perm), w, perm)
+        y.backward(dy)
+        return [y.detach()] + [t.grad for t in leaves]
+
+    clean, stale = run(0.0), run(float("nan"))
+    _cuda.check_status()
+    for a, b in zip(clean, stale):
+        assert torch.isfinite(b).all() and torch.equal(a, b)
+    for grad in stale[2:]:
+        for e in range(E):
+            assert bool((grad[e] == 0).all()) == (e not in (2, 5))
+
+
 def test_moe_model_trains():
     from lmms_engine_b200.models import MoEConfig, MoEDecoderLM
     from lmms_engine_b200.parallel.owner_sharded import OwnerShardedRuntime
