@@ -362,16 +362,17 @@ class DecoderBackbone(nn.Module):
         invf = self.inv_freq
         if invf.dtype == torch.float32 and invf.device == device:
             return invf
-        kept, key = None, None
-        if torch.device(device).type == "cuda" and not torch.cuda.is_current_stream_capturing():
-            kept = self.__dict__.setdefault("_fp32_frequencies", {})
-            key = (dim, float(self.cfg.rope_theta), device, torch.cuda.current_stream(device).cuda_stream)
-            if key in kept:
-                return kept[key]
-        fresh = rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
-        if kept is not None and type(fresh) is torch.Tensor:
-            kept[key] = fresh
-        return fresh
+        if device.type != "cuda":
+            return rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
+        kept = self.__dict__.setdefault("_fp32_frequencies", {})
+        index = device.index if device.index is not None else torch.cuda.current_device()
+        key = (dim, self.cfg.rope_theta, index, torch._C._cuda_getCurrentRawStream(index))
+        got = kept.get(key)
+        if got is None:
+            got = rope_ops.inv_freq(dim, self.cfg.rope_theta, device=device)
+            if type(got) is torch.Tensor and not torch.cuda.is_current_stream_capturing():
+                kept[key] = got
+        return got
 
     def __getstate__(self):
         # a copy of the model computes its own: copies are made on other streams
