@@ -94,10 +94,11 @@ def _delta(items, net, cls, eps, H):
     if net.eps != eps or type(m["norm"]) is not torch.nn.Module:
         raise _Unfit
     key, val, hv = net.key_dim, net.value_dim, net.hv
-    for i, (name, n) in enumerate((("in_proj_qkv", 2 * key + val), ("in_proj_z", val), ("in_proj_b", hv), ("in_proj_a", hv))):
-        items.append((1 + i, _own(m[name]).get("weight"), (n, H)))
-    items += ((9, _own(m["conv1d"], torch.nn.Conv1d).get("weight"), (2 * key + val, 1, net.kernel)), (10, own.get("A_log"), (hv,)),
-              (16, own.get("dt_bias"), (hv,)), (17, m["norm"]._parameters.get("weight"), (net.dv,)),
+    heads, conv = (hv, H), 2 * key + val
+    items += ((1, _own(m["in_proj_qkv"]).get("weight"), (conv, H)), (2, _own(m["in_proj_z"]).get("weight"), (val, H)),
+              (3, _own(m["in_proj_b"]).get("weight"), heads), (4, _own(m["in_proj_a"]).get("weight"), heads),
+              (9, _own(m["conv1d"], torch.nn.Conv1d).get("weight"), (conv, 1, net.kernel)), (10, own.get("A_log"), (hv,)),
+              (16, own.get("dt_bias"), (hv,)), (17, m["norm"].__dict__["_parameters"].get("weight"), (net.dv,)),
               (11, _own(m["out_proj"]).get("weight"), (H, val)))
 
 
@@ -119,7 +120,7 @@ def _delta_state(store, net, seqs, where):
             tail, S = tail.to(_BF16).contiguous(), S.float().clone(memory_format=torch.contiguous_format)
         tail_out, S_out = torch.empty_like(tail), torch.empty_like(S)
         ptrs += (tail.data_ptr(), tail_out.data_ptr(), S.data_ptr(), S_out.data_ptr())
-        new.append((i, tail, S, (tail_out, S_out)))
+        new.append((i, (tail_out, S_out), tail, S))  # the old ones until the kernels are queued
     return ptrs, new
 
 
@@ -217,8 +218,7 @@ def _run(backbone, embeds, ctx, cache, seqs):
     # shares of a key head: enough to fill the chip about twice or 512 keys each (a batch waits for its longest sequence),
     # whichever are more, and at least 64 keys each
     splits = max(1, min(max(-(-2 * _sms(dev) // (nkv * M)), -(-longest // 512)), -(-longest // 64), 64))
-    has_attn = any(t != 2 for t in types)
-    np_ = max(nq * D * 2 + 2 * nkv * D if has_attn else 0, (2 * hk + 2 * hv) * 128 + 2 * hv)
+    np_ = max(nq * D * 2 + 2 * nkv * D if len(nets) < len(types) else 0, (2 * hk + 2 * hv) * 128 + 2 * hv)
     work = torch.empty(2 * M * (np_ + max(nq * D, hv * 128) + I + H) + 4096, dtype=torch.uint8, device=dev)
     n_ws = M * nkv * splits * (nq // nkv) * (D + 2)
     shares = torch.empty(n_ws if splits > 1 else 1, dtype=torch.float32, device=dev)
@@ -232,6 +232,6 @@ def _run(backbone, embeds, ctx, cache, seqs):
                float(cfg.rms_norm_eps), norm_off, D ** -0.5, cos.data_ptr(), sin.data_ptr(), res.data_ptr(), hidden.data_ptr(), final,
                work.data_ptr(), work.numel(), shares.data_ptr(), count.data_ptr(), _cuda.stream())
     for store, new in news:
-        for i, _, _, entry in new:
+        for i, entry, _, _ in new:
             store[i] = entry
     return hidden
