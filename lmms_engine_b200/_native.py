@@ -59,6 +59,13 @@ def _nvcc() -> Optional[str]:
     return None
 
 
+def _nvcc_flags(src: Path) -> List[str]:
+    """Flags of one source.  A file whose values have to be as precise as the framework operations that it takes the place of says
+    ``// build: without --use_fast_math``."""
+    plain = "// build: without --use_fast_math" in src.read_text(errors="ignore")
+    return [f for f in NVCC_FLAGS if not (plain and f == "--use_fast_math")]
+
+
 def cuda_sources() -> List[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -129,7 +136,7 @@ def _compile(src: Path, verbose: bool = False) -> str:
         nvcc = _nvcc()
         if nvcc is None:
             raise RuntimeError(f"nvcc not found; cannot build {src.name}")
-        cmd = [nvcc, *NVCC_FLAGS, "-I", str(CSRC), "-o", str(out), str(src)]
+        cmd = [nvcc, *_nvcc_flags(src), "-I", str(CSRC), "-o", str(out), str(src)]
         if verbose:
             cmd.insert(1, "-Xptxas")
             cmd.insert(2, "-v")

@@ -8,8 +8,8 @@
 //     launch, ramp-up and DRAM latency of one kernel hide behind the tail of another; the row norm and the Gated-DeltaNet step
 //     have nothing that they could load early and only launch early;
 //   * read weights straight from global memory into mma.sync fragments (no shared-memory staging, see skinny_kernel);
-//   * round to bf16 where the layer-by-layer path does (projection outputs, normalised rows, the residual stream), so
-//     both paths compute the same numbers up to the order of fp32 sums.
+//   * round to bf16 where the layer-by-layer path does (projection outputs, normalised rows, the residual stream) and evaluate
+//     gates and decays as precisely as it does, so both paths compute the same numbers up to the order of fp32 sums.
 //
 //   skinny_kernel   y[M, N] = x[M, K] w[N, K]^T for M <= 64 rows, RMSNorm of x in its prologue (M <= 4), bias /
 //                   residual add / SwiGLU in its epilogue, up to four weight matrices side by side along N
@@ -19,6 +19,8 @@
 //
 // Reference counterpart: the same modules run one by one through transformers' generate
 // (src/lmms_engine/models/aero_realtime/modeling_aero_realtime.py:700-1385 for the streaming loop).
+// build: without --use_fast_math (gates and decays as the framework operations of the layer loop compute them; where the kernels of
+// that path use the fast exponential and division, these are written out)
 #include <atomic>
 
 #include "common.cuh"
@@ -44,8 +46,8 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + __expf(-x)); }
 __device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
   const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kSkWarps * 32) skinny_kernel(const __grid_cons
       if (p.bias[1] != nullptr) uv += __bfloat162float(p.bias[1][n]);
       gv = round_bf16(gv);
       uv = round_bf16(uv);
-      p.y[m * p.ldy + n] = __float2bfloat16(gv / (1.0f + __expf(-gv)) * uv);
+      p.y[m * p.ldy + n] = __float2bfloat16(__fdividef(gv, 1.0f + __expf(-gv)) * uv);
     }
   } else {
     for (int i = threadIdx.x; i < p.M * kCols; i += kSkWarps * 32) {
@@ -553,7 +555,7 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
       }
     }
     if (p.splits == 1) {
-      store(h, d, v / l);
+      store(h, d, __fdividef(v, l));
     } else {
       wo[(split * p.group + h) * D + d] = v;
       if (d == 0) wml[split * p.group + h] = make_float2(m, l);
@@ -600,7 +602,8 @@ __global__ void __launch_bounds__(128) dec_attn_kernel(const __grid_constant__ D
       v.z += __shfl_xor_sync(0xffffffffu, v.z, 16); v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
     }
     if (sg == 0) {
-      store(h, d0, v.x / l); store(h, d0 + 1, v.y / l); store(h, d0 + 2, v.z / l); store(h, d0 + 3, v.w / l);
+      const float inv = __fdividef(1.f, l);
+      store(h, d0, v.x * inv); store(h, d0 + 1, v.y * inv); store(h, d0 + 2, v.z * inv); store(h, d0 + 3, v.w * inv);
     }
   }
 }
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(256) gdn_step_kernel(const __grid_constant__ G
       if (keeper && p.taps - 2 - j >= 0) to[static_cast<size_t>(p.taps - 2 - j) * p.conv_dim + ch] = old;
     }
     if (keeper) to[static_cast<size_t>(p.taps - 2) * p.conv_dim + ch] = pr[ch];
-    const float y = round_bf16(acc / (1.0f + __expf(-acc)));
+    const float y = round_bf16(__fdividef(acc, 1.0f + __expf(-acc)));
     (which == 0 ? sq : (which == 1 ? sk : sv))[d] = y;
   }
   __syncthreads();
@@ -698,7 +701,7 @@ __global__ void __launch_bounds__(256) gdn_step_kernel(const __grid_constant__ G
     const float rstd = rsqrtf((red[0] + red[1] + red[2] + red[3]) / kGdnD + p.eps);
     const float n = round_bf16(o * rstd * __bfloat162float(p.norm_w[col]));
     const float z = __bfloat162float(pr[p.z_off + vh * kGdnD + col]);
-    p.out[seq * p.ldo + static_cast<long>(vh) * kGdnD + col] = __float2bfloat16(n * (z / (1.0f + __expf(-z))));
+    p.out[seq * p.ldo + static_cast<long>(vh) * kGdnD + col] = __float2bfloat16(n * (z / (1.0f + expf(-z))));
   }
 }
 

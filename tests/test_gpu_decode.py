@@ -15,7 +15,7 @@ def _model(kind, **sizes):
         cfg = dict(DENSE, num_attention_heads=4, num_key_value_heads=2, head_dim=128, linear_conv_kernel_dim=4, linear_key_head_dim=128,
                    linear_value_head_dim=128, linear_num_key_heads=4, linear_num_value_heads=8, partial_rotary_factor=0.25,
                    full_attention_interval=2)
-        m = create_model_from_config("qwen3_5_text", cfg)
+        m = create_model_from_config("qwen3_5_text", dict(cfg, **sizes))
     else:
         heads, kv, dim, extra = {"grouped": (14, 2, 128, {}), "normed": (4, 2, 128, dict(attention_bias=False, qk_norm=True)),
                                  "narrow": (4, 4, 64, {}), "wide_group": (12, 1, 128, {}),
@@ -275,3 +275,38 @@ def test_an_earlier_recurrent_state_stays_as_it_was():
         assert held and all(torch.equal(a, b) for layer in held for i in held[layer] for a, b in zip(held[layer][i], copies[layer][i]))
         cache.state, cache.lens = {layer: dict(e) for layer, e in held.items()}, [31]
         assert torch.equal(token(7), first)
+
+
+def _one_token(model, cache, embeds):
+    """A pass of one token with given embeddings (the layer loop where the one-call path declines)."""
+    from lmms_engine_b200.models.decoder_lm import PackedContext
+
+    pos = cache.advance([1])
+    ctx = PackedContext(torch.tensor([0, 1], dtype=torch.int32, device="cuda"), 1, *model.model.rope_tables(pos), True)
+    ctx.kv_cache = cache
+    with torch.no_grad():
+        return model.model(embeds, ctx)
+
+
+def test_decay_of_a_token_is_as_precise_as_in_the_layer_loop(monkeypatch):
+    """A token of zeros leaves only the decay of the state: exp(-exp(A) softplus(dt)) against 64 bits, decays down to e^-13."""
+    from lmms_engine_b200.models import decode_path
+    from lmms_engine_b200.models.kv_cache import PackedKVCache
+
+    model = _model("hybrid", linear_num_value_heads=256, linear_num_key_heads=8, num_hidden_layers=1)
+    net = model.model.layers[0].linear_attn
+    with torch.no_grad():
+        net.A_log.copy_(torch.linspace(-4.0, 1.5, 256))
+        net.dt_bias.copy_(torch.randn(256) * 1.5)
+    want = (-net.A_log.double().exp() * torch.nn.functional.softplus(net.dt_bias.double())).exp()
+    err = {}
+    for native in (True, False):
+        monkeypatch.setattr(decode_path, "MAX_SEQS", 64 if native else 0)
+        cache = PackedKVCache(1, [4], device=torch.device("cuda", 0))
+        cache.state[0] = {0: (torch.zeros(3, 2 * net.key_dim + net.value_dim, device="cuda", dtype=torch.bfloat16),
+                              torch.ones(256, 128, 128, device="cuda"))}
+        _one_token(model, cache, torch.zeros(1, 256, device="cuda", dtype=torch.bfloat16))
+        got = cache.state[0][0][1]
+        assert torch.equal(got, got[:, :1, :1].expand_as(got))
+        err[native] = ((got[:, 0, 0].double() / want) - 1).abs()
+    assert err[True].norm() < 1.1 * err[False].norm() + 1e-7, (err[True].norm().item(), err[False].norm().item())
