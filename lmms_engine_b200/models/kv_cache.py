@@ -28,7 +28,8 @@ class PackedKVCache:
         self.device = device
         self._rows: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, int]] = None
         # layers that carry a recurrent state instead of keys / values (linear attention) keep it here:
-        # ``state[layer][sequence]`` is whatever that layer stores (convolution tail, state matrix)
+        # ``state[layer][sequence]`` is whatever that layer stores (convolution tail, state matrix); a pass replaces an entry
+        # and writes into no tensor of it, so a caller may keep one to go back to
         self.state: dict = {}
         self.new_lens: List[int] = []
         self.had: List[int] = []
